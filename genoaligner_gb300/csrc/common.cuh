@@ -27,7 +27,7 @@ enum : int {
 struct PairDesc {
     const uint8_t* seq;
     const uint64_t* packed;   // 2-bit arena (32 bases per word)
-    const uint8_t* pure;      // per sequence: 1 if every byte is A, C, G or T
+    const uint8_t* pure;      // per sequence: 1 if every byte is A, C, G or T; 2 (no 2-bit arena) if some are N; else 0
     const int64_t* a_off;
     const int32_t* a_len;
     const int64_t* b_off;

@@ -172,7 +172,7 @@ __global__ void __launch_bounds__(128) sw_kernel(SwArgs A)
         int best = 0, bi = 0, bj = 0;
         uint64_t bkey = ~0ull;
         if (m > 0 && n > 0) {
-            const bool pure = A.D.pure && A.D.pure[p] && A.D.pure[A.D.n + p];
+            const bool pure = A.D.pure && A.D.pure[p] == 1 && A.D.pure[A.D.n + p] == 1;
             if (pure) sw_forward<C, true>(A, m, n, text, pat, eslot, prof, t, best, bi, bj, bkey);
             else      sw_forward<C, false>(A, m, n, text, pat, eslot, prof, t, best, bi, bj, bkey);
             // warp reduction of the best cell: the smallest key among the maxima

@@ -47,12 +47,15 @@ constexpr int CK_BIAS = BIAS16;          // value bias of the recompute pass
 constexpr int CK_MAX_TG = 4;             // widest recompute window, tiles
 // shared memory words per warp: the forward band profile, or the window
 // profile (TW * TG / 32 columns per lane) plus the window's column edges
-constexpr int CK_LETTERS = 5;           // forward profile rows per pair: A C G T, then the padding row
-constexpr int CK_FWD_WORDS = 2 * CK_LETTERS * (CK_C / 2) * 32;
-constexpr int CK_WIN_WORDS = 2 * 4 * (TW * CK_MAX_TG / 64) * 32 + 2 * CK_MAX_TG * CK_K;
+constexpr int CK_WL = 5;                // profile rows per pair: A C G T N
+constexpr int CK_PAD = 2 * CK_WL;       // the forward profile's padding row, one for both pairs
+constexpr int CK_FWD_WORDS = (CK_PAD + 1) * (CK_C / 2) * 32;
+constexpr int CK_WIN_WORDS = 2 * CK_WL * (TW * CK_MAX_TG / 64) * 32 + 2 * CK_MAX_TG * CK_K;
 constexpr int CK_WARP_WORDS = CK_FWD_WORDS > CK_WIN_WORDS ? CK_FWD_WORDS : CK_WIN_WORDS;
 
-__device__ __forceinline__ int ck_code(uint32_t c) { return (int)(((c >> 1) ^ (c >> 2)) & 3u); }
+// Profile row of a byte of a 16-bit pair (A, C, G, T or N; N matches N alone,
+// as the reference's byte comparison has it).
+__device__ __forceinline__ int ck_code(uint32_t c) { return c == 'N' ? 4 : (int)(((c >> 1) ^ (c >> 2)) & 3u); }
 __device__ __forceinline__ int lo16s(uint32_t x) { return (int)(int16_t)(x & 0xffffu); }
 __device__ __forceinline__ int hi16s(uint32_t x) { return (int)(int16_t)(x >> 16); }
 
@@ -90,9 +93,9 @@ __device__ __forceinline__ bool ck_better(int v, int r, int c, int bv, int br, i
 }
 
 // Forward profile of a band at CB columns per lane:
-// prof[((pair * 5 + letter) * (CB / 2) + h) * 32 + t] holds the 16-bit scores
-// (s + gap_open) of this lane's columns 2h, 2h+1.  Past a pattern's end, and
-// in the padding letter 4 (the rows past a pair's text), a score far below any
+// prof[((pair * CK_WL + letter) * (CB / 2) + h) * 32 + t] holds the 16-bit
+// scores (s + gap_open) of this lane's columns 2h, 2h+1.  Past a pattern's end,
+// and in the padding row CK_PAD (the rows past a pair's text), a score far below any
 // reachable value: there H is at most the best of the rows above less
 // gap_open, so padding cells never hold a new best.
 template <int CB>
@@ -104,20 +107,19 @@ __device__ __forceinline__ void ck_profile_fwd(uint32_t* prof, const uint8_t* pa
 #pragma unroll
     for (int h = 0; h < CB / 2; ++h) {
         const int c0 = 2 * h, c1 = 2 * h + 1;
-        const int a0 = c0 < nvA ? ck_code(__ldg(patA + j0 + c0)) : 4;
-        const int a1 = c1 < nvA ? ck_code(__ldg(patA + j0 + c1)) : 4;
-        const int b0 = c0 < nvB ? ck_code(__ldg(patB + j0 + c0)) : 4;
-        const int b1 = c1 < nvB ? ck_code(__ldg(patB + j0 + c1)) : 4;
+        const int a0 = c0 < nvA ? ck_code(__ldg(patA + j0 + c0)) : CK_PAD;
+        const int a1 = c1 < nvA ? ck_code(__ldg(patA + j0 + c1)) : CK_PAD;
+        const int b0 = c0 < nvB ? ck_code(__ldg(patB + j0 + c0)) : CK_PAD;
+        const int b1 = c1 < nvB ? ck_code(__ldg(patB + j0 + c1)) : CK_PAD;
+        // off a match: PAD past the pattern's end, else the mismatch
+        const int xa0 = a0 == CK_PAD ? PAD : sx, xa1 = a1 == CK_PAD ? PAD : sx;
+        const int xb0 = b0 == CK_PAD ? PAD : sx, xb1 = b1 == CK_PAD ? PAD : sx;
 #pragma unroll
-        for (int L = 0; L < 4; ++L) {
-            const int va0 = a0 == 4 ? PAD : (a0 == L ? sm : sx), va1 = a1 == 4 ? PAD : (a1 == L ? sm : sx);
-            const int vb0 = b0 == 4 ? PAD : (b0 == L ? sm : sx), vb1 = b1 == 4 ? PAD : (b1 == L ? sm : sx);
-            prof[((0 * CK_LETTERS + L) * (CB / 2) + h) * 32 + t] = ((uint32_t)va0 & 0xffffu) | ((uint32_t)va1 << 16);
-            prof[((1 * CK_LETTERS + L) * (CB / 2) + h) * 32 + t] = ((uint32_t)vb0 & 0xffffu) | ((uint32_t)vb1 << 16);
+        for (int L = 0; L < CK_WL; ++L) {
+            prof[(L * (CB / 2) + h) * 32 + t] = __byte_perm(a0 == L ? sm : xa0, a1 == L ? sm : xa1, 0x5410);
+            prof[((CK_WL + L) * (CB / 2) + h) * 32 + t] = __byte_perm(b0 == L ? sm : xb0, b1 == L ? sm : xb1, 0x5410);
         }
-        const uint32_t pad2 = ((uint32_t)PAD & 0xffffu) * 0x10001u;
-        prof[((0 * CK_LETTERS + 4) * (CB / 2) + h) * 32 + t] = pad2;
-        prof[((1 * CK_LETTERS + 4) * (CB / 2) + h) * 32 + t] = pad2;
+        prof[(CK_PAD * (CB / 2) + h) * 32 + t] = ((uint32_t)PAD & 0xffffu) * 0x10001u;
     }
     __syncwarp();
 }
@@ -243,9 +245,9 @@ __device__ void fwd_band(const FwdCtx& X, int b0, int t, int& vA, int& rA, int& 
     // edge -- are read by all lanes together (lane u: row 32k + u) and handed
     // to lane 0 by a shuffle each step, so no step runs a lane-0-only branch.
     auto row_off = [&](int r) -> uint32_t {
-        const int la = r < mA ? ck_code(__ldg(X.textA + r)) : CK_LETTERS - 1;
-        const int lb = r < mB ? ck_code(__ldg(X.textB + r)) : CK_LETTERS - 1;
-        return (uint32_t)(la * NH * 32) | ((uint32_t)((CK_LETTERS + lb) * NH * 32) << 16);
+        const int la = r < mA ? ck_code(__ldg(X.textA + r)) : CK_PAD;
+        const int lb = r < mB ? CK_WL + ck_code(__ldg(X.textB + r)) : CK_PAD;
+        return (uint32_t)(la * NH * 32) | ((uint32_t)(lb * NH * 32) << 16);
     };
     uint32_t rb_off = 0u, rb_hg = NGO2, rb_e = 0u;       // this lane's row of the current 32
     uint32_t ch = 0;
@@ -400,9 +402,9 @@ __device__ void fwd_band2(const FwdCtx& X, int b0, int t, int& vA, int& rA, int&
     const int kout = (j0 + CB) % TW == 0 && j0 + CB < X.ncol ? (j0 + CB) / TW : 0;
     uint32_t* eout = kout ? X.ce + 2 * (int64_t)(kout - 1) * M : nullptr;
     auto row_off = [&](int r) -> uint32_t {
-        const int la = r < mA ? ck_code(__ldg(X.textA + r)) : CK_LETTERS - 1;
-        const int lb = r < mB ? ck_code(__ldg(X.textB + r)) : CK_LETTERS - 1;
-        return (uint32_t)(la * NH * 32) | ((uint32_t)((CK_LETTERS + lb) * NH * 32) << 16);
+        const int la = r < mA ? ck_code(__ldg(X.textA + r)) : CK_PAD;
+        const int lb = r < mB ? CK_WL + ck_code(__ldg(X.textB + r)) : CK_PAD;
+        return (uint32_t)(la * NH * 32) | ((uint32_t)(lb * NH * 32) << 16);
     };
     // lane 0's inputs of 64 rows at a time (lane u: rows 64k + 2u and + 1,
     // 0-based), handed to lane 0 by shuffles
@@ -525,7 +527,7 @@ __device__ void fwd_band2(const FwdCtx& X, int b0, int t, int& vA, int& rA, int&
 }
 
 // Tile profile of one pair for a lane of a tile group (CT columns per lane):
-// prof[((pair * 4 + letter) * CT/2 + h) * 32 + t] holds the 16-bit scores of
+// prof[((pair * CK_WL + letter) * CT/2 + h) * 32 + t] holds the 16-bit scores of
 // the lane's columns col0 + 2h, col0 + 2h + 1 (0-based); past the pattern's
 // end or left of column 0: mismatch.
 template <int CT>
@@ -535,12 +537,12 @@ __device__ __forceinline__ void ck_profile_tile(uint32_t* prof, const uint8_t* p
 #pragma unroll
     for (int h = 0; h < CT / 2; ++h) {
         const int c0 = col0 + 2 * h, c1 = c0 + 1;
-        const int a0 = (c0 >= 0 && c0 < n) ? ck_code(__ldg(pat + c0)) : 4;
-        const int a1 = (c1 >= 0 && c1 < n) ? ck_code(__ldg(pat + c1)) : 4;
+        const int a0 = (c0 >= 0 && c0 < n) ? ck_code(__ldg(pat + c0)) : CK_WL;
+        const int a1 = (c1 >= 0 && c1 < n) ? ck_code(__ldg(pat + c1)) : CK_WL;
 #pragma unroll
-        for (int L = 0; L < 4; ++L) {
-            const int v0 = a0 == L ? sm : sx, v1 = a1 == L ? sm : sx;
-            prof[((pair * 4 + L) * (CT / 2) + h) * 32 + t] = ((uint32_t)v0 & 0xffffu) | ((uint32_t)v1 << 16);
+        for (int L = 0; L < CK_WL; ++L) {
+            prof[((pair * CK_WL + L) * (CT / 2) + h) * 32 + t] =
+                __byte_perm(a0 == L ? sm : sx, a1 == L ? sm : sx, 0x5410);
         }
     }
 }
@@ -743,7 +745,7 @@ __device__ void ck_item(const Sw16Args& A, const int32_t* __restrict__ pwork, in
         }
         // the groups' left boundaries per tile row (column edges at TW * tile),
         // combined and biased into shared memory: edg[(group * CK_K + row) * 2]
-        uint32_t* edg = prof + 2 * 4 * (CT / 2) * 32;
+        uint32_t* edg = prof + 2 * CK_WL * (CT / 2) * 32;
         for (int idx = t; idx < TG * CK_K; idx += 32) {
             const int gg = idx / CK_K, r = idx - gg * CK_K;
             const int ka = tb[0] - (TG - 1) + gg, kb = tb[1] - (TG - 1) + gg;
@@ -769,8 +771,8 @@ __device__ void ck_item(const Sw16Args& A, const int32_t* __restrict__ pwork, in
         // interleave.
         uint32_t ch0 = 0, ch1 = 0, rb_ch0 = 0, rb_ch1 = 0;
         uint32_t out_hg1 = B2 - GO2, out_e1 = B2;
-        const uint32_t* pA0 = prof + (0 * 4 * (CT / 2)) * 32 + t;
-        const uint32_t* pB0 = prof + (1 * 4 * (CT / 2)) * 32 + t;
+        const uint32_t* pA0 = prof + t;
+        const uint32_t* pB0 = prof + (CK_WL * (CT / 2)) * 32 + t;
         uint32_t* hrow = Ht + g * TW + CT * tl;                         // + (row - 1) * WCOL
         const int steps2 = (R + 1) / 2 + LG - 1;
         for (int tau = 0; tau < steps2; ++tau) {
@@ -1208,6 +1210,8 @@ static size_t sw16ck_smem() { return (size_t)4 * CK_WARP_WORDS * sizeof(uint32_t
 
 int sw16so_max_slots(int sm_count)
 {
+    // both variants launch with this shared memory: raise both limits
+    blocks_per_sm((const void*)sw16so_kernel<true>, 128, sw16ck_smem());
     return blocks_per_sm((const void*)sw16so_kernel<false>, 128, sw16ck_smem()) * sm_count * 4;
 }
 
@@ -1222,11 +1226,19 @@ cudaError_t launch_sw16so(const Sw16Args& A, int slots, cudaStream_t st)
     return cudaGetLastError();
 }
 
+template <int TG>
+static int ck_per_sm()
+{
+    // every variant launches with this shared memory: raise all limits
+    blocks_per_sm((const void*)sw16ck_kernel<TG, false, false>, 128, sw16ck_smem());
+    blocks_per_sm((const void*)sw16ck_kernel<TG, false, true>, 128, sw16ck_smem());
+    blocks_per_sm((const void*)sw16ck_kernel<TG, true, true>, 128, sw16ck_smem());
+    return blocks_per_sm((const void*)sw16ck_kernel<TG, true, false>, 128, sw16ck_smem());
+}
+
 int sw16ck_max_slots(int sm_count, int window)
 {
-    const int per_sm = window == 4 ? blocks_per_sm((const void*)sw16ck_kernel<4, true, false>, 128, sw16ck_smem())
-                                   : blocks_per_sm((const void*)sw16ck_kernel<2, true, false>, 128, sw16ck_smem());
-    return per_sm * sm_count * 4;
+    return (window == 4 ? ck_per_sm<4>() : ck_per_sm<2>()) * sm_count * 4;
 }
 
 cudaError_t launch_sw16ck(const Sw16Args& A, int slots, int window, bool blocks, cudaStream_t st)

@@ -296,7 +296,7 @@ __device__ void c32_pair(const SwArgs& A, int p, bool coop, int wib, int t, uint
         }
         return;
     }
-    const bool pure = A.D.pure && A.D.pure[p] && A.D.pure[A.D.n + p];
+    const bool pure = A.D.pure && A.D.pure[p] == 1 && A.D.pure[A.D.n + p] == 1;
     // tiles reach up to a multiple of TW: checkpoint rows are that wide (the
     // columns past the forward bands are padding, never read into a real cell)
     const int ncol = c32_ncol(n);

@@ -1,7 +1,7 @@
 // sw_plan.cu -- the Smith-Waterman traceback work plan, built on the device.
 //
 // The plan sorts the pairs of a batch into the kernels' work lists, largest
-// first: the two-pairs-per-warp 16-bit list (pure-ACGT pairs whose scores fit
+// first: the two-pairs-per-warp 16-bit list (A, C, G, T, N pairs whose scores fit
 // 16 bits; consecutive entries share a warp) and the 32-bit lists (short and
 // long shapes of sw32ck.cu).  It is a counting sort on a size key (16-bit
 // pairs: forward column extent, then rows; 32-bit pairs: 64 buckets per

@@ -10,7 +10,7 @@ namespace ga {
 
 // ---- 16-bit two-pairs-per-warp kernels --------------------------------------
 // Every value is stored as value + BIAS16 so each 16-bit half stays in
-// [0, 32767].  A pair qualifies when both sides are pure ACGT and
+// [0, 32767].  A pair qualifies when both sides hold only A, C, G, T and N and
 // match * min(m, n) + BIAS16 + gap_open < 32000, gap_open + gap_extend < BIAS16
 // and mismatch + gap_open >= 0 (host-side check; purity comes from the device).
 constexpr int BIAS16 = 1024;

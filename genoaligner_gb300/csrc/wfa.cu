@@ -57,13 +57,6 @@ __global__ void __launch_bounds__(256) pack_chunks_kernel(const uint8_t* __restr
     }
 }
 
-// 1 when byte c is one of A, C, G, T.
-__device__ __forceinline__ uint32_t acgt_byte(uint32_t c)
-{
-    // 'A'=0x41 'C'=0x43 'G'=0x47 'T'=0x54: all in 0x40..0x5f; low 5 bits 1, 3, 7, 20
-    return ((c >> 5) == 2u) & ((0x0010008au >> (c & 31u)) & 1u);
-}
-
 // Purity flag per sequence (a-sides q < n, then b-sides) from the per-chunk
 // masks of pack_chunks_kernel: bit b of bad[c] = byte 32c + b is not A/C/G/T.
 __global__ void __launch_bounds__(256) purity_mask_kernel(PairDesc D, const uint32_t* __restrict__ bad,
@@ -82,24 +75,43 @@ __global__ void __launch_bounds__(256) purity_mask_kernel(PairDesc D, const uint
     }
 }
 
-// Purity flag per sequence straight from the bytes, one thread each (the
-// Smith-Waterman paths, which read bytes and build no 2-bit arena).
+// Letters of each sequence straight from the bytes (the Smith-Waterman paths,
+// which build no 2-bit arena): 1 every byte is A, C, G or T; 2 some are N; 0
+// some are neither.  A warp per sequence, 512 bytes a step: the loads of a
+// sequence are contiguous, and a sequence takes length / 512 steps where a
+// thread took length / 16 (600 pairs up to 1 kb: 31 -> 7.5 us; 200,000 uneven
+// pairs, 260 MB: 226 -> 154 us, bound by the latency of the few loads a warp has
+// in flight).
 __global__ void __launch_bounds__(256) purity_kernel(PairDesc D, uint8_t* __restrict__ pure)
 {
-    for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < 2 * D.n; q += gridDim.x * blockDim.x) {
+    const int lane = threadIdx.x & 31;
+    const int nw = (gridDim.x * blockDim.x) >> 5;
+    for (int q = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; q < 2 * D.n; q += nw) {
         const bool is_a = q < D.n;
         const int p = is_a ? q : q - D.n;
         const uint8_t* s = D.seq + (is_a ? D.a_off[p] : D.b_off[p]);
         const int len = is_a ? D.a_len[p] : D.b_len[p];
-        uint32_t ok = 1;
-        for (int o = 0; o < len && ok; o += 16) {
+        uint32_t other = 0, n_seen = 0;                 // bits 0, 8, 16, 24: a byte outside ACGT; an N
+        for (int o = 16 * lane; o < len; o += 512) {
             const uint4 v = __ldg(reinterpret_cast<const uint4*>(s + o));
             const uint32_t w[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
-            for (int b = 0; b < 16; ++b)
-                if (o + b < len) ok &= acgt_byte((w[b >> 2] >> (8 * (b & 3))) & 0xffu);
+            for (int k = 0; k < 4; ++k) {
+                const int left = len - o - 4 * k;       // bytes of this word inside the sequence
+                if (left <= 0) break;
+                const uint32_t in = left >= 4 ? 0x01010101u : 0x01010101u >> (8 * (4 - left));
+                // a byte is A, C, G or T iff it equals "ACGT"[its code]
+                const uint32_t codes = ((w[k] >> 1) ^ (w[k] >> 2)) & 0x03030303u;
+                const uint32_t sel = (codes & 3u) | ((codes >> 4) & 0x30u) | ((codes >> 8) & 0x300u) | ((codes >> 12) & 0x3000u);
+                const uint32_t da = __byte_perm(0x54474341u, 0u, sel) ^ w[k], dn = w[k] ^ 0x4e4e4e4eu;
+                const uint32_t not_a = ((((da & 0x7f7f7f7fu) + 0x7f7f7f7fu) | da) >> 7) & in;
+                const uint32_t not_n = ((((dn & 0x7f7f7f7fu) + 0x7f7f7f7fu) | dn) >> 7) & in;
+                other |= not_a & not_n;
+                n_seen |= not_a & ~not_n;
+            }
         }
-        pure[q] = (uint8_t)ok;
+        const bool bad = __any_sync(FULL, other != 0), some_n = __any_sync(FULL, n_seen != 0);
+        if (lane == 0) pure[q] = bad ? 0 : (some_n ? 2 : 1);
     }
 }
 
@@ -285,6 +297,7 @@ cudaError_t launch_pack(const PairDesc& D, int64_t seq_bytes, uint64_t* packed, 
         return cudaGetLastError();
     }
     launch_begin(K_PACK, st);
+    blocks = (int)std::min<int64_t>(((int64_t)2 * D.n + 7) / 8, (int64_t)device_sms() * 32);      // a warp per sequence
     purity_kernel<<<blocks, 256, 0, st>>>(D, pure);
     launch_end(K_PACK, st);
     return cudaGetLastError();

@@ -14,14 +14,14 @@
 //     so long and short pairs balance across the grid;
 //   * the diagonals of wavefront s are spread over the 32 lanes; the previous
 //     and current wavefront live in a per-warp shared-memory ping-pong;
-//   * extension compares 32 bases per step on the 2-bit arena (XOR +
+//   * extension compares 16 bases per step on the 2-bit arena (XOR +
 //     find-first-set); pairs with any byte outside ACGT compare 8 raw bytes
 //     per step instead, so byte-equality semantics hold for N, lowercase, etc.;
 //   * for CIGARs every wavefront is also written to a per-warp triangular stack
 //     in global memory (wavefront s at s*s, 2s+1 entries); the walk then runs
 //     warp-uniformly over it and writes the CIGAR back to front into the
 //     pair's output slot, runs of matches written by all lanes at once.
-#include "kernels.cuh"
+#include "wfa_step.cuh"
 
 namespace ga {
 
@@ -116,115 +116,19 @@ __global__ void __launch_bounds__(256) purity_kernel(PairDesc D, uint8_t* __rest
 }
 
 // ------------------------------------------------------------------- WFA --
-// Cooperative emission of a run of `len` copies of `c` ending just before
-// slot[pos]; returns the new (lower) position.
-__device__ __forceinline__ int emit_run(char* slot, int pos, int len, char c, int lane, int* err)
-{
-    if (len <= 0) return pos;
-    if (len > pos) {
-        if (lane == 0) atomicOr(err, ERR_CIGAR_OVERFLOW);
-        len = pos;
-    }
-    for (int q = lane; q < len; q += 32) slot[pos - len + q] = c;
-    return pos - len;
-}
-
 template <bool TRACE, int BITS>
-__device__ void wfa_pair(const WfaArgs& A, int p, const uint64_t* __restrict__ P,
-                         const uint64_t* __restrict__ T, int m, int n, int32_t* wf0, int32_t* wf1,
-                         int32_t* stk, int lane)
+__device__ void wfa_pair(const WfaArgs& A, int p, const uint64_t* __restrict__ P, const uint64_t* __restrict__ T, int m,
+                         int n, int32_t* wf0, int32_t* wf1, int32_t* stk, int lane)
 {
-    const int smax = A.smax;
-    const int WS = 2 * smax + 3;
-    const int base = smax + 1;                 // slot of diagonal 0
-    for (int t = lane; t < WS; t += 32) { wf0[t] = WFA_NULL; wf1[t] = WFA_NULL; }
-    const int off0 = match_run<BITS>(P, T, 0, 0, m, n);   // computed redundantly by every lane
-    __syncwarp();
-    if (lane == 0) {
-        wf0[base] = off0;
-        if (TRACE) stk[0] = off0;
-    }
-    const int kfinal = n - m;
-    int score = -1;
-    if (kfinal == 0 && off0 >= n) {
-        score = 0;
-    } else {
-        int32_t* prev = wf0;
-        int32_t* cur = wf1;
-        for (int s = 1; s <= smax; ++s) {
-            __syncwarp();
-            for (int k = lane - s; k <= s; k += 32) {
-                const int ins = prev[base + k - 1];
-                const int del = prev[base + k + 1];
-                const int mis = prev[base + k];
-                int x = max(del, max(ins, mis) + 1);
-                if (!wfa_live(x) || x > n || x - k > m) x = WFA_NULL;
-                else x += match_run<BITS>(P, T, x - k, x, m, n);
-                cur[base + k] = x;
-                if (TRACE) stk[s * s + s + k] = x;
-            }
-            __syncwarp();
-            if (kfinal >= -s && kfinal <= s) {
-                const int fo = cur[base + kfinal];
-                if (wfa_live(fo) && fo >= n) { score = s; break; }
-            }
-            int32_t* t = prev; prev = cur; cur = t;
-        }
-    }
-    if (!TRACE || score < 0) {
-        if (lane == 0) {
-            A.out_score[p] = score;
-            if (A.out_len) A.out_len[p] = 0;
-        }
-        return;
-    }
-    char* slot = A.out_cigar + A.D.out_off[p];
-    int pos = m + n;
-    if (score == 0) {
-        pos = emit_run(slot, pos, n, 'M', lane, A.err);
-    } else {
+    const int score = wfa_forward<TRACE, BITS, 32>(P, T, m, n, A.smax, wf0, wf1, stk, lane, FULL);
+    int len = 0;
+    if (TRACE && score >= 0) {
         __syncwarp();                      // stack writes of every lane are visible below
-        int s = score, k = kfinal;
-        int off = stk[s * s + s + k];
-        int h = off, v = off - k;
-        pos = emit_run(slot, pos, v - m, 'D', lane, A.err);
-        pos = emit_run(slot, pos, h - n, 'I', lane, A.err);
-        v = min(v, m);
-        h = min(h, n);
-        while (v > 0 && h > 0 && s > 0) {
-            const int sp = s - 1;
-            const int32_t* W = stk + sp * sp + sp;     // W[k] = offset of diagonal k at score sp
-            const int c_mis = (k >= -sp && k <= sp) ? W[k] + 1 : WFA_NULL;
-            const int c_ins = (k - 1 >= -sp && k - 1 <= sp) ? W[k - 1] + 1 : WFA_NULL;
-            const int c_del = (k + 1 >= -sp && k + 1 <= sp) ? W[k + 1] : WFA_NULL;
-            int best = WFA_NULL;
-            char op = 0;
-            if (wfa_live(c_mis) && c_mis >= best) { best = c_mis; op = 'X'; }
-            if (wfa_live(c_ins) && c_ins > best)  { best = c_ins; op = 'I'; }
-            if (wfa_live(c_del) && c_del > best)  { best = c_del; op = 'D'; }
-            if (!op) break;
-            pos = emit_run(slot, pos, off - best, 'M', lane, A.err);
-            pos = emit_run(slot, pos, 1, op, lane, A.err);
-            off = best;
-            if (op == 'X')      { off -= 1; }
-            else if (op == 'I') { k -= 1; off -= 1; }
-            else                { k += 1; }
-            h = off;
-            v = off - k;
-            --s;
-        }
-        if (v > 0 && h > 0) {
-            const int run = min(v, h);
-            pos = emit_run(slot, pos, run, 'M', lane, A.err);
-            v -= run;
-            h -= run;
-        }
-        pos = emit_run(slot, pos, v, 'D', lane, A.err);
-        pos = emit_run(slot, pos, h, 'I', lane, A.err);
+        len = m + n - walk_g<32>(A, p, score, n - m, m, n, stk, lane, FULL);
     }
     if (lane == 0) {
         A.out_score[p] = score;
-        A.out_len[p] = m + n - pos;
+        if (A.out_len) A.out_len[p] = len;
     }
 }
 
@@ -254,7 +158,8 @@ __global__ void __launch_bounds__(128) wfa_kernel(WfaArgs A)
             // the CIGAR is all insertions (empty pattern) or all deletions
             // (wfa_kernel.hip:480-502)
             const int len = m <= 0 ? max(n, 0) : m;
-            if (TRACE) emit_run(A.out_cigar + A.D.out_off[p], len, len, m <= 0 ? 'I' : 'D', lane, A.err);
+            if (TRACE) emit_run_g<32>(A.out_cigar + A.D.out_off[p], len, len, m <= 0 ? 'I' : 'D',
+                                      m <= 0 ? 'I' : 'D', lane, A.err);
             if (lane == 0) {
                 A.out_score[p] = len;
                 if (A.out_len) A.out_len[p] = TRACE ? len : 0;

@@ -32,7 +32,7 @@
 // same for every smax >= s, so a pair resolved at any smax >= d returns the
 // reference's score and CIGAR.  All counts live in device memory, so the
 // whole sequence of launches is a fixed graph.
-#include "kernels.cuh"
+#include "wfa_step.cuh"
 #include "route.cuh"
 
 namespace ga {
@@ -55,26 +55,6 @@ constexpr int LANE_NULL = -16384;
 // a warp's pairs are still unresolved, they move to the warp queue.
 constexpr int LANE_HAND_S = 6;
 constexpr int LANE_HAND_DIV = 16;
-
-template <int G>
-__device__ __forceinline__ void gsync(unsigned gmask)
-{
-    if (G == 128) __syncthreads();
-    else if (G == 32) __syncwarp();
-    else __syncwarp(gmask);
-}
-
-template <int G>
-__device__ __forceinline__ int emit_run_g(char* slot, int pos, int len, char c, int gl, int* err)
-{
-    if (len <= 0) return pos;
-    if (len > pos) {
-        if (gl == 0) atomicOr(err, ERR_CIGAR_OVERFLOW);
-        len = pos;
-    }
-    for (int q = gl; q < len; q += G) slot[pos - len + q] = c;
-    return pos - len;
-}
 
 // ------------------------------------------------------------ lane queue --
 // One lane writes ops [pos - len, pos) of its own slot: bytes up to a 4-byte
@@ -270,60 +250,6 @@ __device__ void lane_phase(const RoutedArgs& R, uint32_t* smem, uint16_t* rec, i
     }
 }
 
-// The walk of a resolved pair (score >= 0) on the G lanes of its group, from
-// the wavefront stack the forward pass left (stk[s * s + s + k]: wavefront s
-// at diagonal k), written backwards from the end of the pair's CIGAR slot.
-// Every lane of the group runs the same walk; the runs are written by all of
-// them.  Returns the position of the CIGAR's first op in the slot.
-template <int G>
-__device__ int walk_g(const WfaArgs& A, int p, int score, int kfinal, int m, int n, const int32_t* stk, int gl)
-{
-    char* slot = A.out_cigar + A.D.out_off[p];
-    int pos = m + n;
-    if (score == 0) {
-        pos = emit_run_g<G>(slot, pos, n, 'M', gl, A.err);
-    } else {
-        int s = score, k = kfinal;
-        int off = stk[s * s + s + k];
-        int h = off, v = off - k;
-        pos = emit_run_g<G>(slot, pos, v - m, 'D', gl, A.err);
-        pos = emit_run_g<G>(slot, pos, h - n, 'I', gl, A.err);
-        v = min(v, m);
-        h = min(h, n);
-        while (v > 0 && h > 0 && s > 0) {
-            const int sp = s - 1;
-            const int32_t* W = stk + sp * sp + sp;
-            const int c_mis = (k >= -sp && k <= sp) ? W[k] + 1 : WFA_NULL;
-            const int c_ins = (k - 1 >= -sp && k - 1 <= sp) ? W[k - 1] + 1 : WFA_NULL;
-            const int c_del = (k + 1 >= -sp && k + 1 <= sp) ? W[k + 1] : WFA_NULL;
-            int best = WFA_NULL;
-            char op = 0;
-            if (wfa_live(c_mis) && c_mis >= best) { best = c_mis; op = 'X'; }
-            if (wfa_live(c_ins) && c_ins > best)  { best = c_ins; op = 'I'; }
-            if (wfa_live(c_del) && c_del > best)  { best = c_del; op = 'D'; }
-            if (!op) break;
-            pos = emit_run_g<G>(slot, pos, off - best, 'M', gl, A.err);
-            pos = emit_run_g<G>(slot, pos, 1, op, gl, A.err);
-            off = best;
-            if (op == 'X')      { off -= 1; }
-            else if (op == 'I') { k -= 1; off -= 1; }
-            else                { k += 1; }
-            h = off;
-            v = off - k;
-            --s;
-        }
-        if (v > 0 && h > 0) {
-            const int run = min(v, h);
-            pos = emit_run_g<G>(slot, pos, run, 'M', gl, A.err);
-            v -= run;
-            h -= run;
-        }
-        pos = emit_run_g<G>(slot, pos, v, 'D', gl, A.err);
-        pos = emit_run_g<G>(slot, pos, h, 'I', gl, A.err);
-    }
-    return pos;
-}
-
 // One pair on a group of G lanes with the given smax.  Returns the score
 // (-1 when unresolved within smax); writes the outputs only when the pair is
 // resolved or `final`.
@@ -333,55 +259,17 @@ __device__ int wfa_pair_g(const RoutedArgs& R, int p, int smax, bool final, cons
                           int gl, unsigned gmask)
 {
     const WfaArgs& A = R.A;
-    const int WS = 2 * smax + 3;
-    const int base = smax + 1;
-    for (int t = gl; t < WS; t += G) { wf0[t] = WFA_NULL; wf1[t] = WFA_NULL; }
-    const int off0 = match_run<BITS>(P, T, 0, 0, m, n);
-    gsync<G>(gmask);
-    if (gl == 0) {
-        wf0[base] = off0;
-        if (TRACE) stk[0] = off0;
-    }
-    const int kfinal = n - m;
-    int score = -1;
-    if (kfinal == 0 && off0 >= n) {
-        score = 0;
-    } else if (kfinal >= -smax && kfinal <= smax) {
-        int32_t* prev = wf0;
-        int32_t* cur = wf1;
-        for (int s = 1; s <= smax; ++s) {
-            gsync<G>(gmask);
-            for (int k = gl - s; k <= s; k += G) {
-                const int ins = prev[base + k - 1];
-                const int del = prev[base + k + 1];
-                const int mis = prev[base + k];
-                int x = max(del, max(ins, mis) + 1);
-                if (!wfa_live(x) || x > n || x - k > m) x = WFA_NULL;
-                else x += match_run<BITS>(P, T, x - k, x, m, n);
-                cur[base + k] = x;
-                if (TRACE) stk[s * s + s + k] = x;
-            }
-            gsync<G>(gmask);
-            if (kfinal >= -s && kfinal <= s) {
-                const int fo = cur[base + kfinal];
-                if (wfa_live(fo) && fo >= n) { score = s; break; }
-            }
-            int32_t* t = prev; prev = cur; cur = t;
-        }
-    }
+    const int score = wfa_forward<TRACE, BITS, G>(P, T, m, n, smax, wf0, wf1, stk, gl, gmask);
     if (score < 0 && !final) return score;
-    if (!TRACE || score < 0) {
-        if (gl == 0) {
-            A.out_score[p] = score;
-            if (A.out_len) A.out_len[p] = 0;
-        }
-        return score;
+    int len = 0;
+    if (TRACE && score >= 0) {
+        gsync<G>(gmask);
+        if constexpr (G <= 32) len = m + n - walk_g<G>(A, p, score, n - m, m, n, stk, gl, gmask);
+        else if (gl < 32) len = m + n - walk_g<32>(A, p, score, n - m, m, n, stk, gl, FULL);
     }
-    if (score > 0) gsync<G>(gmask);
-    const int pos = walk_g<G>(A, p, score, n - m, m, n, stk, gl);
     if (gl == 0) {
         A.out_score[p] = score;
-        A.out_len[p] = m + n - pos;
+        if (A.out_len) A.out_len[p] = len;
     }
     return score;
 }
@@ -395,7 +283,8 @@ __device__ void run_item(const RoutedArgs& R, int2 item, int32_t* wf0, int32_t* 
     const int m = A.D.a_len[p], n = A.D.b_len[p];
     if (m <= 0 || n <= 0) {
         const int len = m <= 0 ? max(n, 0) : m;
-        if (TRACE) emit_run_g<G>(A.out_cigar + A.D.out_off[p], len, len, m <= 0 ? 'I' : 'D', gl, A.err);
+        if (TRACE) emit_run_g<G>(A.out_cigar + A.D.out_off[p], len, len, m <= 0 ? 'I' : 'D', m <= 0 ? 'I' : 'D',
+                                              gl, A.err);
         if (gl == 0) {
             A.out_score[p] = len;
             if (A.out_len) A.out_len[p] = TRACE ? len : 0;
@@ -435,8 +324,9 @@ __device__ void group_phase(const RoutedArgs& R, const int2* __restrict__ items,
     constexpr int NG = 32 / G;
     const WfaArgs& A = R.A;
     const int grp = lane / G, gl = lane % G;
+    const unsigned gmask = (0xffffffffu >> (32 - G)) << (grp * G);
     const int smax = A.smax;
-    const int WS = 2 * smax + 3, base = smax + 1;
+    const int WS = 2 * smax + 3;
     int32_t* const wfa = wsm + grp * 2 * WS;
     int32_t* const wfb = wfa + WS;
     int32_t* const stk = TRACE ? wstk + grp * (int64_t)(smax + 1) * (smax + 1) : nullptr;
@@ -454,7 +344,8 @@ __device__ void group_phase(const RoutedArgs& R, const int2* __restrict__ items,
             n = A.D.b_len[p];
             if (m <= 0 || n <= 0) {
                 const int len = m <= 0 ? max(n, 0) : m;
-                if (TRACE) emit_run_g<G>(A.out_cigar + A.D.out_off[p], len, len, m <= 0 ? 'I' : 'D', gl, A.err);
+                if (TRACE) emit_run_g<G>(A.out_cigar + A.D.out_off[p], len, len, m <= 0 ? 'I' : 'D', m <= 0 ? 'I' : 'D',
+                                              gl, A.err);
                 if (gl == 0) {
                     A.out_score[p] = len;
                     if (A.out_len) A.out_len[p] = TRACE ? len : 0;
@@ -472,43 +363,36 @@ __device__ void group_phase(const RoutedArgs& R, const int2* __restrict__ items,
         }
         for (int t = gl; t < WS; t += G) { wfa[t] = WFA_NULL; wfb[t] = WFA_NULL; }
         int off0 = 0;
-        if (have) off0 = packed ? match_run<2>(P, T, 0, 0, m, n) : match_run<8>(P, T, 0, 0, m, n);
+        if (have) off0 = packed ? extend_run<2>(P, T, 0, 0, m, n) : extend_run<8>(P, T, 0, 0, m, n);
         __syncwarp();
+        int32_t* prev = wfa + smax + 1;                    // diagonal 0
+        int32_t* cur = wfb + smax + 1;
         if (have && gl == 0) {
-            wfa[base] = off0;
+            prev[0] = off0;
             if (TRACE) stk[0] = off0;
         }
         const int kfinal = n - m;
         int score = -1;
         bool act = have && kfinal >= -smax && kfinal <= smax;
         if (have && kfinal == 0 && off0 >= n) { score = 0; act = false; }
-        int32_t* prev = wfa;
-        int32_t* cur = wfb;
+        __syncwarp();
         for (int s = 1; s <= smax; ++s) {
             if (!__any_sync(FULL, act)) break;
-            __syncwarp();
             if (act) {
-                for (int k = gl - s; k <= s; k += G) {
-                    const int ins = prev[base + k - 1];
-                    const int del = prev[base + k + 1];
-                    const int mis = prev[base + k];
-                    int x = max(del, max(ins, mis) + 1);
-                    if (!wfa_live(x) || x > n || x - k > m) x = WFA_NULL;
-                    else x += packed ? match_run<2>(P, T, x - k, x, m, n) : match_run<8>(P, T, x - k, x, m, n);
-                    cur[base + k] = x;
+                const int hi = wave_hi(s, n, kfinal, smax);
+                for (int k = wave_lo(s, m, kfinal, smax) + gl; k <= hi; k += G) {
+                    const int x = packed ? next_offset<2>(prev, k, P, T, m, n) : next_offset<8>(prev, k, P, T, m, n);
+                    cur[k] = x;
                     if (TRACE) stk[s * s + s + k] = x;
                 }
             }
             __syncwarp();
-            if (act && kfinal >= -s && kfinal <= s) {
-                const int fo = cur[base + kfinal];
-                if (wfa_live(fo) && fo >= n) { score = s; act = false; }
-            }
+            if (act && cur[kfinal] >= n) { score = s; act = false; }
             int32_t* t = prev; prev = cur; cur = t;
         }
         if (have) {
             int len = 0;
-            if (TRACE && score >= 0) len = m + n - walk_g<G>(A, p, score, kfinal, m, n, stk, gl);
+            if (TRACE && score >= 0) len = m + n - walk_g<G>(A, p, score, kfinal, m, n, stk, gl, gmask);
             if (gl == 0) {
                 A.out_score[p] = score;
                 if (A.out_len) A.out_len[p] = len;

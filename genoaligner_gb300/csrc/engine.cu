@@ -625,29 +625,48 @@ struct WfaScratch {
     int slots = 0;                   // warp slots of the WFA (or warp-queue) kernel
     int lane_slots = 0;              // learned: warp slots of the lane kernel
     int64_t stack_slot = 0;
+    int cap = 0;                     // edits the warp kernels search; the pairs left below smax go to the block kernel
+    int blocks = 0;                  // blocks of the block kernel (0: not launched)
+    int32_t* blk = nullptr;          // the pairs left to it
+    int smax = 0;
     int warp_smem = 0;
     int group = 32;                  // learned: lanes per warp-queue pair
     int64_t seq_bytes = 0;
     int chunk = 1;
 };
 
+// Edits the warp kernels search before a pair moves to a whole block
+// (wfa_block.cu).  Their shared memory and stacks are sized for it: at 511, 27
+// warps of 8 KB share an SM where 4 fitted at smax 2048.  The learned path sends
+// pairs estimated at 256 edits and more to blocks at once; the plain path, which
+// knows nothing of a pair, restarts the ones past 255 there (a 64th of the work
+// of a pair at 2048).
+constexpr int WFA_WARP_CAP = 511, WFA_PLAIN_CAP = 255;
+// Below this no pair is estimated at the block kernel's distances.
+constexpr int WFA_BLOCK_MIN = 256;
+
 // group: the tuned lanes per warp-queue pair (ga_tune.wfa_group).
 static void size_wfa(WfaScratch& S, int n, int smax, bool trace, bool learned, int sm_count, int group)
 {
+    S.smax = smax;
+    S.cap = smax <= WFA_WARP_CAP ? smax : (learned ? WFA_WARP_CAP : WFA_PLAIN_CAP);
+    const bool blocks = S.cap < smax || (learned && smax >= WFA_BLOCK_MIN);
     if (learned) {
         prepare_mlp();
         S.group = routed_group(smax, group);
-        S.slots = (int)std::min<int64_t>(routed_max_slots(smax, trace, sm_count, S.group), ((int64_t)n + 3) / 4 * 4);
+        S.slots = (int)std::min<int64_t>(routed_max_slots(S.cap, trace, sm_count, S.group), ((int64_t)n + 3) / 4 * 4);
         S.lane_slots = (int)std::min<int64_t>(lane_max_slots(trace, sm_count), ((int64_t)n + 127) / 128 * 4);
-        S.stack_slot = routed_stack_slot(smax, S.group);
-        S.warp_smem = routed_warp_smem(smax, S.group);
+        S.stack_slot = routed_stack_slot(S.cap, S.group);
+        S.warp_smem = routed_warp_smem(S.cap, S.group);
     } else {
-        S.slots = (int)std::min<int64_t>(wfa_max_slots(smax, trace, sm_count), ((int64_t)n + 3) / 4 * 4);
-        S.stack_slot = (int64_t)(smax + 1) * (smax + 1);
+        S.slots = (int)std::min<int64_t>(wfa_max_slots(S.cap, trace, sm_count), ((int64_t)n + 3) / 4 * 4);
+        S.stack_slot = (int64_t)(S.cap + 1) * (S.cap + 1);
     }
+    if (blocks) S.blocks = std::min(wfa_block_slots(smax, trace, sm_count), std::max(n, 1));
     if (trace) {
         const int64_t budget = (int64_t)16 << 30;     // stack memory cap
         S.slots = (int)std::min<int64_t>(S.slots, std::max<int64_t>(4, budget / (S.stack_slot * 4) / 4 * 4));
+        S.blocks = (int)std::min<int64_t>(S.blocks, std::max<int64_t>(1, budget / ((int64_t)(smax + 1) * (smax + 1) * 4)));
     }
     // pairs per counter increment: keep >= 8 grabs per warp
     S.chunk = (int)std::max<int64_t>(1, std::min<int64_t>(16, (int64_t)n / ((int64_t)S.slots * 8)));
@@ -659,7 +678,11 @@ static void carve_wfa(Carve& k, WfaScratch& S, int n, int64_t arena, bool trace,
     S.packed = k.take<uint64_t>(packed_arena_words(arena));
     S.pure = k.take<uint8_t>(2 * (size_t)n);
     S.ctr = k.take<int32_t>(64, 256);
-    S.stack = trace ? k.take<int32_t>((size_t)S.slots * S.stack_slot) : nullptr;
+    // the warp kernels and the block kernel run one after the other and share the stacks
+    S.stack = trace ? k.take<int32_t>((size_t)std::max<int64_t>((int64_t)S.slots * S.stack_slot,
+                                                                (int64_t)S.blocks * (S.smax + 1) * (S.smax + 1)))
+                    : nullptr;
+    S.blk = k.take<int32_t>(S.blocks > 0 ? n : 0);
     if (learned) {
         S.item = k.take<int32_t>(n);
         S.lb = k.take<int32_t>(n);
@@ -685,10 +708,18 @@ static cudaError_t enqueue_wfa(const WfaScratch& S, PairDesc D, int smax, bool t
     A.out_score = score; A.out_len = len; A.out_cigar = cig;
     A.stack = S.stack; A.stack_slot = S.stack_slot; A.counter = S.ctr; A.err = err;
     A.chunk = S.chunk;
+    A.cap = S.cap; A.blk = S.blk; A.blk_count = S.ctr + 33;
+    WfaBlockArgs B;
+    B.A = A;
+    B.next = S.ctr + 3;
     cudaError_t e = cudaMemsetAsync(S.ctr, 0, 64 * sizeof(int32_t), st);
     if (e == cudaSuccess) e = launch_pack(D, S.seq_bytes, S.packed, S.pure, st);
     if (e != cudaSuccess) return e;
-    if (route == 0) return launch_wfa(A, S.slots, st);
+    if (route == 0) {
+        e = launch_wfa(A, S.slots, st);
+        if (e == cudaSuccess && S.blocks > 0) e = launch_wfa_block(B, S.blocks, trace ? K_WFA_TRACE : K_WFA_SCORE, st);
+        return e;
+    }
     const int NB = route_buckets();
     if ((e = cudaMemsetAsync(S.counts, 0, sizeof(int32_t) * (2 * NB + 4), st)) != cudaSuccess) return e;
     if ((e = launch_route_model(D, smax, lane_smax, route == 1, S.item, S.lb, S.y, S.counts, score, len, st)) !=
@@ -696,8 +727,9 @@ static cudaError_t enqueue_wfa(const WfaScratch& S, PairDesc D, int smax, bool t
         return e;
     if ((e = launch_route(D.n, S.item, S.counts, S.starts, S.big, S.small, st)) != cudaSuccess) return e;
     // ctr layout: [0] warp-queue next, [1] lane-queue next, [2] escalation
-    // next, [3] whole-block next, [32] escalation count; counts[2 NB + 2]:
-    // whole-block items (the warp queue's first ones)
+    // next, [3] whole-block next, [32] escalation count, [33] pairs left to
+    // whole blocks; counts[2 NB + 2]: whole-block items (the warp queue's first
+    // ones)
     RoutedArgs R;
     R.A = A;
     R.warp_smem = S.warp_smem;
@@ -712,9 +744,12 @@ static cudaError_t enqueue_wfa(const WfaScratch& S, PairDesc D, int smax, bool t
     R.esc_count = S.ctr + 32;
     R.esc_next = S.ctr + 2;
     R.lane_rec = S.lane_rec;
-    R.block_count = S.counts + 2 * NB + 2;
-    R.block_next = S.ctr + 3;
-    return launch_routed(R, S.lane_slots, S.slots, st);
+    R.block_count = S.blocks > 0 ? S.counts + 2 * NB + 2 : nullptr;
+    e = launch_routed(R, S.lane_slots, S.slots, st);
+    if (e != cudaSuccess || S.blocks == 0) return e;
+    B.big = S.big;
+    B.big_count = R.block_count;
+    return launch_wfa_block(B, S.blocks, K_WFA_ROUTED, st);
 }
 
 // Replays `exec` when `key` (everything the enqueued launches bake in) is the

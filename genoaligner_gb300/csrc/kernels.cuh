@@ -18,6 +18,12 @@ struct WfaArgs {
     int32_t* counter;        // next pair index
     int32_t* err;
     int32_t chunk = 1;       // pairs taken per counter increment
+    // The warp kernels search each pair up to `cap` edits (their wavefronts and
+    // stacks are sized for it); below smax, the pairs unresolved there are
+    // appended to blk[*blk_count] for the block kernel (wfa_block.cu).
+    int32_t cap;
+    int32_t* blk = nullptr;
+    int32_t* blk_count = nullptr;
 };
 
 struct SwArgs {
@@ -84,13 +90,23 @@ struct RoutedArgs {
     int2* esc;                   // escalations from the lane queue: (pair, batch smax)
     int32_t* esc_count;
     int32_t* esc_next;
-    const int32_t* block_count;  // the first *block_count warp-queue items run on whole blocks (null: none)
-    int32_t* block_next;
+    const int32_t* block_count;  // the first *block_count warp-queue items are the block kernel's (null: none)
     uint16_t* lane_rec;          // lane kernel: per warp slot, lane_rec_slot() walk records (trace only)
-    int32_t warp_smem;           // warp kernel: shared-memory ints per warp
+    int32_t warp_smem;           // warp kernel: shared-memory ints per warp, for A.cap
     int32_t group;               // warp kernel: lanes per warp-queue pair (8, 16 or 32; routed_group)
 };
 
+// Pairs on whole blocks (wfa_block.cu): the first *big_count of the warp queue
+// (null: none), then the warp kernels' unresolved ones (A.blk).  A.stack: per
+// block (A.smax + 1)^2 offsets.
+struct WfaBlockArgs {
+    WfaArgs A;
+    const int2* big = nullptr;
+    const int32_t* big_count = nullptr;
+    int32_t* next;
+};
+int wfa_block_slots(int smax, bool trace, int sm_count);
+cudaError_t launch_wfa_block(const WfaBlockArgs& B, int blocks, int kernel_id, cudaStream_t st);
 // Packs seq into the 2-bit arena `packed` (packed_arena_words(seq_bytes)
 // words; null: purity flags only) and sets pure[2n].
 cudaError_t launch_pack(const PairDesc& D, int64_t seq_bytes, uint64_t* packed, uint8_t* pure, cudaStream_t st);

@@ -162,7 +162,7 @@ extern "C" int32_t ga_wfa_device_noalloc(const ga_device_batch* b, int32_t smax,
     D.a_off = b->a_off; D.a_len = b->a_len; D.b_off = b->b_off; D.b_len = b->b_len;
     D.out_off = b->out_off; D.n = b->n;
     WfaArgs A;
-    A.D = D; A.smax = smax; A.trace = trace ? 1 : 0;
+    A.D = D; A.smax = smax; A.cap = smax; A.trace = trace ? 1 : 0;
     A.out_score = out_score; A.out_len = out_len; A.out_cigar = out_cigar;
     A.stack = stk; A.stack_slot = ((int64_t)smax + 1) * ((int64_t)smax + 1);
     A.counter = ctr; A.err = ctr + 1;

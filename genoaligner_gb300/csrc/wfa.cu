@@ -120,7 +120,11 @@ template <bool TRACE, int BITS>
 __device__ void wfa_pair(const WfaArgs& A, int p, const uint64_t* __restrict__ P, const uint64_t* __restrict__ T, int m,
                          int n, int32_t* wf0, int32_t* wf1, int32_t* stk, int lane)
 {
-    const int score = wfa_forward<TRACE, BITS, 32>(P, T, m, n, A.smax, wf0, wf1, stk, lane, FULL);
+    const int score = wfa_forward<TRACE, BITS, 32>(P, T, m, n, A.cap, wf0, wf1, stk, lane, FULL);
+    if (score < 0 && A.cap < A.smax) {                      // left to the block kernel
+        if (lane == 0) A.blk[atomicAdd(A.blk_count, 1)] = p;
+        return;
+    }
     int len = 0;
     if (TRACE && score >= 0) {
         __syncwarp();                      // stack writes of every lane are visible below
@@ -138,7 +142,7 @@ __global__ void __launch_bounds__(128) wfa_kernel(WfaArgs A)
     extern __shared__ int32_t smem[];
     const int lane = threadIdx.x & 31;
     const int wib = threadIdx.x >> 5;
-    const int WS = 2 * A.smax + 3;
+    const int WS = 2 * A.cap + 3;
     int32_t* wf0 = smem + wib * 2 * WS;
     int32_t* wf1 = wf0 + WS;
     const int64_t slot = (int64_t)blockIdx.x * (blockDim.x >> 5) + wib;
@@ -381,7 +385,7 @@ cudaError_t launch_wfa(const WfaArgs& A, int slots, cudaStream_t st)
 {
     if (A.D.n <= 0) return cudaSuccess;
     const int blocks = (slots + 3) / 4;
-    const size_t smem = wfa_smem_bytes(A.smax);
+    const size_t smem = wfa_smem_bytes(A.cap);
     const int id = A.trace ? K_WFA_TRACE : K_WFA_SCORE;
     launch_begin(id, st);
     if (A.trace) wfa_kernel<true><<<blocks, 128, smem, st>>>(A);

@@ -1,6 +1,6 @@
 // wfa_routed.cu -- the learned-bucketed WFA path: routing and two persistent
 // kernels over two bucketed queues, one served by single lanes, one by
-// groups of lanes, warps or whole blocks.
+// groups of lanes or warps (its largest items by whole blocks, wfa_block.cu).
 //
 // Same recurrence and walk as wfa.cu (the reference's wfa_trace_kernel,
 // include/genoaligner/backend/wfa_kernel.hip:119-145, 338-437); what changes is
@@ -18,7 +18,8 @@
 //     one pair per group of lanes (8 or 16 lanes, several pairs per warp
 //     stepping through their wavefronts together, at batch smax <= 128; else
 //     one pair per warp), lanes over the diagonals of a wavefront; items
-//     estimated at s >= 256 first on whole blocks;
+//     estimated at s >= 256, and those unresolved at WFA_WARP_CAP edits, on
+//     whole blocks;
 //   * the router sorts both queues, largest first -- the lane queue by first
 //     smax, the warp queue by the bit length of the estimate -- with a
 //     counting sort (bucket counts in the route pass, then a scan and a
@@ -250,60 +251,42 @@ __device__ void lane_phase(const RoutedArgs& R, uint32_t* smem, uint16_t* rec, i
     }
 }
 
-// One pair on a group of G lanes with the given smax.  Returns the score
-// (-1 when unresolved within smax); writes the outputs only when the pair is
-// resolved or `final`.
-template <bool TRACE, int BITS, int G>
-__device__ int wfa_pair_g(const RoutedArgs& R, int p, int smax, bool final, const uint64_t* __restrict__ P,
-                          const uint64_t* __restrict__ T, int m, int n, int32_t* wf0, int32_t* wf1, int32_t* stk,
-                          int gl, unsigned gmask)
+// One warp-queue item on a warp, searched up to A.cap edits; unresolved there
+// below the batch smax, it is the block kernel's.
+template <bool TRACE>
+__device__ void run_item(const WfaArgs& A, int p, int32_t* wf0, int32_t* wf1, int32_t* stk, int lane)
 {
-    const WfaArgs& A = R.A;
-    const int score = wfa_forward<TRACE, BITS, G>(P, T, m, n, smax, wf0, wf1, stk, gl, gmask);
-    if (score < 0 && !final) return score;
-    int len = 0;
-    if (TRACE && score >= 0) {
-        gsync<G>(gmask);
-        if constexpr (G <= 32) len = m + n - walk_g<G>(A, p, score, n - m, m, n, stk, gl, gmask);
-        else if (gl < 32) len = m + n - walk_g<32>(A, p, score, n - m, m, n, stk, gl, FULL);
-    }
-    if (gl == 0) {
-        A.out_score[p] = score;
-        if (A.out_len) A.out_len[p] = len;
-    }
-    return score;
-}
-
-template <bool TRACE, int G>
-__device__ void run_item(const RoutedArgs& R, int2 item, int32_t* wf0, int32_t* wf1, int32_t* stk, int gl,
-                         unsigned gmask)
-{
-    const WfaArgs& A = R.A;
-    const int p = item.x, smax = item.y;
     const int m = A.D.a_len[p], n = A.D.b_len[p];
     if (m <= 0 || n <= 0) {
         const int len = m <= 0 ? max(n, 0) : m;
-        if (TRACE) emit_run_g<G>(A.out_cigar + A.D.out_off[p], len, len, m <= 0 ? 'I' : 'D', m <= 0 ? 'I' : 'D',
-                                              gl, A.err);
-        if (gl == 0) {
+        const char op = m <= 0 ? 'I' : 'D';
+        if (TRACE) emit_run_g<32>(A.out_cigar + A.D.out_off[p], len, len, op, op, lane, A.err);
+        if (lane == 0) {
             A.out_score[p] = len;
             if (A.out_len) A.out_len[p] = TRACE ? len : 0;
         }
         return;
     }
-    const bool final = smax >= A.smax;
     int score;
-    if (A.D.pure[p] && A.D.pure[A.D.n + p]) {
-        score = wfa_pair_g<TRACE, 2, G>(R, p, smax, final, A.D.packed + (A.D.a_off[p] >> 5),
-                                        A.D.packed + (A.D.b_off[p] >> 5), m, n, wf0, wf1, stk, gl, gmask);
-    } else {
-        score = wfa_pair_g<TRACE, 8, G>(R, p, smax, final, reinterpret_cast<const uint64_t*>(A.D.seq + A.D.a_off[p]),
-                                        reinterpret_cast<const uint64_t*>(A.D.seq + A.D.b_off[p]), m, n, wf0, wf1,
-                                        stk, gl, gmask);
+    if (A.D.pure[p] && A.D.pure[A.D.n + p])
+        score = wfa_forward<TRACE, 2, 32>(A.D.packed + (A.D.a_off[p] >> 5), A.D.packed + (A.D.b_off[p] >> 5), m, n, A.cap,
+                                          wf0, wf1, stk, lane, FULL);
+    else
+        score = wfa_forward<TRACE, 8, 32>(reinterpret_cast<const uint64_t*>(A.D.seq + A.D.a_off[p]),
+                                          reinterpret_cast<const uint64_t*>(A.D.seq + A.D.b_off[p]), m, n, A.cap, wf0,
+                                          wf1, stk, lane, FULL);
+    if (score < 0 && A.cap < A.smax) {
+        if (lane == 0) A.blk[atomicAdd(A.blk_count, 1)] = p;
+        return;
     }
-    if (score < 0 && !final && gl == 0) {
-        const int q = atomicAdd(R.esc_count, 1);
-        R.esc[q] = make_int2(p, A.smax);
+    int len = 0;
+    if (TRACE && score >= 0) {
+        __syncwarp();
+        len = m + n - walk_g<32>(A, p, score, n - m, m, n, stk, lane, FULL);
+    }
+    if (lane == 0) {
+        A.out_score[p] = score;
+        if (A.out_len) A.out_len[p] = len;
     }
 }
 
@@ -415,53 +398,33 @@ __global__ void __launch_bounds__(128) wfa_lane_kernel(RoutedArgs R)
     lane_phase<TRACE>(R, lsmem + wib * LANE_WARP_SMEM, rec, lane);
 }
 
-// Warp queue (persistent): the routed pairs largest first, then the lane
-// queue's escalations, one pair per warp (G = 32) or per group of G lanes.
-// Every item runs with the batch smax and is final.
+// Warp queue (persistent): the routed pairs largest first (but for the block
+// kernel's), then the lane queue's escalations, one pair per warp (G = 32) or
+// per group of G lanes.
 template <bool TRACE, int G>
 __global__ void __launch_bounds__(128) wfa_routed_kernel(RoutedArgs R)
 {
     extern __shared__ __align__(16) int32_t rsmem[];
-    __shared__ int s_q;
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     int32_t* wsm = rsmem + wib * R.warp_smem;
     const int64_t slot = (int64_t)blockIdx.x * (blockDim.x >> 5) + wib;
     int32_t* stk = TRACE ? R.A.stack + slot * R.A.stack_slot : nullptr;
-    // the warp queue's largest items first, each on the whole block: its 128
-    // threads split the diagonals of every step (one block barrier a step),
-    // in warp 0's shared memory and stack
-    const int nblock = R.block_count ? *R.block_count : 0;
-    if (nblock > 0) {
-        int32_t* bstk = TRACE ? R.A.stack + (int64_t)blockIdx.x * (blockDim.x >> 5) * R.A.stack_slot : nullptr;
-        for (;;) {
-            if (threadIdx.x == 0) s_q = atomicAdd(R.block_next, 1);
-            __syncthreads();
-            const int q = s_q;
-            __syncthreads();
-            if (q >= nblock) break;
-            const int2 it = R.big[q];
-            run_item<TRACE, 128>(R, it, rsmem, rsmem + 2 * it.y + 3, bstk, threadIdx.x, FULL);
-            __syncthreads();
-        }
-    }
     for (int list = 0; list < 2; ++list) {
         const int2* items = list ? R.esc : R.big;
         const int cnt = list ? *R.esc_count : *R.big_count;
         int32_t* next = list ? R.esc_next : R.big_next;
-        const int first = list ? 0 : nblock;            // (items before it ran on blocks)
+        const int first = list || !R.block_count ? 0 : *R.block_count;
         if constexpr (G < 32) {
             group_phase<TRACE, G>(R, items, cnt, next, first, wsm, stk, lane);
-            __syncwarp();
-            continue;
-        }
-        for (;;) {
-            int q = 0;
-            if (lane == 0) q = atomicAdd(next, 1) + first;
-            q = __shfl_sync(FULL, q, 0);
-            if (q >= cnt) break;
-            __syncwarp();
-            const int2 it = items[q];
-            run_item<TRACE, 32>(R, it, wsm, wsm + 2 * it.y + 3, stk, lane, FULL);
+        } else {
+            for (;;) {
+                int q = 0;
+                if (lane == 0) q = atomicAdd(next, 1) + first;
+                q = __shfl_sync(FULL, q, 0);
+                if (q >= cnt) break;
+                __syncwarp();
+                run_item<TRACE>(R.A, items[q].x, wsm, wsm + 2 * R.A.cap + 3, stk, lane);
+            }
         }
         __syncwarp();
     }

@@ -732,6 +732,7 @@ static cudaError_t enqueue_wfa(const WfaScratch& S, PairDesc D, int smax, bool t
     // ones)
     RoutedArgs R;
     R.A = A;
+    R.ahead = D.n <= S.slots;                 // no more pairs than warps: bound by each pair's chain
     R.warp_smem = S.warp_smem;
     R.group = S.group;
     R.big = S.big;

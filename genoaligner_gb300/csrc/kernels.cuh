@@ -92,6 +92,7 @@ struct RoutedArgs {
     int32_t* esc_next;
     const int32_t* block_count;  // the first *block_count warp-queue items are the block kernel's (null: none)
     uint16_t* lane_rec;          // lane kernel: per warp slot, lane_rec_slot() walk records (trace only)
+    int32_t ahead;               // warp kernel: two diagonals a lane at once (wfa_forward)
     int32_t warp_smem;           // warp kernel: shared-memory ints per warp, for A.cap
     int32_t group;               // warp kernel: lanes per warp-queue pair (8, 16 or 32; routed_group)
 };

@@ -253,7 +253,7 @@ __device__ void lane_phase(const RoutedArgs& R, uint32_t* smem, uint16_t* rec, i
 
 // One warp-queue item on a warp, searched up to A.cap edits; unresolved there
 // below the batch smax, it is the block kernel's.
-template <bool TRACE>
+template <bool TRACE, bool AHEAD>
 __device__ void run_item(const WfaArgs& A, int p, int32_t* wf0, int32_t* wf1, int32_t* stk, int lane)
 {
     const int m = A.D.a_len[p], n = A.D.b_len[p];
@@ -269,8 +269,8 @@ __device__ void run_item(const WfaArgs& A, int p, int32_t* wf0, int32_t* wf1, in
     }
     int score;
     if (A.D.pure[p] && A.D.pure[A.D.n + p])
-        score = wfa_forward<TRACE, 2, 32>(A.D.packed + (A.D.a_off[p] >> 5), A.D.packed + (A.D.b_off[p] >> 5), m, n, A.cap,
-                                          wf0, wf1, stk, lane, FULL);
+        score = wfa_forward<TRACE, 2, 32, AHEAD>(A.D.packed + (A.D.a_off[p] >> 5), A.D.packed + (A.D.b_off[p] >> 5), m, n,
+                                                 A.cap, wf0, wf1, stk, lane, FULL);
     else
         score = wfa_forward<TRACE, 8, 32>(reinterpret_cast<const uint64_t*>(A.D.seq + A.D.a_off[p]),
                                           reinterpret_cast<const uint64_t*>(A.D.seq + A.D.b_off[p]), m, n, A.cap, wf0,
@@ -423,7 +423,8 @@ __global__ void __launch_bounds__(128) wfa_routed_kernel(RoutedArgs R)
                 q = __shfl_sync(FULL, q, 0);
                 if (q >= cnt) break;
                 __syncwarp();
-                run_item<TRACE>(R.A, items[q].x, wsm, wsm + 2 * R.A.cap + 3, stk, lane);
+                if (R.ahead) run_item<TRACE, true>(R.A, items[q].x, wsm, wsm + 2 * R.A.cap + 3, stk, lane);
+                else run_item<TRACE, false>(R.A, items[q].x, wsm, wsm + 2 * R.A.cap + 3, stk, lane);
             }
         }
         __syncwarp();

@@ -72,6 +72,34 @@ __device__ __forceinline__ int next_offset(const int32_t* W, int k, const uint64
     return x + extend_run<BITS>(P, T, x - k, x, m, n);
 }
 
+// Wavefront values of diagonals k and k + G (the second where k + G <= hi; else it
+// is WFA_NULL) on 2-bit codes: next_offset for both with their first 16 bases
+// loaded together, so the two chains from wavefront to words to result overlap.
+__device__ __forceinline__ void next_offsets2(const int32_t* W, int k, int k2, bool two, const uint64_t* __restrict__ P,
+                                              const uint64_t* __restrict__ T, int m, int n, int& r0, int& r1)
+{
+    const uint32_t* p = reinterpret_cast<const uint32_t*>(P);
+    const uint32_t* t = reinterpret_cast<const uint32_t*>(T);
+    const int x0 = max(W[k + 1], max(W[k - 1], W[k]) + 1);
+    const int x1 = two ? max(W[k2 + 1], max(W[k2 - 1], W[k2]) + 1) : WFA_NULL;
+    const int lim0 = min(m - (x0 - k), n - x0), lim1 = min(m - (x1 - k2), n - x1);
+    const bool live0 = (unsigned)x0 <= (unsigned)n && x0 - k <= m, live1 = (unsigned)x1 <= (unsigned)n && x1 - k2 <= m;
+    const int v0 = live0 ? x0 - k : 0, h0 = live0 ? x0 : 0, v1 = live1 ? x1 - k2 : 0, h1 = live1 ? x1 : 0;
+    const uint32_t a0 = __ldg(p + (v0 >> 4)), a1 = __ldg(p + (v0 >> 4) + 1), b0 = __ldg(t + (h0 >> 4)),
+                   b1 = __ldg(t + (h0 >> 4) + 1);
+    const uint32_t c0 = __ldg(p + (v1 >> 4)), c1 = __ldg(p + (v1 >> 4) + 1), d0 = __ldg(t + (h1 >> 4)),
+                   d1 = __ldg(t + (h1 >> 4) + 1);
+    const uint32_t e0 = __funnelshift_r(a0, a1, 2 * v0) ^ __funnelshift_r(b0, b1, 2 * h0);
+    const uint32_t e1 = __funnelshift_r(c0, c1, 2 * v1) ^ __funnelshift_r(d0, d1, 2 * h1);
+    int run0 = e0 ? __clz((int)__brev(e0)) >> 1 : 16, run1 = e1 ? __clz((int)__brev(e1)) >> 1 : 16;
+    run0 = min(run0, lim0);
+    run1 = min(run1, lim1);
+    if (live0 && run0 == 16 && lim0 > 16) run0 += extend_run<2>(P, T, v0 + 16, h0 + 16, m, n);
+    if (live1 && run1 == 16 && lim1 > 16) run1 += extend_run<2>(P, T, v1 + 16, h1 + 16, m, n);
+    r0 = live0 ? x0 + run0 : WFA_NULL;
+    r1 = live1 ? x1 + run1 : WFA_NULL;
+}
+
 // Diagonals of wavefront s that can matter: within reach of s edits, inside the
 // matrix, and close enough to the final diagonal for the edits left up to smax.
 // The values there are the full wavefront's: what they read of the one before
@@ -83,7 +111,12 @@ __device__ __forceinline__ int wave_hi(int s, int n, int kfinal, int smax) { ret
 // wf0, wf1: 2 smax + 3 ints each; stk (trace): wavefront s at diagonal k goes to
 // stk[s * s + s + k].  One barrier a step: a step reads the wavefront before and
 // writes the other buffer, which the step before it was the last to read.
-template <bool TRACE, int BITS, int G>
+// AHEAD: two diagonals a lane at once (next_offsets2).  It shortens a lone pair's
+// chain and lengthens the code: a batch of no more pairs than resident warps, bound
+// by that chain, gains (the warps' 669 pairs of the 2,000-pair long batch: 1.0 ->
+// 0.73 ms), a full device, bound by instruction issue, loses (20,000 x 2 kb: 656 ->
+// 695 us).
+template <bool TRACE, int BITS, int G, bool AHEAD = false>
 __device__ int wfa_forward(const uint64_t* __restrict__ P, const uint64_t* __restrict__ T, int m, int n, int smax,
                            int32_t* wf0, int32_t* wf1, int32_t* stk, int gl, unsigned gmask)
 {
@@ -103,10 +136,25 @@ __device__ int wfa_forward(const uint64_t* __restrict__ P, const uint64_t* __res
     gsync<G>(gmask);
     for (int s = 1; s <= smax; ++s) {
         const int hi = wave_hi(s, n, kfinal, smax);
-        for (int k = wave_lo(s, m, kfinal, smax) + gl; k <= hi; k += G) {
-            const int x = next_offset<BITS>(prev, k, P, T, m, n);
-            cur[k] = x;
-            if (TRACE) stk[(int64_t)s * s + s + k] = x;
+        int32_t* const row = TRACE ? stk + (int64_t)s * s + s : nullptr;
+        if constexpr (BITS == 2 && AHEAD) {
+            for (int k = wave_lo(s, m, kfinal, smax) + gl; k <= hi; k += 2 * G) {
+                const bool two = k + G <= hi;
+                int x0, x1;
+                next_offsets2(prev, k, k + G, two, P, T, m, n, x0, x1);
+                cur[k] = x0;
+                if (TRACE) row[k] = x0;
+                if (two) {
+                    cur[k + G] = x1;
+                    if (TRACE) row[k + G] = x1;
+                }
+            }
+        } else {
+            for (int k = wave_lo(s, m, kfinal, smax) + gl; k <= hi; k += G) {
+                const int x = next_offset<BITS>(prev, k, P, T, m, n);
+                cur[k] = x;
+                if (TRACE) row[k] = x;
+            }
         }
         gsync<G>(gmask);
         if (cur[kfinal] >= n) return s;

@@ -64,3 +64,18 @@ def test_smax_at_the_distance():
         for smax in (int(d[k]), int(d[k]) - 1):
             want = oracle.wfa_batch(ps[k:k + 1], ts[k:k + 1], smax=smax, with_cigar=True)
             assert_wfa_equal(wfa_gpu(ps[k:k + 1], ts[k:k + 1], smax=smax), want, f"pair {k}, smax {smax}")
+
+
+@pytest.mark.parametrize("copies", [1, 60])
+def test_one_and_two_diagonals_a_lane(copies):
+    """The warp queue with no more pairs than warps (two diagonals a lane) and with more."""
+    assert cost_model.load_default()
+    ps, ts = _pairs(34)
+    ps, ts = ps * copies, ts * copies
+    before = api.tune_get()
+    try:
+        api.tune_set(wfa_lane_smax=0, wfa_group=32)
+        want = oracle.wfa_batch(ps, ts, smax=100, with_cigar=True)
+        assert_wfa_equal(wfa_gpu(ps, ts, smax=100, learned=True), want, f"{len(ps)} pairs")
+    finally:
+        api.tune_set(**before)

@@ -16,8 +16,7 @@
 // MLP: 66 -> 128 (ReLU) -> 128 (ReLU) -> 2, weights stored as bf16 and
 // computed in fp32 (fp32 master copy for Adam).  Outputs: log2(d + 1) and
 // log2(wavefront cells + 1) with wavefront cells = (d + 1)^2.  It is a tiny
-// GEMM (25k multiply-adds per pair), run as shared-memory-tiled FMA: 64 pairs
-// per block, 256 threads, every thread 32 outputs of one pair.
+// GEMM (25k multiply-adds per pair); training runs it as register-tiled fp32 FMA.
 #include <mutex>
 #include <vector>
 
@@ -31,7 +30,6 @@ namespace ga {
 constexpr int NF = 66, NH1 = 128, NH2 = 128, NO = 2;
 constexpr int OFF_W1 = 0, OFF_B1 = OFF_W1 + NH1 * NF, OFF_W2 = OFF_B1 + NH1, OFF_B2 = OFF_W2 + NH2 * NH1,
               OFF_W3 = OFF_B2 + NH2, OFF_B3 = OFF_W3 + NO * NH2, NPARAM = OFF_B3 + NO;
-constexpr int TILE = 64;
 
 void prepare_mlp();
 const __nv_bfloat16* cost_model_weights();
@@ -124,178 +122,290 @@ __global__ void __launch_bounds__(256) sketch_packed_kernel(PairDesc D, float* _
 }
 
 // ------------------------------------------------------------------- MLP --
-struct MlpParams {
-    const __nv_bfloat16* w;   // NPARAM bf16 (weights and biases)
-};
+// Training and the fp32 forward pass: a block of 512 threads per tile of 64 rows.
+// All weights stay in shared memory as fp32 for the block's life (one copy of each
+// matrix, [out][in]: a product over `in` reads four of them at once, a product over
+// `out` reads rows), and each thread keeps a register tile of its product: 4 x 4 cells
+// of a layer, 8 x 4 of dW2, so shared memory is read once per 10 multiply-adds or so
+// (twice per multiply-add before).  Bound by FMA issue (66 k multiply-adds a row: the
+// products whose operands lie in pairs run two to an instruction) and by the latency
+// of eight phases on one tile.  Gradient of 8,192 rows: kernel 150 -> 43.6 us, call
+// 182 -> 76 us.  Every sum runs over its index in order, 64 rows to an atomic.  Tiles
+// of 16 rows are quicker on batches that leave multiprocessors idle (500 rows: 56 us a
+// call against 68), but four times as many atomics carry the sum: relative error 1.0e-7
+// against 7.7e-8 there.
+constexpr int MLP_T = 512, TILE = 64;
+constexpr int MLP_S1 = 68, MLP_S2 = 132;      // row strides: 16-byte rows, 8 rows on 8 bank quads
 
-// Shared-memory image of one tile's layers.
 struct MlpSmem {
-    float W[NH2 * NH1];        // the current layer's weights, transposed [in][out]
-    float X[TILE * (NF + 2)];
-    float H1[TILE * (NH1 + 1)];
-    float H2[TILE * (NH2 + 1)];
+    float W1[NH1 * MLP_S1];       // columns 66, 67 zero
+    float W2[NH2 * MLP_S2];
+    float W3[NO * NH2];
+    float b1[NH1], b2[NH2], b3[4];
+    float X[TILE * MLP_S1];          // columns 66, 67 zero, rows past the batch zero
+    float H1[TILE * MLP_S2];         // then dL/dH1
+    float H2[TILE * MLP_S2];         // then dL/dH2
+    float y[2 * TILE], dy[2 * TILE], loss[4];
 };
 
-// out[r][o] = act(sum_i in[r][i] * W[o][i] + b[o]) for the tile's rows; W is
-// staged transposed in smem with outputs interleaved by 4 (o = 4k + oq) so the
-// four output groups of a warp read four different banks.
-template <int IN, int OUT, bool RELU>
-__device__ __forceinline__ void dense(const __nv_bfloat16* __restrict__ w, const __nv_bfloat16* __restrict__ b,
-                                      float* Ws, const float* in, int in_stride, float* out, int out_stride,
-                                      int rows)
+__device__ __forceinline__ void load_weights(const __nv_bfloat16* __restrict__ w, MlpSmem& S)
 {
-    __syncthreads();
-    for (int idx = threadIdx.x; idx < IN * OUT; idx += blockDim.x) {
-        const int o = idx / IN, i = idx - o * IN;
-        Ws[i * OUT + o] = __bfloat162float(w[idx]);
+    for (int idx = threadIdx.x; idx < NH1 * (NF / 2); idx += MLP_T) {
+        const int o = idx / (NF / 2), i = 2 * (idx - o * (NF / 2));
+        const float2 v = __bfloat1622float2(*(const __nv_bfloat162*)(w + OFF_W1 + o * NF + i));
+        *(float2*)&S.W1[o * MLP_S1 + i] = v;
+    }
+    for (int o = threadIdx.x; o < NH1; o += MLP_T) *(float2*)&S.W1[o * MLP_S1 + NF] = make_float2(0.f, 0.f);
+    for (int idx = threadIdx.x; idx < NH2 * NH1 / 4; idx += MLP_T) {
+        const int o = idx / (NH1 / 4), i = 4 * (idx - o * (NH1 / 4));
+        const __nv_bfloat162* q = (const __nv_bfloat162*)(w + OFF_W2 + o * NH1 + i);
+        const float2 u = __bfloat1622float2(q[0]), v = __bfloat1622float2(q[1]);
+        *(float4*)&S.W2[o * MLP_S2 + i] = make_float4(u.x, u.y, v.x, v.y);
+    }
+    for (int i = threadIdx.x; i < NO * NH2; i += MLP_T) S.W3[i] = __bfloat162float(w[OFF_W3 + i]);
+    for (int i = threadIdx.x; i < NH1; i += MLP_T) S.b1[i] = __bfloat162float(w[OFF_B1 + i]);
+    for (int i = threadIdx.x; i < NH2; i += MLP_T) S.b2[i] = __bfloat162float(w[OFF_B2 + i]);
+    if (threadIdx.x < NO) S.b3[threadIdx.x] = __bfloat162float(w[OFF_B3 + threadIdx.x]);
+}
+
+// out[r][o] = max(0, b[o] + sum_i in[r][i] W[o][i]), r < 64, o < 128, i < K.  A warp
+// holds 4 row groups x 8 output groups: rows rg + 16 j, outputs cg + 32 k, so both
+// operands' 16-byte reads are one shared-memory pass each.
+template <int K>
+__device__ __forceinline__ void dense_relu(const float* W, int ws, const float* b, const float* in, int is, float* out)
+{
+    constexpr int NR = TILE / 16;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const int rg = (wid & 3) * 4 + (lane >> 3), cg = (wid >> 2) * 8 + (lane & 7);
+    float acc[NR][4];
+#pragma unroll
+    for (int j = 0; j < NR; ++j)
+#pragma unroll
+        for (int k = 0; k < 4; ++k) acc[j][k] = b[cg + 32 * k];
+#pragma unroll 2
+    for (int i = 0; i < K; i += 4) {
+        float4 x[NR], v[4];
+#pragma unroll
+        for (int j = 0; j < NR; ++j) x[j] = *(const float4*)&in[(rg + 16 * j) * is + i];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) v[k] = *(const float4*)&W[(cg + 32 * k) * ws + i];
+#pragma unroll
+        for (int j = 0; j < NR; ++j)
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                float t = fmaf(x[j].x, v[k].x, acc[j][k]);
+                t = fmaf(x[j].y, v[k].y, t);
+                t = fmaf(x[j].z, v[k].z, t);
+                acc[j][k] = fmaf(x[j].w, v[k].w, t);
+            }
+    }
+#pragma unroll
+    for (int j = 0; j < NR; ++j)
+#pragma unroll
+        for (int k = 0; k < 4; ++k) out[(rg + 16 * j) * MLP_S2 + cg + 32 * k] = fmaxf(acc[j][k], 0.f);
+}
+
+// Rows [base, base + rows) through the network: S.H1, S.H2 and S.y.
+__device__ __forceinline__ void forward_tile(const float* __restrict__ feat, int64_t base, int rows, MlpSmem& S)
+{
+    for (int idx = threadIdx.x; idx < TILE * MLP_S1; idx += MLP_T) {
+        const int r = idx / MLP_S1, i = idx - r * MLP_S1;
+        S.X[idx] = (r < rows && i < NF) ? feat[(base + r) * NF + i] : 0.f;
     }
     __syncthreads();
-    constexpr int PER = OUT / 4;                  // outputs per thread (4 threads per row)
-    const int r = threadIdx.x >> 2, oq = threadIdx.x & 3;
-    if (r < rows) {
-        float acc[PER];
-#pragma unroll
-        for (int k = 0; k < PER; ++k) acc[k] = __bfloat162float(b[4 * k + oq]);
-        for (int i = 0; i < IN; ++i) {
-            const float x = in[r * in_stride + i];
-            const float* wr = Ws + i * OUT;
-#pragma unroll
-            for (int k = 0; k < PER; ++k) acc[k] = fmaf(x, wr[4 * k + oq], acc[k]);
+    dense_relu<MLP_S1>(S.W1, MLP_S1, S.b1, S.X, MLP_S1, S.H1);
+    __syncthreads();
+    dense_relu<NH1>(S.W2, MLP_S2, S.b2, S.H1, MLP_S2, S.H2);
+    __syncthreads();
+    if (threadIdx.x < 2 * TILE) {
+        const int r = threadIdx.x >> 1, o = threadIdx.x & 1;
+        float acc = S.b3[o];
+#pragma unroll 4
+        for (int i = 0; i < NH2; i += 4) {
+            const float4 h = *(const float4*)&S.H2[r * MLP_S2 + i], v = *(const float4*)&S.W3[o * NH2 + i];
+            acc = fmaf(h.x, v.x, acc);
+            acc = fmaf(h.y, v.y, acc);
+            acc = fmaf(h.z, v.z, acc);
+            acc = fmaf(h.w, v.w, acc);
         }
-#pragma unroll
-        for (int k = 0; k < PER; ++k) out[r * out_stride + 4 * k + oq] = RELU ? fmaxf(acc[k], 0.f) : acc[k];
+        S.y[threadIdx.x] = acc;
     }
-}
-
-// The output layer (2 outputs) by one thread per row.
-__device__ __forceinline__ void dense_out(const __nv_bfloat16* __restrict__ w, const float* H2, float* y, int rows)
-{
-    const int r = threadIdx.x;
-    if (r < rows) {
-        float a0 = __bfloat162float(w[OFF_B3]), a1 = __bfloat162float(w[OFF_B3 + 1]);
-        for (int i = 0; i < NH2; ++i) {
-            const float h = H2[r * (NH2 + 1) + i];
-            a0 = fmaf(h, __bfloat162float(w[OFF_W3 + i]), a0);
-            a1 = fmaf(h, __bfloat162float(w[OFF_W3 + NH2 + i]), a1);
-        }
-        y[2 * r] = a0;
-        y[2 * r + 1] = a1;
-    }
-}
-
-__device__ __forceinline__ void forward_tile(const __nv_bfloat16* w, const float* __restrict__ feat, int64_t base,
-                                             int rows, MlpSmem& S, float* ytile)
-{
-    for (int idx = threadIdx.x; idx < rows * NF; idx += blockDim.x) {
-        const int r = idx / NF, i = idx - r * NF;
-        S.X[r * (NF + 2) + i] = feat[(base + r) * NF + i];
-    }
-    dense<NF, NH1, true>(w + OFF_W1, w + OFF_B1, S.W, S.X, NF + 2, S.H1, NH1 + 1, rows);
-    dense<NH1, NH2, true>(w + OFF_W2, w + OFF_B2, S.W, S.H1, NH1 + 1, S.H2, NH2 + 1, rows);
-    __syncthreads();
-    dense_out(w, S.H2, ytile, rows);
     __syncthreads();
 }
 
-__global__ void __launch_bounds__(256) mlp_forward_kernel(const __nv_bfloat16* __restrict__ w,
-                                                          const float* __restrict__ feat, int n, float* __restrict__ y)
+__global__ void __launch_bounds__(MLP_T, 1) mlp_forward_kernel(const __nv_bfloat16* __restrict__ w,
+                                                            const float* __restrict__ feat, int n, float* __restrict__ y)
 {
-    extern __shared__ float mlp_smem[];
+    extern __shared__ __align__(16) float mlp_smem[];
     MlpSmem& S = *reinterpret_cast<MlpSmem*>(mlp_smem);
-    __shared__ float ytile[2 * TILE];
+    load_weights(w, S);
     for (int64_t base = (int64_t)blockIdx.x * TILE; base < n; base += (int64_t)gridDim.x * TILE) {
         const int rows = (n - base < TILE) ? (int)(n - base) : TILE;
-        forward_tile(w, feat, base, rows, S, ytile);
-        for (int idx = threadIdx.x; idx < 2 * rows; idx += blockDim.x) y[2 * base + idx] = ytile[idx];
+        forward_tile(feat, base, rows, S);
+        for (int idx = threadIdx.x; idx < 2 * rows; idx += MLP_T) y[2 * base + idx] = S.y[idx];
         __syncthreads();
     }
+}
+
+__device__ __forceinline__ void add4(float4& a, float s, const float4& v)
+{
+    const float2 ss = make_float2(s, s);
+    const float2 lo = __ffma2_rn(ss, make_float2(v.x, v.y), make_float2(a.x, a.y));
+    const float2 hi = __ffma2_rn(ss, make_float2(v.z, v.w), make_float2(a.z, a.w));
+    a = make_float4(lo.x, lo.y, hi.x, hi.y);
 }
 
 // Forward + backward of the mean squared error over the batch; gradients of
 // every parameter (with respect to the bf16-rounded weights) accumulate into
-// grad (fp32) and the summed squared error into loss.
-__global__ void __launch_bounds__(256) mlp_backward_kernel(const __nv_bfloat16* __restrict__ w,
-                                                           const float* __restrict__ feat,
-                                                           const float* __restrict__ target, int n,
-                                                           float inv_batch, float* __restrict__ grad,
-                                                           float* __restrict__ loss)
+// grad (fp32, 16-byte aligned), the summed squared error behind them.  Blocks add to
+// GRAD_COPIES copies in turn and fold_grad_kernel adds the copies: a quarter of the
+// partial sums in a row, so a smaller rounding error (8,192 rows: 5.5e-8 relative against
+// 1.7e-7 with one copy), for 3 us.
+constexpr int GRAD_COPIES = 4, GRAD_STRIDE = (NPARAM + 1 + 3) / 4 * 4;
+
+__global__ void fold_grad_kernel(float* __restrict__ grad)
 {
-    extern __shared__ float mlp_smem[];
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i <= NPARAM)
+        grad[i] = (grad[i] + grad[GRAD_STRIDE + i]) + (grad[2 * GRAD_STRIDE + i] + grad[3 * GRAD_STRIDE + i]);
+}
+
+__global__ void __launch_bounds__(MLP_T, 1) mlp_backward_kernel(const __nv_bfloat16* __restrict__ w,
+                                                             const float* __restrict__ feat,
+                                                             const float* __restrict__ target, int n,
+                                                             float inv_batch, float* __restrict__ grad)
+{
+    extern __shared__ __align__(16) float mlp_smem[];
     MlpSmem& S = *reinterpret_cast<MlpSmem*>(mlp_smem);
-    __shared__ float ytile[2 * TILE];
-    __shared__ float dy[2 * TILE];
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    grad += (blockIdx.x % GRAD_COPIES) * GRAD_STRIDE;
+    load_weights(w, S);
     for (int64_t base = (int64_t)blockIdx.x * TILE; base < n; base += (int64_t)gridDim.x * TILE) {
         const int rows = (n - base < TILE) ? (int)(n - base) : TILE;
-        forward_tile(w, feat, base, rows, S, ytile);
+        forward_tile(feat, base, rows, S);
         // dL/dy = 2 (y - t) / B
-        float lsum = 0.f;
-        for (int idx = threadIdx.x; idx < 2 * TILE; idx += blockDim.x) {
-            float g = 0.f;
-            if (idx < 2 * rows) {
-                const float e = ytile[idx] - target[2 * base + idx];
-                lsum += e * e;
-                g = 2.f * e * inv_batch;
+        if (tid < 2 * TILE) {
+            float e = 0.f;
+            if (tid < 2 * rows) e = S.y[tid] - target[2 * base + tid];
+            S.dy[tid] = 2.f * e * inv_batch;
+            float lsum = e * e;
+            for (int o = 16; o > 0; o >>= 1) lsum += __shfl_xor_sync(FULL, lsum, o);
+            if (lane == 0) S.loss[wid] = lsum;
+        }
+        __syncthreads();
+        // output layer: dW3, db3; dH2 = dy W3 * relu'(H2), H2's column overwritten by the thread that summed it
+        if (tid < NH2) {
+            const float w0 = S.W3[tid], w1 = S.W3[NH2 + tid];
+            float g0 = 0.f, g1 = 0.f, gb = 0.f;
+#pragma unroll 4
+            for (int r = 0; r < rows; ++r) {
+                const float2 d = *(const float2*)&S.dy[2 * r];
+                float* hp = &S.H2[r * MLP_S2 + tid];
+                const float h = *hp;
+                g0 = fmaf(d.x, h, g0);
+                g1 = fmaf(d.y, h, g1);
+                const float g = h > 0.f ? d.x * w0 + d.y * w1 : 0.f;
+                gb += g;
+                *hp = g;
             }
-            dy[idx] = g;
-        }
-        for (int o = 16; o > 0; o >>= 1) lsum += __shfl_xor_sync(FULL, lsum, o);
-        if ((threadIdx.x & 31) == 0) atomicAdd(loss, lsum);
-        __syncthreads();
-        // output layer: dW3, db3; dH2 = dy W3 * relu'(H2) (H2 overwritten in place)
-        for (int idx = threadIdx.x; idx < NO * NH2; idx += blockDim.x) {
-            const int o = idx / NH2, i = idx - o * NH2;
+            atomicAdd(&grad[OFF_W3 + tid], g0);
+            atomicAdd(&grad[OFF_W3 + NH2 + tid], g1);
+            atomicAdd(&grad[OFF_B2 + tid], gb);
+        } else if (tid < NH2 + NO) {
             float g = 0.f;
-            for (int r = 0; r < rows; ++r) g = fmaf(dy[2 * r + o], S.H2[r * (NH2 + 1) + i], g);
-            atomicAdd(&grad[OFF_W3 + idx], g);
-        }
-        if (threadIdx.x < NO) {
-            float g = 0.f;
-            for (int r = 0; r < rows; ++r) g += dy[2 * r + threadIdx.x];
-            atomicAdd(&grad[OFF_B3 + threadIdx.x], g);
+            for (int r = 0; r < rows; ++r) g += S.dy[2 * r + tid - NH2];
+            atomicAdd(&grad[OFF_B3 + tid - NH2], g);
+        } else if (tid == NH2 + NO) {
+            atomicAdd(&grad[NPARAM], (S.loss[0] + S.loss[1]) + (S.loss[2] + S.loss[3]));
         }
         __syncthreads();
-        for (int idx = threadIdx.x; idx < rows * NH2; idx += blockDim.x) {
-            const int r = idx / NH2, i = idx - r * NH2;
-            float* h = &S.H2[r * (NH2 + 1) + i];
-            const float g = dy[2 * r] * __bfloat162float(w[OFF_W3 + i]) + dy[2 * r + 1] * __bfloat162float(w[OFF_W3 + NH2 + i]);
-            *h = (*h > 0.f) ? g : 0.f;
+        // layer 2: dW2[o][i] = sum_r dH2[r][o] H1[r][i], 8 outputs (the warp's) x 4 inputs (the lane's) a thread
+        {
+            float4 acc[8];
+#pragma unroll
+            for (int k = 0; k < 8; ++k) acc[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 2
+            for (int r = 0; r < rows; ++r) {
+                const float4 h = *(const float4*)&S.H1[r * MLP_S2 + 4 * lane];
+                const float4 d0 = *(const float4*)&S.H2[r * MLP_S2 + 8 * wid];
+                const float4 d1 = *(const float4*)&S.H2[r * MLP_S2 + 8 * wid + 4];
+                add4(acc[0], d0.x, h);
+                add4(acc[1], d0.y, h);
+                add4(acc[2], d0.z, h);
+                add4(acc[3], d0.w, h);
+                add4(acc[4], d1.x, h);
+                add4(acc[5], d1.y, h);
+                add4(acc[6], d1.z, h);
+                add4(acc[7], d1.w, h);
+            }
+#pragma unroll
+            for (int k = 0; k < 8; ++k) atomicAdd((float4*)&grad[OFF_W2 + (8 * wid + k) * NH1 + 4 * lane], acc[k]);
+        }
+        // dH1[r][i] = sum_o dH2[r][o] W2[o][i] * relu'(H1), in place
+        {
+            constexpr int NR = TILE / 16;
+            const int rg = (wid & 3) * 4 + (lane >> 3), i0 = 4 * ((wid >> 2) * 8 + (lane & 7));
+            float4 acc[NR];
+#pragma unroll
+            for (int j = 0; j < NR; ++j) acc[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 2
+            for (int o = 0; o < NH2; o += 4) {
+                float4 d[NR], v[4];
+#pragma unroll
+                for (int j = 0; j < NR; ++j) d[j] = *(const float4*)&S.H2[(rg + 16 * j) * MLP_S2 + o];
+#pragma unroll
+                for (int k = 0; k < 4; ++k) v[k] = *(const float4*)&S.W2[(o + k) * MLP_S2 + i0];
+#pragma unroll
+                for (int j = 0; j < NR; ++j) {
+                    add4(acc[j], d[j].x, v[0]);
+                    add4(acc[j], d[j].y, v[1]);
+                    add4(acc[j], d[j].z, v[2]);
+                    add4(acc[j], d[j].w, v[3]);
+                }
+            }
+            __syncthreads();                       // dW2 has read H1
+#pragma unroll
+            for (int j = 0; j < NR; ++j) {
+                float4* hp = (float4*)&S.H1[(rg + 16 * j) * MLP_S2 + i0];
+                const float4 h = *hp;
+                *hp = make_float4(h.x > 0.f ? acc[j].x : 0.f, h.y > 0.f ? acc[j].y : 0.f, h.z > 0.f ? acc[j].z : 0.f,
+                                  h.w > 0.f ? acc[j].w : 0.f);
+            }
         }
         __syncthreads();
-        // layer 2: dW2[o][i] = sum_r dH2[r][o] H1[r][i]; db2; dH1 = dH2 W2 * relu'(H1)
-        for (int idx = threadIdx.x; idx < NH2 * NH1; idx += blockDim.x) {
-            const int o = idx / NH1, i = idx - o * NH1;
-            float g = 0.f;
-            for (int r = 0; r < rows; ++r) g = fmaf(S.H2[r * (NH2 + 1) + o], S.H1[r * (NH1 + 1) + i], g);
-            atomicAdd(&grad[OFF_W2 + idx], g);
-        }
-        for (int o = threadIdx.x; o < NH2; o += blockDim.x) {
-            float g = 0.f;
-            for (int r = 0; r < rows; ++r) g += S.H2[r * (NH2 + 1) + o];
-            atomicAdd(&grad[OFF_B2 + o], g);
-        }
-        // W2 (not transposed) into S.W: W[o][i]
-        for (int idx = threadIdx.x; idx < NH2 * NH1; idx += blockDim.x) S.W[idx] = __bfloat162float(w[OFF_W2 + idx]);
-        __syncthreads();
-        for (int idx = threadIdx.x; idx < rows * NH1; idx += blockDim.x) {
-            const int r = idx / NH1, i = idx - r * NH1;
-            float g = 0.f;
-            for (int o = 0; o < NH2; ++o) g = fmaf(S.H2[r * (NH2 + 1) + o], S.W[o * NH1 + i], g);
-            // each thread reads and overwrites only its own H1 entry: dH1 in place
-            const float h = S.H1[r * (NH1 + 1) + i];
-            S.H1[r * (NH1 + 1) + i] = (h > 0.f) ? g : 0.f;
-        }
-        __syncthreads();
-        // layer 1: dW1[o][i] = sum_r dH1[r][o] X[r][i]; db1
-        for (int idx = threadIdx.x; idx < NH1 * NF; idx += blockDim.x) {
-            const int o = idx / NF, i = idx - o * NF;
-            float g = 0.f;
-            for (int r = 0; r < rows; ++r) g = fmaf(S.H1[r * (NH1 + 1) + o], S.X[r * (NF + 2) + i], g);
-            atomicAdd(&grad[OFF_W1 + idx], g);
-        }
-        for (int o = threadIdx.x; o < NH1; o += blockDim.x) {
-            float g = 0.f;
-            for (int r = 0; r < rows; ++r) g += S.H1[r * (NH1 + 1) + o];
-            atomicAdd(&grad[OFF_B1 + o], g);
+        // layer 1: dW1[o][i] = sum_r dH1[r][o] X[r][i]: 4 x 4 a thread for i < 64, then the last two inputs and db1
+        {
+            const int o0 = 4 * (tid >> 4), i0 = 4 * (tid & 15);
+            float4 acc[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) acc[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 2
+            for (int r = 0; r < rows; ++r) {
+                const float4 d = *(const float4*)&S.H1[r * MLP_S2 + o0], x = *(const float4*)&S.X[r * MLP_S1 + i0];
+                add4(acc[0], d.x, x);
+                add4(acc[1], d.y, x);
+                add4(acc[2], d.z, x);
+                add4(acc[3], d.w, x);
+            }
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                float* g = &grad[OFF_W1 + (o0 + k) * NF + i0];
+                atomicAdd((float2*)g, make_float2(acc[k].x, acc[k].y));
+                atomicAdd((float2*)(g + 2), make_float2(acc[k].z, acc[k].w));
+            }
+            if (tid < 2 * NH1) {
+                const int o = tid & (NH1 - 1), i = NF - 2 + tid / NH1;
+                float g = 0.f;
+#pragma unroll 4
+                for (int r = 0; r < rows; ++r) g = fmaf(S.H1[r * MLP_S2 + o], S.X[r * MLP_S1 + i], g);
+                atomicAdd(&grad[OFF_W1 + o * NF + i], g);
+            } else if (tid < 3 * NH1) {
+                const int o = tid - 2 * NH1;
+                float g = 0.f;
+#pragma unroll 4
+                for (int r = 0; r < rows; ++r) g += S.H1[r * MLP_S2 + o];
+                atomicAdd(&grad[OFF_B1 + o], g);
+            }
         }
         __syncthreads();
     }
@@ -623,7 +733,7 @@ static cudaError_t run_forward_tc(const __nv_bfloat16* w, const float* feat, int
 struct Model {
     float* master = nullptr;
     __nv_bfloat16* w = nullptr;
-    float *m1 = nullptr, *m2 = nullptr, *grad = nullptr, *loss = nullptr;
+    float *m1 = nullptr, *m2 = nullptr, *grad = nullptr;   // grad: GRAD_COPIES copies; the loss behind the first
     int step = 0;
     bool ready = false;
 };
@@ -647,8 +757,7 @@ static Model* model_for(int slot, bool create)
             cudaMalloc(&M.w, NPARAM * sizeof(__nv_bfloat16)) != cudaSuccess ||
             cudaMalloc(&M.m1, NPARAM * sizeof(float)) != cudaSuccess ||
             cudaMalloc(&M.m2, NPARAM * sizeof(float)) != cudaSuccess ||
-            cudaMalloc(&M.grad, NPARAM * sizeof(float)) != cudaSuccess ||
-            cudaMalloc(&M.loss, sizeof(float)) != cudaSuccess) {
+            cudaMalloc(&M.grad, GRAD_COPIES * GRAD_STRIDE * sizeof(float)) != cudaSuccess) {
             cudaGetLastError();
             return nullptr;
         }
@@ -656,16 +765,14 @@ static Model* model_for(int slot, bool create)
     return M.master ? &M : nullptr;
 }
 
-static size_t mlp_smem_bytes() { return sizeof(MlpSmem); }
-
 // Kernel attributes are set outside any stream capture (prepare_mlp is called
 // while planning a batch).
 void prepare_mlp()
 {
     static std::once_flag once;
     std::call_once(once, [] {
-        cudaFuncSetAttribute(mlp_forward_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)mlp_smem_bytes());
-        cudaFuncSetAttribute(mlp_backward_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)mlp_smem_bytes());
+        cudaFuncSetAttribute(mlp_forward_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(MlpSmem));
+        cudaFuncSetAttribute(mlp_backward_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(MlpSmem));
         cudaFuncSetAttribute(mlp_forward_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(TcSmem));
         cudaFuncSetAttribute(route_model_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)route_model_smem());
@@ -674,28 +781,28 @@ void prepare_mlp()
     });
 }
 
+// A tile a block, no more blocks than multiprocessors (a block's shared memory fills one).
+static int mlp_blocks(int n) { return std::min((int)(((int64_t)n + TILE - 1) / TILE), device_sms()); }
+
 static cudaError_t run_forward(const __nv_bfloat16* w, const float* feat, int n, float* y, cudaStream_t st)
 {
     if (n <= 0) return cudaSuccess;
     prepare_mlp();
-    int blocks = (n + TILE - 1) / TILE;
-    blocks = std::min(blocks, device_sms() * 2);
     launch_begin(K_MLP, st);
-    mlp_forward_kernel<<<blocks, 256, mlp_smem_bytes(), st>>>(w, feat, n, y);
+    mlp_forward_kernel<<<mlp_blocks(n), MLP_T, sizeof(MlpSmem), st>>>(w, feat, n, y);
     launch_end(K_MLP, st);
     return cudaGetLastError();
 }
 
+// grad: GRAD_COPIES copies of GRAD_STRIDE floats; the result is the first, the loss at NPARAM.
 static cudaError_t run_backward(const __nv_bfloat16* w, const float* feat, const float* target, int n, float* grad,
-                                float* loss, cudaStream_t st)
+                                cudaStream_t st)
 {
     prepare_mlp();
-    cudaMemsetAsync(grad, 0, NPARAM * sizeof(float), st);
-    cudaMemsetAsync(loss, 0, sizeof(float), st);
-    int blocks = (n + TILE - 1) / TILE;
-    blocks = std::min(blocks, device_sms() * 2);
+    cudaMemsetAsync(grad, 0, GRAD_COPIES * GRAD_STRIDE * sizeof(float), st);
     launch_begin(K_MLP, st);
-    mlp_backward_kernel<<<blocks, 256, mlp_smem_bytes(), st>>>(w, feat, target, n, 1.0f / (float)n, grad, loss);
+    mlp_backward_kernel<<<mlp_blocks(n), MLP_T, sizeof(MlpSmem), st>>>(w, feat, target, n, 1.0f / (float)n, grad);
+    fold_grad_kernel<<<(NPARAM + 256) / 256, 256, 0, st>>>(grad);
     launch_end(K_MLP, st);
     return cudaGetLastError();
 }
@@ -871,9 +978,9 @@ int32_t ga_mlp_gradient(const float* feat, const float* target, int32_t n, float
     std::lock_guard<std::mutex> lk(g_model_mu);
     Model* M = model_for_current(false);
     if (!M || !M->ready) return GA_INVALID_ARGUMENT;
-    if (run_backward(M->w, feat, target, n, M->grad, M->loss, 0) != cudaSuccess ||
+    if (run_backward(M->w, feat, target, n, M->grad, 0) != cudaSuccess ||
         cudaMemcpy(grad_host, M->grad, NPARAM * sizeof(float), cudaMemcpyDeviceToHost) != cudaSuccess ||
-        (loss_host && cudaMemcpy(loss_host, M->loss, sizeof(float), cudaMemcpyDeviceToHost) != cudaSuccess)) {
+        (loss_host && cudaMemcpy(loss_host, M->grad + NPARAM, sizeof(float), cudaMemcpyDeviceToHost) != cudaSuccess)) {
         cudaGetLastError();
         return GA_DEVICE_ERROR;
     }
@@ -887,7 +994,7 @@ int32_t ga_mlp_train_step(const float* feat, const float* target, int32_t n, flo
     Model* M = model_for_current(false);
     if (!M || !M->ready) return GA_INVALID_ARGUMENT;
     cudaStream_t st = (cudaStream_t)stream;
-    if (run_backward(M->w, feat, target, n, M->grad, M->loss, st) != cudaSuccess) { cudaGetLastError(); return GA_DEVICE_ERROR; }
+    if (run_backward(M->w, feat, target, n, M->grad, st) != cudaSuccess) { cudaGetLastError(); return GA_DEVICE_ERROR; }
     M->step += 1;
     const float b1 = 0.9f, b2 = 0.999f;
     const float c1 = 1.f / (1.f - powf(b1, (float)M->step)), c2 = 1.f / (1.f - powf(b2, (float)M->step));
@@ -896,7 +1003,7 @@ int32_t ga_mlp_train_step(const float* feat, const float* target, int32_t n, flo
     launch_end(K_MLP, st);
     if (cudaGetLastError() != cudaSuccess) return GA_DEVICE_ERROR;
     if (loss_host) {
-        if (cudaMemcpyAsync(loss_host, M->loss, sizeof(float), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
+        if (cudaMemcpyAsync(loss_host, M->grad + NPARAM, sizeof(float), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
             cudaStreamSynchronize(st) != cudaSuccess) {
             cudaGetLastError();
             return GA_DEVICE_ERROR;

@@ -1146,17 +1146,36 @@ int32_t sw_check(const ga_sw_request* reqs, int32_t n, const char** err)
 struct SwPlan {
     int64_t ints[SP_LISTS] = {0, 0, 0};
     int64_t dir[SP_LISTS] = {0, 0, 0};
+    int64_t ncoop[SP_LISTS] = {0, 0, 0};             // leading whole-block items (bounds: 1 if there may be any)
+    int32_t w[SP_LISTS] = {4, 4, 4};                 // warps per block: the whole-block items', 4 without any
     int64_t edge_slot = 2;
-    int64_t max16_cells = 0;
     int64_t n_opt = 0, dir_opt = 0;
 };
 
+static int64_t sw_coop_limit(const ga_tune& T) { return T.sw_coop_log2 < 40 ? ((int64_t)1 << T.sw_coop_log2) : -1; }
+
+// Resident warps of a list's kernel, 0 without a whole-block phase.
+static int sw_coop_warps(int l, bool trace, const ga_tune& T)
+{
+    if (!trace) return l == SP_L16 ? sw16so_max_slots(device_sms()) : 0;
+    return l == SP_L16 ? sw16ck_max_slots(device_sms(), T.sw_window) : sw32ck_max_slots(l == SP_L32LONG, device_sms());
+}
+
 // The plan, built on the device (sw_plan.cu) into `dwork`, its record into dres.
+// launched: when set, the launches' block sizes are its (and the 16-bit launch has
+// the whole-block phase only if it counts such items); otherwise the device's choice.
 static cudaError_t enqueue_plan_sw(const PairDesc& D, const ga_sw_scoring& sc, bool trace, int64_t cell_limit,
                                    int32_t too_large_score, int32_t* out_score, int32_t* dwork, int32_t* scratch,
-                                   long long* dres, const ga_tune& T, cudaStream_t st, const uint8_t* try16 = nullptr)
+                                   long long* dres, const ga_tune& T, cudaStream_t st, const uint8_t* try16 = nullptr,
+                                   const SwPlan* launched = nullptr)
 {
     SwPlanArgs A;
+    A.coop_limit = sw_coop_limit(T);
+    for (int l = 0; l < SP_LISTS; ++l) {
+        A.coop_warps[l] = l == SP_L16 && launched && launched->ncoop[l] <= 0 ? 0 : sw_coop_warps(l, trace, T);
+        A.coop_block[l] = launched ? launched->w[l] : 0;
+    }
+    A.sms = device_sms();
     A.D = D;
     A.match = sc.match; A.mismatch = sc.mismatch; A.gap_open = sc.gap_open; A.gap_extend = sc.gap_extend;
     A.cell_limit = cell_limit;
@@ -1188,9 +1207,10 @@ static cudaError_t device_plan_sw(const PairDesc& D, const ga_sw_scoring& sc, bo
     for (int l = 0; l < SP_LISTS; ++l) {
         P.ints[l] = hres[SP_INTS + l];
         P.dir[l] = (hres[SP_DIR + l] + 3) / 4 * 4;
+        P.ncoop[l] = hres[SP_NCOOP + l];
+        P.w[l] = P.ncoop[l] > 0 ? (int32_t)hres[SP_COOPW + l] : 4;
     }
     P.edge_slot = std::max<int64_t>(2, hres[SP_EDGE]);
-    P.max16_cells = hres[SP_MAXC16];
     P.n_opt = hres[SP_NOPT];
     P.dir_opt = (hres[SP_DIROPT] + 3) / 4 * 4;
     return cudaSuccess;
@@ -1208,7 +1228,20 @@ static SwPlan bound_plan_sw(const ga_sw_request* reqs, int32_t n, bool trace, in
     SwPlan P;
     const ga_sw_scoring sc = reqs[0].scoring;
     int maxM16 = 0, maxN16 = 0;
-    int64_t n16 = 0, cnt[SP_LISTS] = {0, 0, 0}, edge = 2;
+    int64_t n16 = 0, cnt[SP_LISTS] = {0, 0, 0}, edge = 2, cells16 = 0, cells = 0, largest = 0, largest16 = 0;
+    int cols = 0;
+    // at most this list's items run on a block whatever the device finds: its share
+    // (sp_coop_cells) grows with the cells of its list, of which these are all
+    const int64_t limit = sw_coop_limit(T);
+    for (int32_t i = 0; i < n; ++i) {
+        const int64_t c = (int64_t)std::max(reqs[i].text_len, 0) * std::max(reqs[i].pattern_len, 0);
+        cells += c;
+        largest = std::max(largest, c);
+        cols = std::max(cols, (int)reqs[i].pattern_len);
+    }
+    const int W32 = sw_coop_block(largest, cols, cells, device_sms());
+    int64_t coop[SP_LISTS];
+    for (int l = SP_L32; l < SP_LISTS; ++l) coop[l] = sp_coop_cells(limit, cells, sw_coop_warps(l, trace, T));
     for (int32_t i = 0; i < n; ++i) {
         const int m = reqs[i].text_len, nn = reqs[i].pattern_len;
         if (cell_limit >= 0 && m > 0 && nn > 0 && ((int64_t)m + 1) * ((int64_t)nn + 1) > cell_limit) continue;
@@ -1221,6 +1254,8 @@ static SwPlan bound_plan_sw(const ga_sw_request* reqs, int32_t n, bool trace, in
                                                                  sc.gap_extend, T.sw_opt16_pct)));
         if (u16) {
             ++n16;
+            cells16 += (int64_t)m * nn;
+            largest16 = std::max(largest16, (int64_t)m * nn);
             maxM16 = std::max(maxM16, m);
             maxN16 = std::max(maxN16, nn);
             if (!strict) {
@@ -1230,12 +1265,33 @@ static SwPlan bound_plan_sw(const ga_sw_request* reqs, int32_t n, bool trace, in
         }
         const int l = (trace && sw32ck_long(m, nn, T.sw_long_log2)) ? SP_L32LONG : SP_L32;
         ++cnt[l];
-        if (trace) P.dir[l] = std::max(P.dir[l], sw32ck_dir_words(m, nn, T.sw_long_log2));
+        if (trace) {
+            int64_t words = sw32ck_dir_words(m, nn, T.sw_long_log2);
+            const int64_t c = (int64_t)std::max(m, 0) * std::max(nn, 0);
+            if (c > coop[l]) words = sw_coop_share(words, W32);
+            if (c > std::min(limit, SW_COOP_MIN) && limit >= 0) {
+                P.ncoop[l] = 1;
+                P.w[l] = W32;
+            }
+            P.dir[l] = std::max(P.dir[l], words);
+        }
         edge = std::max<int64_t>(edge, 2 * (int64_t)std::max(m, 0));
     }
     P.ints[SP_L16] = 2 * ((n16 + 1) / 2);
     P.dir[SP_L16] = n16 ? (trace ? sw16ck_dir_words(maxM16, maxN16, T.sw_window) : sw16so_dir_words(maxM16, maxN16)) : 0;
-    P.max16_cells = (int64_t)maxM16 * maxN16;
+    // the 16-bit list has its whole-block phase when the widest possible item is above its share of them all
+    const int64_t warps16 = sw_coop_warps(SP_L16, trace, T), coop16 = sp_coop_cells(limit, cells16 / 2, warps16);
+    if ((int64_t)maxM16 * maxN16 > coop16) {
+        P.ncoop[SP_L16] = 1;
+        // with a block for each item, the largest per-warp memory is a share of the
+        // widest item's or the whole of one of coop16 cells (M rows, at most 255
+        // padding columns, two words per 64 cells for rows and for edges each)
+        const int W = P.w[SP_L16] = sw_coop_block(largest16, maxN16, cells16 / 2, device_sms());
+        const int64_t own = trace ? 0 : SO_ROW_WORDS, fix = trace ? CK_K * T.sw_window * CK_TW : SO_ROW_WORDS;
+        if (W * ((n16 + 1) / 2) <= warps16)
+            P.dir[SP_L16] = std::min(P.dir[SP_L16], std::max(sw_coop_share(P.dir[SP_L16], W, own),
+                                                             coop16 / 16 + 16 * (int64_t)maxM16 + fix + 8));
+    }
     P.ints[SP_L32] = cnt[SP_L32];
     P.ints[SP_L32LONG] = cnt[SP_L32LONG];
     for (int l = 0; l < SP_LISTS; ++l) P.dir[l] = (P.dir[l] + 3) / 4 * 4;
@@ -1273,16 +1329,18 @@ static SwSlots size_sw(const SwPlan& P, bool trace, const ga_tune& T, int sm_cou
     SwSlots S;
     for (int l = 0; l < SP_LISTS; ++l) {
         if (P.ints[l] <= 0) continue;
-        // warp slots come in blocks of 4
+        // warp slots come in blocks of w; a whole-block item has a block to itself
+        const int w = P.w[l];
         int s;
         if (l == SP_L16) {
             s = trace ? sw16ck_max_slots(sm_count, T.sw_window) : sw16so_max_slots(sm_count);
-            s = (int)std::min<int64_t>(s, (P.ints[l] / 2 + 3) / 4 * 4);
+            s = (int)std::min<int64_t>(s, P.ncoop[l] > 0 ? P.ints[l] / 2 * w : (P.ints[l] / 2 + 3) / 4 * 4);
         } else {
             s = trace ? sw32ck_max_slots(l == SP_L32LONG, sm_count) : sw_max_slots(sm_count);
-            s = (int)std::min<int64_t>(s, (P.ints[l] + 3) / 4 * 4);
+            s = (int)std::min<int64_t>(s, P.ncoop[l] > 0 ? P.ints[l] * w : (P.ints[l] + 3) / 4 * 4);
         }
-        if (P.dir[l] > 0) s = (int)std::min<int64_t>(s, std::max<int64_t>(4, budget / (P.dir[l] * 4) / 4 * 4));
+        if (P.dir[l] > 0) s = (int)std::min<int64_t>(s, std::max<int64_t>(w, budget / (P.dir[l] * 4)));
+        s = std::max(w, s / w * w);
         S.s[l] = s;
         S.dir_words = std::max(S.dir_words, (int64_t)s * P.dir[l]);
         S.max_slots = std::max<int64_t>(S.max_slots, s);
@@ -1312,7 +1370,6 @@ static cudaError_t launch_plan(const SwPlan& P, const SwSlots& S, const PairDesc
     const int64_t dir_cap = S.dir_words, edge_cap = S.max_slots * P.edge_slot;
     // ctr: [l] list l's item counter, [6] pairs handed over, [7] their counter
     const bool opt = trace && P.n_opt > 0 && esc_list && S.s_esc > 0;
-    const int64_t coop = T.sw_coop_log2 < 40 ? ((int64_t)1 << T.sw_coop_log2) : -1;
     int64_t base = 0;
     if (P.ints[SP_L16] > 0) {
         Sw16Args A;
@@ -1321,16 +1378,15 @@ static cudaError_t launch_plan(const SwPlan& P, const SwSlots& S, const PairDesc
         A.out_score = out_score; A.out_pos = out_pos; A.out_len = out_len; A.out_cigar = out_cigar;
         A.dirs = dirs; A.dir_slot = P.dir[SP_L16]; A.edge = edge; A.edge_slot = P.edge_slot;
         A.counter = ctr + SP_L16; A.err = err;
-        A.coop_cells = coop;
+        A.ncoop = (int32_t)P.ncoop[SP_L16];
         if (dplan) { A.plan = dplan; A.plan_list = SP_L16; A.dir_cap = dir_cap; A.edge_cap = 0; }
         if (opt) {
             A.ovf_limit = sw16_overflow_limit(sc.match);
             A.esc_list = esc_list;
             A.esc_count = ctr + 6;
         }
-        const bool blocks = A.coop_cells >= 0 && P.max16_cells > A.coop_cells;
-        const cudaError_t e = trace ? launch_sw16ck(A, S.s[SP_L16], T.sw_window, blocks, st)
-                                    : launch_sw16so(A, S.s[SP_L16], st);
+        const cudaError_t e = trace ? launch_sw16ck(A, S.s[SP_L16], T.sw_window, P.w[SP_L16], st)
+                                    : launch_sw16so(A, S.s[SP_L16], P.w[SP_L16], st);
         if (e != cudaSuccess) return e;
         if (opt) {
             // the pairs the 16-bit kernel handed over, on the 32-bit long shape
@@ -1340,9 +1396,9 @@ static cudaError_t launch_plan(const SwPlan& P, const SwSlots& S, const PairDesc
             B.out_score = out_score; B.out_pos = out_pos; B.out_len = out_len; B.out_cigar = out_cigar;
             B.dirs = dirs; B.dir_slot = P.dir_opt; B.edge = edge; B.edge_slot = P.edge_slot;
             B.counter = ctr + 7; B.err = err;
-            B.coop_cells = coop;
+            B.coop_cells = sw_coop_limit(T);
             if (dplan) { B.plan = dplan; B.plan_list = SP_ESC; B.dir_cap = dir_cap; B.edge_cap = 0; }
-            const cudaError_t e2 = launch_sw32ck(B, true, S.s_esc, st);
+            const cudaError_t e2 = launch_sw32ck(B, true, S.s_esc, 4, st);
             if (e2 != cudaSuccess) return e2;
         }
     }
@@ -1355,7 +1411,7 @@ static cudaError_t launch_plan(const SwPlan& P, const SwSlots& S, const PairDesc
             A.out_score = out_score; A.out_pos = out_pos; A.out_len = out_len; A.out_cigar = out_cigar;
             A.dirs = dirs; A.dir_slot = P.dir[l]; A.edge = edge; A.edge_slot = P.edge_slot;
             A.counter = ctr + l; A.err = err;
-            A.coop_cells = l == SP_L32LONG ? coop : -1;
+            A.ncoop = (int32_t)P.ncoop[l];
             if (dplan) {
                 A.plan = dplan;
                 A.plan_list = l;
@@ -1363,7 +1419,7 @@ static cudaError_t launch_plan(const SwPlan& P, const SwSlots& S, const PairDesc
                 A.dir_cap = trace ? dir_cap : 0;
                 A.edge_cap = trace ? 0 : edge_cap;
             }
-            const cudaError_t e = trace ? launch_sw32ck(A, l == SP_L32LONG, S.s[l], st) : launch_sw(A, S.s[l], st);
+            const cudaError_t e = trace ? launch_sw32ck(A, l == SP_L32LONG, S.s[l], P.w[l], st) : launch_sw(A, S.s[l], st);
             if (e != cudaSuccess) return e;
         }
         base += P.ints[l];
@@ -1421,7 +1477,10 @@ static int32_t sw_batch_range(const ga_sw_request* reqs, int32_t n, int64_t base
     // quarters of the device's blocks: the next range's pack and plan kernels
     // then find room while this range runs, instead of waiting for its tail
     // (200,000-pair batch end to end: 30.2 -> 29.7 ms; half the blocks: 30.3).
-    if (parts > 1 && S.s[SP_L16] > 0) S.s[SP_L16] = std::max(4, S.s[SP_L16] * 3 / 4 / 4 * 4);
+    if (parts > 1 && S.s[SP_L16] > 0) {
+        const int w = P.w[SP_L16];
+        S.s[SP_L16] = std::max(w, S.s[SP_L16] * 3 / 4 / w * w);
+    }
 
     // Host staging: [descriptors (span offsets) | arena] in, [score pos len
     // checks err | packed CIGARs] back.  Device: the same blocks, then the CIGAR
@@ -1528,7 +1587,8 @@ static int32_t sw_batch_range(const ga_sw_request* reqs, int32_t n, int64_t base
         if (e == cudaSuccess) e = launch_pack(D, arena, nullptr, dpure, st);
         if (e == cudaSuccess && route) e = launch_sw_route(D, s0.match, s0.gap_open, dfeat, dy, dtry, st);
         if (e == cudaSuccess)
-            e = enqueue_plan_sw(D, s0, trace, trace ? cell_limit : -1, -1, dsc, dwork, dscr, dres, T, st, dtry);
+            e = enqueue_plan_sw(D, s0, trace, trace ? cell_limit : -1, -1, dsc, dwork, dscr, dres, T, st, dtry,
+                                &P);
         if (e == cudaSuccess)
             e = launch_plan(P, S, D, s0, trace, T, dwork, dsc, dpos, dln, dcg, ddirs, dedge, dctr, der, st, dscr, dres);
         if (e == cudaSuccess && trace)
@@ -1551,7 +1611,8 @@ static int32_t sw_batch_range(const ga_sw_request* reqs, int32_t n, int64_t base
                 (uint64_t)T.sw_pack16 | (uint64_t)T.sw_window << 8 | (uint64_t)T.sw_long_log2 << 16 |
                     (uint64_t)T.sw_coop_log2 << 24 | (uint64_t)T.sw_opt16_pct << 32,
                 (uint64_t)P.ints[0], (uint64_t)P.ints[1], (uint64_t)P.ints[2], (uint64_t)P.dir[0],
-                (uint64_t)P.dir[1], (uint64_t)P.dir[2], (uint64_t)P.edge_slot, (uint64_t)P.max16_cells,
+                (uint64_t)P.dir[1], (uint64_t)P.dir[2], (uint64_t)P.edge_slot,
+                (uint64_t)P.w[0] | (uint64_t)P.w[1] << 8 | (uint64_t)P.w[2] << 16 | (uint64_t)(P.ncoop[0] > 0) << 24,
                 (uint64_t)P.n_opt, (uint64_t)P.dir_opt, (uint64_t)S.dir_words, (uint64_t)S.max_slots,
                 (uint64_t)S.s[0] | (uint64_t)S.s[1] << 32, (uint64_t)S.s[2] | (uint64_t)S.s_esc << 32};
             le = replay_graph(c->swexec, c->swkey, key, c->swlaunches, c->stream, enqueue);
@@ -2143,8 +2204,7 @@ int32_t ga_sw_device_ex(const ga_device_batch* b, ga_sw_scoring sc, int32_t trac
         return device_plan_sw(D, sc, trace != 0, cell_limit, -2, out_score, dwork, dscr, dres, hres, T, st, P, dtry) ==
                cudaSuccess;
     };
-    if (!plan()) return fail(E_LAUNCH);
-    const SwSlots S = size_sw(P, trace != 0, T, c->sm_count, sw_dir_budget(c, 1));
+    SwSlots S;
     auto run_layout = [&](char* base, int32_t** ctr, int32_t** edge, uint32_t** dirs) {
         Carve k(base);
         k.off = plan_bytes;
@@ -2155,9 +2215,16 @@ int32_t ga_sw_device_ex(const ga_device_batch* b, ga_sw_scoring sc, int32_t trac
     };
     int32_t *dctr, *dedge;
     uint32_t* ddirs;
-    const uint64_t gen_before = c->dev_gen;
-    if (!ensure_dev(c, run_layout(nullptr, &dctr, &dedge, &ddirs))) return fail(E_ALLOC);
-    if (c->dev_gen != gen_before && !plan()) return fail(E_LAUNCH);      // the arena moved: plan again in the new one
+    // An arena that has to grow moves, and the plan with it.  The new plan may pair the
+    // 16-bit list's neighbours otherwise (equal buckets fill in no order) and need a
+    // little more, so it is sized again, with room to spare.
+    for (int attempt = 0;; ++attempt) {
+        if (!plan()) return fail(E_LAUNCH);
+        S = size_sw(P, trace != 0, T, c->sm_count, sw_dir_budget(c, 1));
+        const size_t need = run_layout(nullptr, &dctr, &dedge, &ddirs);
+        if (need <= c->dev_cap) break;
+        if (attempt == 4 || !ensure_dev(c, need + need / 32)) return fail(E_ALLOC);
+    }
     run_layout(c->dev, &dctr, &dedge, &ddirs);
     if (graph) {
         // the launches of this shape in plan mode, captured with the memsets,
@@ -2170,7 +2237,8 @@ int32_t ga_sw_device_ex(const ga_device_batch* b, ga_sw_scoring sc, int32_t trac
             if (x == cudaSuccess) x = launch_pack(D, b->seq_bytes, nullptr, dpure, st);
             if (x == cudaSuccess && route) x = launch_sw_route(D, sc.match, sc.gap_open, dfeat, dy, dtry, st);
             if (x == cudaSuccess)
-                x = enqueue_plan_sw(D, sc, true, cell_limit, -2, out_score, dwork, dscr, dres, T, st, dtry);
+                x = enqueue_plan_sw(D, sc, true, cell_limit, -2, out_score, dwork, dscr, dres, T, st, dtry,
+                                    &P);
             if (x == cudaSuccess)
                 x = launch_plan(P, S, D, sc, true, T, dwork, out_score, out_pos, out_len, out_cigar, ddirs, dedge, dctr,
                                 dctr + 32, st, dscr, dres);

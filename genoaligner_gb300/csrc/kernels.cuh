@@ -41,7 +41,8 @@ struct SwArgs {
     int64_t edge_slot;
     int32_t* counter;
     int32_t* err;
-    int64_t coop_cells = -1; // sw32ck: items above this many cells run on a whole block (< 0: none)
+    int32_t ncoop = 0;       // sw32ck: the list's first ncoop items run on a whole block each
+    int64_t coop_cells = -1; // ... and, when >= 0, the leading items above this many cells instead
     const int32_t* nwork_dev = nullptr;   // when set, the item count is read here at launch (device)
     // Sizes read on the device (no plan read back before the launch): when
     // plan is set, list plan_list of the device-built plan (plan_view) gives
@@ -69,7 +70,7 @@ struct Sw16Args {
     int64_t edge_slot;
     int32_t* counter;
     int32_t* err;
-    int64_t coop_cells = -1; // sw16ck: items above this many cells run on a whole block (< 0: none)
+    int32_t ncoop = 0;       // sw16ck: the list's first ncoop items run on a whole block each
     int32_t ovf_limit = 1 << 30;          // a pair whose best reaches this is handed over ...
     int32_t* esc_list = nullptr;          // ... to the 32-bit kernel: appended here
     int32_t* esc_count = nullptr;
@@ -170,13 +171,17 @@ cudaError_t launch_sw(const SwArgs& A, int slots, cudaStream_t st);
 // list (sw32ck long shape; traceback only).  The record `res` (SP_RES long longs):
 // per list its pair count, its length in the flattened work array and its
 // offset there, the largest per-warp memory of its items (32-bit words), the
-// band-edge slot (2 * the longest text), the 16-bit list's largest item
-// (larger row count x larger column count of its two pairs), and the pairs
-// taken on the optimistic 16-bit rule only: their count and the largest
-// per-warp memory the 32-bit long-shape kernel would need for them.
+// band-edge slot (2 * the longest text), the pairs
+// taken on the optimistic 16-bit rule only (their count and the largest
+// per-warp memory the 32-bit long-shape kernel would need for them), and per list
+// its cells, its largest pair's, the most columns, how many of its leading items run on
+// a whole block (sp_coop_cells) and the warps of such a block.
+// Such an item has all shares of its block's memory, so its part of one (sw_coop_share)
+// counts as its per-warp memory.
 constexpr int SP_LISTS = 3, SP_L16 = 0, SP_L32 = 1, SP_L32LONG = 2;
-constexpr int SP_COUNT = 0, SP_INTS = 3, SP_BASE = 6, SP_DIR = 9, SP_EDGE = 12, SP_MAXC16 = 13, SP_NOPT = 14,
-              SP_DIROPT = 15, SP_RES = 16;
+constexpr int SP_COUNT = 0, SP_INTS = 3, SP_BASE = 6, SP_DIR = 9, SP_EDGE = 12, SP_NOPT = 13,
+              SP_DIROPT = 14, SP_CELLS = 15, SP_NCOOP = 18, SP_LARGEST = 21, SP_COLS = 24, SP_COOPW = 27,
+              SP_RES = 30;
 // plan_list of the launch that takes the pairs the 16-bit kernel hands over
 constexpr int SP_ESC = SP_LISTS;
 
@@ -184,20 +189,21 @@ constexpr int SP_ESC = SP_LISTS;
 // With one: the list's items (work0 + its base in the flattened lists; the
 // hand-over list: work0 itself and the count at nwork_dev), item count and
 // per-warp memory from the record, and whether this block runs: blocks past
-// dir_cap / (4 * dir_slot) (and edge_cap / (4 * edge_slot)) return at once.
-// A list whose one block of 4 warps does not fit runs nowhere and sets
+// dir_cap / (warps * dir_slot) (and edge_cap / (warps * edge_slot)) return at once.
+// A list whose one block does not fit runs nowhere and sets
 // ERR_SCRATCH.
 struct PlanView {
     const int32_t* work;
     int nwork;
     int64_t dir_slot, edge_slot;
     bool run;
+    int ncoop;
 };
 __device__ __forceinline__ PlanView plan_view(const long long* plan, int list, const int32_t* work0, int nwork0,
                                               const int32_t* nwork_dev, int64_t dir_slot0, int64_t edge_slot0,
                                               int64_t dir_cap, int64_t edge_cap, int32_t* err)
 {
-    PlanView v{work0, nwork_dev ? *nwork_dev : nwork0, dir_slot0, edge_slot0, true};
+    PlanView v{work0, nwork_dev ? *nwork_dev : nwork0, dir_slot0, edge_slot0, true, 0};
     if (!plan) return v;
     if (list == SP_ESC) {
         v.dir_slot = (plan[SP_DIROPT] + 3) / 4 * 4;
@@ -206,11 +212,12 @@ __device__ __forceinline__ PlanView plan_view(const long long* plan, int list, c
         v.work = work0 + plan[SP_BASE + list];
         v.nwork = (int)(list == SP_L16 ? ints / 2 : ints);
         v.dir_slot = (plan[SP_DIR + list] + 3) / 4 * 4;
+        v.ncoop = (int)plan[SP_NCOOP + list];
     }
     v.edge_slot = plan[SP_EDGE] > 2 ? plan[SP_EDGE] : 2;
     long long blocks = gridDim.x;
-    if (v.dir_slot > 0) blocks = min(blocks, (long long)(dir_cap / (4 * v.dir_slot)));
-    if (edge_cap > 0) blocks = min(blocks, (long long)(edge_cap / (4 * v.edge_slot)));
+    if (v.dir_slot > 0) blocks = min(blocks, (long long)(dir_cap / ((blockDim.x >> 5) * v.dir_slot)));
+    if (edge_cap > 0) blocks = min(blocks, (long long)(edge_cap / ((blockDim.x >> 5) * v.edge_slot)));
     if (blocks < 1 && v.nwork > 0 && blockIdx.x == 0 && threadIdx.x == 0) atomicOr(err, ERR_SCRATCH);
     v.run = blockIdx.x < blocks;
     return v;
@@ -225,6 +232,10 @@ struct SwPlanArgs {
     const uint8_t* try16 = nullptr;   // when set: the optimistic rule per pair (the SW model's routing) instead
     int32_t long_log2;           // sw32ck long shape above 2^long_log2 cells
     int32_t too_large_score;     // score written for pairs above cell_limit
+    int64_t coop_limit;          // items above this many cells run on a whole block (sp_coop_cells; < 0: none do)
+    int32_t coop_warps[SP_LISTS];     // per list: resident warps of its kernel, 0 if it has no whole-block phase
+    int32_t coop_block[SP_LISTS];     // ... and the warps of such a block, 0: chosen here (sw_coop_block)
+    int32_t sms;
     int32_t score_only;          // 1: lists of the score-only kernels (sw16so, sw_kernel)
     int32_t* out_score;
     int32_t* work;               // flattened work lists (2n + 8 ints)
@@ -242,11 +253,11 @@ cudaError_t launch_sw_validate(const PairDesc& D, const ga_sw_scoring_t& sc, con
 // sw32ck has a short-pair shape and a long-pair shape (sw32ck_long); sizes
 // in sw_sizes.cuh.
 int sw32ck_max_slots(bool long_pairs, int sm_count);
-cudaError_t launch_sw32ck(const SwArgs& A, bool long_pairs, int slots, cudaStream_t st);
+cudaError_t launch_sw32ck(const SwArgs& A, bool long_pairs, int slots, int warps, cudaStream_t st);
 int sw16ck_max_slots(int sm_count, int window);
 int sw16so_max_slots(int sm_count);
-cudaError_t launch_sw16so(const Sw16Args& A, int slots, cudaStream_t st);
-// blocks: the variant with the whole-block phase (items above A.coop_cells)
-cudaError_t launch_sw16ck(const Sw16Args& A, int slots, int window, bool blocks, cudaStream_t st);
+cudaError_t launch_sw16so(const Sw16Args& A, int slots, int warps, cudaStream_t st);
+// warps: per block, slots a multiple of it; A.ncoop > 0 (with a plan: if any) takes the whole-block variant
+cudaError_t launch_sw16ck(const Sw16Args& A, int slots, int window, int warps, cudaStream_t st);
 
 }  // namespace ga

@@ -206,15 +206,15 @@ __device__ __forceinline__ void q9_resolve(const uint32_t* src, int& pend, int v
 // COOP: the band is one of an item's bands run by the warps of a block
 // together (fwd16_coop); the warp then meets the block's barrier after every
 // 32 steps, ceil((M + 31) / 32) times per band.
-// Q9: the score-only form (sw16so_kernel): no checkpoint rows, and per pair
-// the best value with the end-cell key of the reference's score-only kernel
-// (c9_key) in (r, c) as its high and low words.
-template <int CB, bool COOP, bool Q9 = false>
-__device__ void fwd_band(const FwdCtx& X, int b0, int t, int& vA, int& rA, int& cA, int& vB, int& rB, int& cB,
-                         int* pend = nullptr)
+// The score-only form: no checkpoint rows, and per pair the best value with
+// the end-cell key of the reference's score-only kernel (c9_key) in (r, c) as
+// its high and low words.
+template <int CB, bool COOP>
+__device__ void fwd_band_so(const FwdCtx& X, int b0, int t, int& vA, int& rA, int& cA, int& vB, int& rB, int& cB,
+                            int* pend)
 {
     constexpr int NH = CB / 2;
-    const uint32_t MIN2 = 0x80008000u, K2 = 0x80008000u;
+    const uint32_t MIN2 = 0x80008000u;
     const uint32_t NGO2 = X.NGO2, NGE2 = X.NGE2;
     const int M = X.M, mA = X.mA, mB = X.mB;
     const int j0 = b0 + t * CB;
@@ -223,15 +223,13 @@ __device__ void fwd_band(const FwdCtx& X, int b0, int t, int& vA, int& rA, int& 
     uint32_t hgu[CB], fv[CB];
 #pragma unroll
     for (int c = 0; c < CB; ++c) { hgu[c] = NGO2; fv[c] = 0u; }
-    uint32_t validA = 0u, validB = 0u;                     // Q9: the pairs' columns, in key order
-    uint32_t* rowsA = Q9 ? X.rows + t * CK_C : nullptr;
-    uint32_t* rowsB = Q9 ? X.rows + (32 + t) * CK_C : nullptr;
-    if constexpr (Q9) {
+    uint32_t validA = 0u, validB = 0u;                     // the pairs' columns, in key order
+    uint32_t* rowsA = X.rows + t * CK_C;
+    uint32_t* rowsB = X.rows + (32 + t) * CK_C;
 #pragma unroll
-        for (int c = 0; c < CB; ++c) {
-            validA |= (uint32_t)(c < nvA) << q9_rank<CB>(c);
-            validB |= (uint32_t)(c < nvB) << q9_rank<CB>(c);
-        }
+    for (int c = 0; c < CB; ++c) {
+        validA |= (uint32_t)(c < nvA) << q9_rank<CB>(c);
+        validB |= (uint32_t)(c < nvB) << q9_rank<CB>(c);
     }
     uint32_t diag_in = NGO2, out_hg = NGO2, out_e = 0u;
     // left boundary: the column edge at column b0
@@ -251,7 +249,6 @@ __device__ void fwd_band(const FwdCtx& X, int b0, int t, int& vA, int& rA, int& 
     };
     uint32_t rb_off = 0u, rb_hg = NGO2, rb_e = 0u;       // this lane's row of the current 32
     uint32_t ch = 0;
-    uint32_t bmax = 0u, brow = 0u;                        // this band: best and its first row, per half
     const int steps = M + 31;
     for (int tau = 0; tau < steps; ++tau) {
         if ((tau & 31) == 0 && tau < M) {
@@ -264,12 +261,10 @@ __device__ void fwd_band(const FwdCtx& X, int b0, int t, int& vA, int& rA, int& 
                     rb_e = lv.y;
                 }
             }
-            if constexpr (Q9) {
-                // the pairs' best so far over the warp: a lower bound of their
-                // final best, below which no cell can be the end cell
-                pend[2] = __reduce_max_sync(FULL, vA);
-                pend[3] = __reduce_max_sync(FULL, vB);
-            }
+            // the pairs' best so far over the warp: a lower bound of their
+            // final best, below which no cell can be the end cell
+            pend[2] = __reduce_max_sync(FULL, vA);
+            pend[3] = __reduce_max_sync(FULL, vB);
         }
         uint32_t in_hg = __shfl_up_sync(FULL, out_hg, 1);
         uint32_t in_e = __shfl_up_sync(FULL, out_e, 1);
@@ -315,74 +310,50 @@ __device__ void fwd_band(const FwdCtx& X, int b0, int t, int& vA, int& rA, int& 
         out_hg = hgl;
         out_e = el;
         if (eout) *reinterpret_cast<uint2*>(eout + 2 * (i - 1)) = make_uint2(out_hg, out_e);
-        if constexpr (Q9) {
-            // a row whose maximum reaches a pair's best so far: that maximum
-            // sits in a column of the pair (padding columns score PAD and
-            // trail the pair's last column by a gap).  A raise stores the row
-            // and defers its key; a tie takes the keys of both rows.
-            const int ra = lo16s(rowmax), rb = hi16s(rowmax);
-            const bool ka = ra > 0 && ra >= max(vA, pend[2]) && i <= X.mA;
-            const bool kb = rb > 0 && rb >= max(vB, pend[3]) && i <= X.mB;
-            if (ka || kb) {
-                if (ka) {
-                    if (ra > vA) {
-                        vA = ra; rA = cA = -1; pend[0] = i;
-                        q9_store<CB>(rowsA, hgu);
-                    } else {
-                        q9_resolve<CB>(rowsA, pend[0], vA, 0, j0, X.GO2, validA, rA, cA);
-                        q9_merge_row<CB>(hgu, i, vA, 0, j0, X.GO2, validA, rA, cA);
-                    }
-                }
-                if (kb) {
-                    if (rb > vB) {
-                        vB = rb; rB = cB = -1; pend[1] = i;
-                        q9_store<CB>(rowsB, hgu);
-                    } else {
-                        q9_resolve<CB>(rowsB, pend[1], vB, 1, j0, X.GO2, validB, rB, cB);
-                        q9_merge_row<CB>(hgu, i, vB, 1, j0, X.GO2, validB, rB, cB);
-                    }
+        // a row whose maximum reaches a pair's best so far: that maximum
+        // sits in a column of the pair (padding columns score PAD and
+        // trail the pair's last column by a gap).  A raise stores the row
+        // and defers its key; a tie takes the keys of both rows.
+        const int ra = lo16s(rowmax), rb = hi16s(rowmax);
+        const bool ka = ra > 0 && ra >= max(vA, pend[2]) && i <= X.mA;
+        const bool kb = rb > 0 && rb >= max(vB, pend[3]) && i <= X.mB;
+        if (ka || kb) {
+            if (ka) {
+                if (ra > vA) {
+                    vA = ra; rA = cA = -1; pend[0] = i;
+                    q9_store<CB>(rowsA, hgu);
+                } else {
+                    q9_resolve<CB>(rowsA, pend[0], vA, 0, j0, X.GO2, validA, rA, cA);
+                    q9_merge_row<CB>(hgu, i, vA, 0, j0, X.GO2, validA, rA, cA);
                 }
             }
-        } else {
-        if ((i & (CK_K - 1)) == 0 && i < M) {                     // checkpoint row i
-            uint4* dst = reinterpret_cast<uint4*>(X.ck + 2 * ((int64_t)(i / CK_K - 1) * X.ncol + j0));
-#pragma unroll
-            for (int c = 0; c < CB; c += 2) dst[c >> 1] = make_uint4(hgu[c], fv[c], hgu[c + 1], fv[c + 1]);
-        }
-        // strict improvement per half (bits 15 / 31 of d clear): this band's
-        // best and the first row holding it; the column is found when the walk
-        // recomputes that row
-        const uint32_t d = bmax - rowmax + K2;
-        const uint32_t imp = ((~d & K2) >> 15) * 0xffffu;
-        bmax = __vmaxs2(bmax, rowmax);
-        brow = (brow & ~imp) | ((uint32_t)i * 0x10001u & imp);
+            if (kb) {
+                if (rb > vB) {
+                    vB = rb; rB = cB = -1; pend[1] = i;
+                    q9_store<CB>(rowsB, hgu);
+                } else {
+                    q9_resolve<CB>(rowsB, pend[1], vB, 1, j0, X.GO2, validB, rB, cB);
+                    q9_merge_row<CB>(hgu, i, vB, 1, j0, X.GO2, validB, rB, cB);
+                }
+            }
         }
         }
         if (COOP && ((tau & 31) == 31 || tau == steps - 1)) __syncthreads();
     }
-    if constexpr (Q9) {                                   // the band's pending rows
-        q9_resolve<CB>(rowsA, pend[0], vA, 0, j0, X.GO2, validA, rA, cA);
-        q9_resolve<CB>(rowsB, pend[1], vB, 1, j0, X.GO2, validB, rB, cB);
-    } else {
-        // merge the band into the lane's best; the column kept is the first of
-        // the lane's span in this band (spans order like their columns)
-        const int v = lo16s(bmax), r = (int)(brow & 0xffffu);
-        if (v > 0 && ck_better(v, r, j0 + 1, vA, rA, cA)) { vA = v; rA = r; cA = j0 + 1; }
-        const int v2 = hi16s(bmax), r2 = (int)(brow >> 16);
-        if (v2 > 0 && ck_better(v2, r2, j0 + 1, vB, rB, cB)) { vB = v2; rB = r2; cB = j0 + 1; }
-    }
+    // the band's pending rows
+    q9_resolve<CB>(rowsA, pend[0], vA, 0, j0, X.GO2, validA, rA, cA);
+    q9_resolve<CB>(rowsB, pend[1], vB, 1, j0, X.GO2, validB, rB, cB);
     __syncwarp();
 }
 
-// fwd_band's traceback form for a warp alone, two rows per step: lane t
+// The traceback form, two rows per step (COOP as above, ceil(((M + 1) / 2 + 31) / 32)
+// barriers per band): lane t
 // takes rows i = 2 (tau - t) + 1 and i + 1 of its CB columns.  Row i + 1's
 // cell in column c needs only row i's cells in columns c - 1 and c, so the
 // two rows' dependency chains (E along a row, H through E) are independent at
 // equal column and interleave: twice the independent integer work per lane
-// between the same per-row shuffles and profile reads.  Values, checkpoint
-// rows, column edges and the best (value, first row) per pair are
-// fwd_band's exactly.
-template <int CB>
+// between the same per-row shuffles and profile reads.
+template <int CB, bool COOP>
 __device__ void fwd_band2(const FwdCtx& X, int b0, int t, int& vA, int& rA, int& cA, int& vB, int& rB, int& cB)
 {
     constexpr int NH = CB / 2;
@@ -518,6 +489,7 @@ __device__ void fwd_band2(const FwdCtx& X, int b0, int t, int& vA, int& rA, int&
                 brow = (brow & ~imp) | ((uint32_t)(i + 1) * 0x10001u & imp);
             }
         }
+        if (COOP && ((tau & 31) == 31 || tau == steps - 1)) __syncthreads();
     }
     const int v = lo16s(bmax), r = (int)(brow & 0xffffu);
     if (v > 0 && ck_better(v, r, j0 + 1, vA, rA, cA)) { vA = v; rA = r; cA = j0 + 1; }
@@ -547,41 +519,49 @@ __device__ __forceinline__ void ck_profile_tile(uint32_t* prof, const uint8_t* p
     }
 }
 
-// The forward pass of one item by the 4 warps of a block: band b runs on warp
-// b % 4, starting at 32-step chunk start(b) = max(start(b-1) + 2, start(b-4) +
-// chunks per band), so each band's first lane reads the left edge of rows
-// 32c+1 .. 32c+32 (written by the band before it up to its step 32c + 62)
-// after the barrier that closed that band's chunk c + 1, and each warp runs
-// its bands one after the other.  Every warp meets the block barrier once per
-// chunk, idle or not: start(last band) + chunks per band times in all.
+// The forward pass of one item by the W = blockDim / 32 warps of a block: band b runs
+// on warp b % W, starting at 32-step chunk start(b) = max(start(b-1) + 2, start(b-W) +
+// chunks per band) = (b / W) * max(chunks, 2 W) + 2 (b % W), so each band's first lane
+// reads the left edge of a chunk's rows (written by the band before it, by its last
+// lane 31 steps later) after the barrier that closed that band's next chunk, and each
+// warp runs its bands one after the other.  Every warp meets the block barrier once
+// per chunk, idle or not: start(last band) + chunks in all.  Bands narrow (CB columns
+// a lane, coop_cb) when the full ones would leave warps idle.
+// SO: the score-only bands (one row a step, two otherwise).
+template <bool SO>
 __device__ void fwd16_coop(const FwdCtx& X, int N, int t, int wib, int& vA, int& rA, int& cA, int& vB, int& rB,
-                           int& cB)
+                           int& cB, int* pend)
 {
-    const int nck = (X.M + 62) / 32;                  // ceil((M + 31) / 32)
-    int g = 0, prev = -2, b = 0;
-    int st4[4] = {0, 0, 0, 0};
+    const int W = blockDim.x >> 5;
+    const int nck = ((SO ? X.M : (X.M + 1) / 2) + 62) / 32;      // ceil(steps / 32)
+    const int full = coop_cb(N, W, nck, 4);
+    int g = 0, b = 0, s = 0;
     for (int b0 = 0; b0 < N; ++b) {
         const int rest = N - b0;
-        const int cb = rest > CK_BW ? CK_C : ck_last_cb(rest);
-        const int s = max(prev + 2, b >= 4 ? st4[b & 3] + nck : 0);
-        prev = s;
-        st4[b & 3] = s;
-        if ((b & 3) == wib) {
+        const int cb = rest > 32 * full ? full : ck_last_cb(rest);
+        s = (b / W) * max(nck, 2 * W) + 2 * (b % W);
+        if (b % W == wib) {
             for (; g < s; ++g) __syncthreads();
-            if (cb == 16) fwd_band<16, true>(X, b0, t, vA, rA, cA, vB, rB, cB);
-            else if (cb == 8) fwd_band<8, true>(X, b0, t, vA, rA, cA, vB, rB, cB);
-            else if (cb == 4) fwd_band<4, true>(X, b0, t, vA, rA, cA, vB, rB, cB);
-            else fwd_band<2, true>(X, b0, t, vA, rA, cA, vB, rB, cB);
+            if constexpr (SO) {
+                if (cb == 16) fwd_band_so<16, true>(X, b0, t, vA, rA, cA, vB, rB, cB, pend);
+                else if (cb == 8) fwd_band_so<8, true>(X, b0, t, vA, rA, cA, vB, rB, cB, pend);
+                else if (cb == 4) fwd_band_so<4, true>(X, b0, t, vA, rA, cA, vB, rB, cB, pend);
+                else fwd_band_so<2, true>(X, b0, t, vA, rA, cA, vB, rB, cB, pend);
+            } else {
+                if (cb == 16) fwd_band2<16, true>(X, b0, t, vA, rA, cA, vB, rB, cB);
+                else if (cb == 8) fwd_band2<8, true>(X, b0, t, vA, rA, cA, vB, rB, cB);
+                else if (cb == 4) fwd_band2<4, true>(X, b0, t, vA, rA, cA, vB, rB, cB);
+                else fwd_band2<2, true>(X, b0, t, vA, rA, cA, vB, rB, cB);
+            }
             g += nck;
         }
         b0 += 32 * cb;
     }
-    const int G = prev + nck;
-    for (; g < G; ++g) __syncthreads();
+    for (; g < s + nck; ++g) __syncthreads();
 }
 
 // One work item (two pairs): the forward pass (by this warp, or by the
-// block's 4 warps when coop), the best cells, the windows and walks (this
+// block's warps when coop), the best cells, the windows and walks (this
 // warp, or warp 0 of the block) and the outputs.  wslot: the item's
 // checkpoint memory (warp 0's slot when coop); prof: this warp's shared
 // memory.  In coop every warp returns after the same barriers; the caller
@@ -624,15 +604,15 @@ __device__ void ck_item(const Sw16Args& A, const int32_t* __restrict__ pwork, in
     {
         FwdCtx X{textA, textB, patA, patB, mA, nA, mB, nB, M, ncol, ck, ce, prof, sm, sx, NGO2, NGE2, GO2};
         if (coop) {
-            fwd16_coop(X, N, t, wib, vA, rA, cA, vB, rB, cB);
+            fwd16_coop<false>(X, N, t, wib, vA, rA, cA, vB, rB, cB, nullptr);
         } else {
             for (int b0 = 0; b0 < N;) {
                 const int rest = N - b0;                          // columns from this band on
                 const int cb = rest > CK_BW ? CK_C : ck_last_cb(rest);
-                if (cb == 16) fwd_band2<16>(X, b0, t, vA, rA, cA, vB, rB, cB);
-                else if (cb == 8) fwd_band2<8>(X, b0, t, vA, rA, cA, vB, rB, cB);
-                else if (cb == 4) fwd_band2<4>(X, b0, t, vA, rA, cA, vB, rB, cB);
-                else fwd_band2<2>(X, b0, t, vA, rA, cA, vB, rB, cB);
+                if (cb == 16) fwd_band2<16, false>(X, b0, t, vA, rA, cA, vB, rB, cB);
+                else if (cb == 8) fwd_band2<8, false>(X, b0, t, vA, rA, cA, vB, rB, cB);
+                else if (cb == 4) fwd_band2<4, false>(X, b0, t, vA, rA, cA, vB, rB, cB);
+                else fwd_band2<2, false>(X, b0, t, vA, rA, cA, vB, rB, cB);
                 b0 += 32 * cb;
             }
         }
@@ -648,7 +628,7 @@ __device__ void ck_item(const Sw16Args& A, const int32_t* __restrict__ pwork, in
         if (ov2 > 0 && ck_better(ov2, orr2, oc2, vB, rB, cB)) { vB = ov2; rB = orr2; cB = oc2; }
     }
     if (coop) {
-        // the block's best per pair: every warp reduces the four warps' bests in the same order
+        // the block's best per pair: every warp reduces the warps' bests in the same order
         if (t == 0) {
             s_best[wib][0] = vA; s_best[wib][1] = rA; s_best[wib][2] = cA;
             s_best[wib][3] = vB; s_best[wib][4] = rB; s_best[wib][5] = cB;
@@ -656,7 +636,7 @@ __device__ void ck_item(const Sw16Args& A, const int32_t* __restrict__ pwork, in
         __syncthreads();
         vA = s_best[0][0]; rA = s_best[0][1]; cA = s_best[0][2];
         vB = s_best[0][3]; rB = s_best[0][4]; cB = s_best[0][5];
-        for (int q = 1; q < 4; ++q) {
+        for (int q = 1; q < (int)(blockDim.x >> 5); ++q) {
             if (s_best[q][0] > 0 && ck_better(s_best[q][0], s_best[q][1], s_best[q][2], vA, rA, cA)) {
                 vA = s_best[q][0]; rA = s_best[q][1]; cA = s_best[q][2];
             }
@@ -1055,31 +1035,32 @@ __device__ void ck_item(const Sw16Args& A, const int32_t* __restrict__ pwork, in
 }
 
 // TG: tiles recomputed per window pass, the walk's and the TG - 1 to its left.
-// Work items come largest first.  Items above A.coop_cells cells (larger row
-// count x larger column count of the two pairs) are taken by a whole block,
-// whose 4 warps share the forward pass; from the first smaller item on, each
-// warp takes items of its own.
+// Work items come largest first.  The first ncoop are taken by a whole block each,
+// whose warps share the forward pass; from the next item on, each warp takes items
+// of its own.
 // BLK: the variant with the whole-block phase; without it every warp takes
 // items of its own and no block barrier is met.
 // PLAN: items and per-warp memory from the device-built plan (plan_view),
 // the list and its length kept in shared memory; otherwise the launch's own.
 template <int TG, bool BLK, bool PLAN>
-__global__ void __launch_bounds__(128, 4) sw16ck_kernel(Sw16Args A)
+__global__ void __launch_bounds__(BLK ? 32 * COOP_MAX_WARPS : 128, BLK ? 1 : 4) sw16ck_kernel(Sw16Args A)
 {
     static_assert(TG == 2 || TG == 4, "tile groups split the warp evenly, window rows are 16-byte vectors");
     extern __shared__ uint32_t ck_smem[];
     __shared__ int s_item;
-    __shared__ int s_best[4][6];
+    __shared__ int s_best[BLK ? COOP_MAX_WARPS : 1][6];
     __shared__ const int32_t* s_work;
     __shared__ int s_nwork;
     const int t = threadIdx.x & 31;
     const int wib = threadIdx.x >> 5;
     int64_t dir_slot = A.dir_slot;
+    int ncoop = A.ncoop;
     if constexpr (PLAN) {
         const PlanView V = plan_view(A.plan, A.plan_list, A.work, A.nwork, nullptr, A.dir_slot, A.edge_slot,
                                      A.dir_cap, A.edge_cap, A.err);
         if (!V.run) return;
         dir_slot = V.dir_slot;
+        ncoop = V.ncoop;
         if (threadIdx.x == 0) { s_work = V.work; s_nwork = V.nwork; }
         __syncthreads();
     }
@@ -1090,7 +1071,7 @@ __global__ void __launch_bounds__(128, 4) sw16ck_kernel(Sw16Args A)
 #define SW16_WORK (PLAN ? s_work : A.work)
 
     // one call site of ck_item, so its body is in the kernel once
-    bool block_phase = BLK && A.coop_cells >= 0;
+    bool block_phase = BLK && ncoop > 0;
     for (;;) {
         int w = -1;
         bool coop = false;
@@ -1100,10 +1081,7 @@ __global__ void __launch_bounds__(128, 4) sw16ck_kernel(Sw16Args A)
             const int wb = s_item;
             __syncthreads();
             if (wb >= SW16_NWORK) break;
-            const int pa = SW16_WORK[2 * wb], pb = SW16_WORK[2 * wb + 1];
-            const int M = max(A.D.a_len[pa], pb >= 0 ? A.D.a_len[pb] : 0);
-            const int N = max(A.D.b_len[pa], pb >= 0 ? A.D.b_len[pb] : 0);
-            if ((int64_t)M * N > A.coop_cells) {
+            if (wb < ncoop) {
                 w = wb;
                 coop = true;
             } else {
@@ -1127,37 +1105,62 @@ __global__ void __launch_bounds__(128, 4) sw16ck_kernel(Sw16Args A)
 // carry the band boundaries), the end cell by the reference's score-only rule
 // (c9_key).  dir_slot = sw16so_dir_words.  Outputs: score, and end_i / end_j
 // (0-based) for a positive score, -1 otherwise; start cells -1.
-template <bool PLAN>
-__global__ void __launch_bounds__(128, 4) sw16so_kernel(Sw16Args A)
+// BLK, whole-block items: as in sw16ck_kernel; a block's rows come before its edges.
+template <bool BLK, bool PLAN>
+__global__ void __launch_bounds__(BLK ? 32 * COOP_MAX_WARPS : 128, BLK ? 1 : 4) sw16so_kernel(Sw16Args A)
 {
     extern __shared__ uint32_t ck_smem[];
     __shared__ const int32_t* s_work;
     __shared__ int s_nwork;
+    __shared__ int s_item;
+    __shared__ int s_best[BLK ? COOP_MAX_WARPS : 1][6];
     const int t = threadIdx.x & 31;
     const int wib = threadIdx.x >> 5;
     int64_t dir_slot = A.dir_slot;
+    int ncoop = A.ncoop;
     if constexpr (PLAN) {
         const PlanView V = plan_view(A.plan, A.plan_list, A.work, A.nwork, nullptr, A.dir_slot, A.edge_slot,
                                      A.dir_cap, A.edge_cap, A.err);
         if (!V.run) return;
         dir_slot = V.dir_slot;
+        ncoop = V.ncoop;
         if (threadIdx.x == 0) { s_work = V.work; s_nwork = V.nwork; }
         __syncthreads();
     }
-    uint32_t* rows = A.dirs + ((int64_t)blockIdx.x * (blockDim.x >> 5) + wib) * dir_slot;
-    uint32_t* ce = rows + SO_ROW_WORDS;
+    uint32_t* wslot = A.dirs + ((int64_t)blockIdx.x * (blockDim.x >> 5) + wib) * dir_slot;
+    uint32_t* bslot = A.dirs + (int64_t)blockIdx.x * (blockDim.x >> 5) * dir_slot;
     uint32_t* prof = ck_smem + wib * CK_WARP_WORDS;
     const int go = A.gap_open, ge = A.gap_extend;
     const int sm = A.match + go, sx = A.mismatch + go;
     const uint32_t NGO2 = ((uint32_t)(-go) & 0xffffu) * 0x10001u;
     const uint32_t NGE2 = ((uint32_t)(-ge) & 0xffffu) * 0x10001u;
     const uint32_t GO2 = (uint32_t)go * 0x10001u;
+    bool block_phase = BLK && ncoop > 0;
     for (;;) {
-        int w = 0;
-        if (t == 0) w = atomicAdd(A.counter, 1);
-        w = __shfl_sync(FULL, w, 0);
-        if (w >= SW16_NWORK) break;
+        int w = -1;
+        bool coop = false;
+        if (block_phase) {
+            if (threadIdx.x == 0) s_item = atomicAdd(A.counter, 1);
+            __syncthreads();
+            const int wb = s_item;
+            __syncthreads();
+            if (wb >= SW16_NWORK) break;
+            if (wb < ncoop) {
+                w = wb;
+                coop = true;
+            } else {
+                block_phase = false;
+                if (wib == 0) w = wb;
+            }
+        }
+        if (!coop && w < 0) {
+            if (t == 0) w = atomicAdd(A.counter, 1);
+            w = __shfl_sync(FULL, w, 0);
+            if (w >= SW16_NWORK) break;
+        }
         __syncwarp();
+        uint32_t* rows = coop ? bslot + wib * SO_ROW_WORDS : wslot;
+        uint32_t* ce = coop ? bslot + (blockDim.x >> 5) * SO_ROW_WORDS : wslot + SO_ROW_WORDS;
         const int pa = SW16_WORK[2 * w];
         const bool has_b = SW16_WORK[2 * w + 1] >= 0;
         const int pb = has_b ? SW16_WORK[2 * w + 1] : pa;
@@ -1168,23 +1171,40 @@ __global__ void __launch_bounds__(128, 4) sw16so_kernel(Sw16Args A)
                  mA, nA, mB, nB, M, ck_ncol(N), nullptr, ce, prof, sm, sx, NGO2, NGE2, GO2, rows};
         int vA = 0, kA1 = -1, kA0 = -1, vB = 0, kB1 = -1, kB0 = -1;    // best and its key (high, low word)
         int pend[4] = {0, 0, 0, 0};      // pending rows of A and B, the warp's best of A and B
-        for (int b0 = 0; b0 < N;) {
-            const int rest = N - b0;
-            const int cb = rest > CK_BW ? CK_C : ck_last_cb(rest);
-            if (cb == 16) fwd_band<16, false, true>(X, b0, t, vA, kA1, kA0, vB, kB1, kB0, pend);
-            else if (cb == 8) fwd_band<8, false, true>(X, b0, t, vA, kA1, kA0, vB, kB1, kB0, pend);
-            else if (cb == 4) fwd_band<4, false, true>(X, b0, t, vA, kA1, kA0, vB, kB1, kB0, pend);
-            else fwd_band<2, false, true>(X, b0, t, vA, kA1, kA0, vB, kB1, kB0, pend);
-            b0 += 32 * cb;
+        if (BLK && coop) {
+            fwd16_coop<true>(X, N, t, wib, vA, kA1, kA0, vB, kB1, kB0, pend);
+        } else {
+            for (int b0 = 0; b0 < N;) {
+                const int rest = N - b0;
+                const int cb = rest > CK_BW ? CK_C : ck_last_cb(rest);
+                if (cb == 16) fwd_band_so<16, false>(X, b0, t, vA, kA1, kA0, vB, kB1, kB0, pend);
+                else if (cb == 8) fwd_band_so<8, false>(X, b0, t, vA, kA1, kA0, vB, kB1, kB0, pend);
+                else if (cb == 4) fwd_band_so<4, false>(X, b0, t, vA, kA1, kA0, vB, kB1, kB0, pend);
+                else fwd_band_so<2, false>(X, b0, t, vA, kA1, kA0, vB, kB1, kB0, pend);
+                b0 += 32 * cb;
+            }
         }
+        auto best = [](int ov, int o1, int o0, int& v, int& k1, int& k0) {
+            if (ov > v || (ov == v && ov > 0 && c9_join(o1, o0) < c9_join(k1, k0))) { v = ov; k1 = o1; k0 = o0; }
+        };
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) {
-            int ov = __shfl_xor_sync(FULL, vA, o), o1 = __shfl_xor_sync(FULL, kA1, o), o0 = __shfl_xor_sync(FULL, kA0, o);
-            if (ov > vA || (ov == vA && ov > 0 && c9_join(o1, o0) < c9_join(kA1, kA0))) { vA = ov; kA1 = o1; kA0 = o0; }
-            ov = __shfl_xor_sync(FULL, vB, o); o1 = __shfl_xor_sync(FULL, kB1, o); o0 = __shfl_xor_sync(FULL, kB0, o);
-            if (ov > vB || (ov == vB && ov > 0 && c9_join(o1, o0) < c9_join(kB1, kB0))) { vB = ov; kB1 = o1; kB0 = o0; }
+            best(__shfl_xor_sync(FULL, vA, o), __shfl_xor_sync(FULL, kA1, o), __shfl_xor_sync(FULL, kA0, o), vA, kA1, kA0);
+            best(__shfl_xor_sync(FULL, vB, o), __shfl_xor_sync(FULL, kB1, o), __shfl_xor_sync(FULL, kB0, o), vB, kB1, kB0);
         }
-        if (t == 0) {
+        if (BLK && coop) {
+            if (t == 0) {
+                s_best[wib][0] = vA; s_best[wib][1] = kA1; s_best[wib][2] = kA0;
+                s_best[wib][3] = vB; s_best[wib][4] = kB1; s_best[wib][5] = kB0;
+            }
+            __syncthreads();
+            if (wib == 0)
+                for (int q = 1; q < (int)(blockDim.x >> 5); ++q) {
+                    best(s_best[q][0], s_best[q][1], s_best[q][2], vA, kA1, kA0);
+                    best(s_best[q][3], s_best[q][4], s_best[q][5], vB, kB1, kB0);
+                }
+        }
+        if (t == 0 && (!coop || wib == 0)) {
 #pragma unroll
             for (int x = 0; x < 2; ++x) {
                 if (x == 1 && !has_b) break;
@@ -1203,37 +1223,35 @@ __global__ void __launch_bounds__(128, 4) sw16so_kernel(Sw16Args A)
     }
 }
 
-static size_t sw16ck_smem() { return (size_t)4 * CK_WARP_WORDS * sizeof(uint32_t); }
+static size_t sw16ck_smem(int warps = 4) { return (size_t)warps * CK_WARP_WORDS * sizeof(uint32_t); }
 
 #undef SW16_NWORK
 #undef SW16_WORK
 
-int sw16so_max_slots(int sm_count)
+// Every variant's shared-memory limit is raised, to its widest block's.
+template <class K>
+static void ck_limits(K plain, K plain_plan, K blk, K blk_plan)
 {
-    // both variants launch with this shared memory: raise both limits
-    blocks_per_sm((const void*)sw16so_kernel<true>, 128, sw16ck_smem());
-    return blocks_per_sm((const void*)sw16so_kernel<false>, 128, sw16ck_smem()) * sm_count * 4;
+    blocks_per_sm((const void*)plain_plan, 128, sw16ck_smem());
+    for (int w = 4; w <= COOP_MAX_WARPS; w *= 2) {
+        blocks_per_sm((const void*)blk, 32 * w, sw16ck_smem(w));
+        blocks_per_sm((const void*)blk_plan, 32 * w, sw16ck_smem(w));
+    }
 }
 
-cudaError_t launch_sw16so(const Sw16Args& A, int slots, cudaStream_t st)
+int sw16so_max_slots(int sm_count)
 {
-    if (A.nwork <= 0 && !A.plan) return cudaSuccess;
-    if (slots < 4) return cudaErrorInvalidValue;
-    launch_begin(K_SW16X2_SCORE, st);
-    if (A.plan) sw16so_kernel<true><<<slots / 4, 128, sw16ck_smem(), st>>>(A);
-    else sw16so_kernel<false><<<slots / 4, 128, sw16ck_smem(), st>>>(A);
-    launch_end(K_SW16X2_SCORE, st);
-    return cudaGetLastError();
+    ck_limits(sw16so_kernel<false, false>, sw16so_kernel<false, true>, sw16so_kernel<true, false>,
+              sw16so_kernel<true, true>);
+    return blocks_per_sm((const void*)sw16so_kernel<false, false>, 128, sw16ck_smem()) * sm_count * 4;
 }
 
 template <int TG>
 static int ck_per_sm()
 {
-    // every variant launches with this shared memory: raise all limits
-    blocks_per_sm((const void*)sw16ck_kernel<TG, false, false>, 128, sw16ck_smem());
-    blocks_per_sm((const void*)sw16ck_kernel<TG, false, true>, 128, sw16ck_smem());
-    blocks_per_sm((const void*)sw16ck_kernel<TG, true, true>, 128, sw16ck_smem());
-    return blocks_per_sm((const void*)sw16ck_kernel<TG, true, false>, 128, sw16ck_smem());
+    ck_limits(sw16ck_kernel<TG, false, false>, sw16ck_kernel<TG, false, true>, sw16ck_kernel<TG, true, false>,
+              sw16ck_kernel<TG, true, true>);
+    return blocks_per_sm((const void*)sw16ck_kernel<TG, false, false>, 128, sw16ck_smem());
 }
 
 int sw16ck_max_slots(int sm_count, int window)
@@ -1241,26 +1259,34 @@ int sw16ck_max_slots(int sm_count, int window)
     return (window == 4 ? ck_per_sm<4>() : ck_per_sm<2>()) * sm_count * 4;
 }
 
-cudaError_t launch_sw16ck(const Sw16Args& A, int slots, int window, bool blocks, cudaStream_t st)
+// A.ncoop > 0: with the whole-block phase.
+template <class K>
+static cudaError_t launch_ck(KernelId id, const Sw16Args& A, int slots, int warps, K plain, K plain_plan, K blk,
+                             K blk_plan, cudaStream_t st)
 {
     if (A.nwork <= 0 && !A.plan) return cudaSuccess;
-    if (window != 2 && window != 4) return cudaErrorInvalidValue;
-    const int grid = (slots + 3) / 4;
-    launch_begin(K_SW16X2_TRACE, st);
-    const bool plan = A.plan != nullptr;
-    if (window == 4) {
-        if (blocks) plan ? sw16ck_kernel<4, true, true><<<grid, 128, sw16ck_smem(), st>>>(A)
-                         : sw16ck_kernel<4, true, false><<<grid, 128, sw16ck_smem(), st>>>(A);
-        else plan ? sw16ck_kernel<4, false, true><<<grid, 128, sw16ck_smem(), st>>>(A)
-                  : sw16ck_kernel<4, false, false><<<grid, 128, sw16ck_smem(), st>>>(A);
-    } else {
-        if (blocks) plan ? sw16ck_kernel<2, true, true><<<grid, 128, sw16ck_smem(), st>>>(A)
-                         : sw16ck_kernel<2, true, false><<<grid, 128, sw16ck_smem(), st>>>(A);
-        else plan ? sw16ck_kernel<2, false, true><<<grid, 128, sw16ck_smem(), st>>>(A)
-                  : sw16ck_kernel<2, false, false><<<grid, 128, sw16ck_smem(), st>>>(A);
-    }
-    launch_end(K_SW16X2_TRACE, st);
+    if (slots < warps || slots % warps != 0) return cudaErrorInvalidValue;
+    const K kernel = A.ncoop > 0 ? (A.plan ? blk_plan : blk) : (A.plan ? plain_plan : plain);
+    launch_begin(id, st);
+    kernel<<<slots / warps, 32 * warps, sw16ck_smem(warps), st>>>(A);
+    launch_end(id, st);
     return cudaGetLastError();
+}
+
+cudaError_t launch_sw16so(const Sw16Args& A, int slots, int warps, cudaStream_t st)
+{
+    return launch_ck(K_SW16X2_SCORE, A, slots, warps, sw16so_kernel<false, false>, sw16so_kernel<false, true>,
+                     sw16so_kernel<true, false>, sw16so_kernel<true, true>, st);
+}
+
+cudaError_t launch_sw16ck(const Sw16Args& A, int slots, int window, int warps, cudaStream_t st)
+{
+    if (window == 4)
+        return launch_ck(K_SW16X2_TRACE, A, slots, warps, sw16ck_kernel<4, false, false>, sw16ck_kernel<4, false, true>,
+                         sw16ck_kernel<4, true, false>, sw16ck_kernel<4, true, true>, st);
+    if (window != 2) return cudaErrorInvalidValue;
+    return launch_ck(K_SW16X2_TRACE, A, slots, warps, sw16ck_kernel<2, false, false>, sw16ck_kernel<2, false, true>,
+                     sw16ck_kernel<2, true, false>, sw16ck_kernel<2, true, true>, st);
 }
 
 }  // namespace ga

@@ -220,36 +220,25 @@ __device__ void fwd32(const Fwd32& X, int t, int& vb, int& rb, int& cb)
     }
 }
 
-// The forward pass of one pair by the W warps of a block (W = blockDim / 32,
-// 4 or 8): band b runs on warp b % W, starting at 32-step chunk start(b) =
-// max(start(b-1) + 2, start(b-W) + chunks per band), so each band's first lane reads the left edge of rows
-// 64c+1 .. 64c+64 (written by the band before it up to its step 32c + 62)
-// after the barrier that closed that band's chunk c + 1, and each warp runs
-// its bands one after the other.  Every warp meets the block barrier once per
-// chunk, idle or not: start(last band) + chunks per band times in all.
+// The forward pass of one pair by the W = blockDim / 32 warps of a block, band b on
+// warp b % W from 32-step chunk start(b) = (b / W) * max(chunks, 2 W) + 2 (b % W) on, so
+// each band's first lane reads the left edge of rows 64c+1 .. 64c+64 (written by the
+// band before it up to its step 32c + 62) after the barrier that closed that band's
+// chunk c + 1, and each warp runs its bands one after the other.  Every warp meets the
+// block barrier once per chunk, idle or not.  Bands narrow (coop_cb) where the column
+// edges, every TW columns, allow it.
 template <bool PROF>
 __device__ void fwd32_coop(const Fwd32& X, int t, int wib, int& vb, int& rb, int& cb)
 {
-    const int W = blockDim.x >> 5;                    // warps of the block (at most C32_MAX_WARPS)
+    const int W = blockDim.x >> 5;
     const int nck = ((X.m + 1) / 2 + 62) / 32;        // chunks per band: ceil(steps / 32)
-    int g = 0, prev = -2, b = 0;
-    int stw[C32_MAX_WARPS];                           // start of the last band of each warp
-#pragma unroll
-    for (int q = 0; q < C32_MAX_WARPS; ++q) stw[q] = 0;
+    const int full = coop_cb(X.n, W, nck, X.TW >= C32_BW ? 16 : 4);
+    int g = 0, b = 0, s = 0;
     for (int b0 = 0; b0 < X.n; ++b) {
         const int rest = X.n - b0;
-        const int w = rest > C32_BW ? C32_C : c32_last_cb(rest);
-        const int ow = b % W;
-        int own = 0;
-#pragma unroll
-        for (int q = 0; q < C32_MAX_WARPS; ++q)
-            if (q == ow) own = stw[q];
-        const int s = max(prev + 2, b >= W ? own + nck : 0);
-        prev = s;
-#pragma unroll
-        for (int q = 0; q < C32_MAX_WARPS; ++q)
-            if (q == ow) stw[q] = s;
-        if (ow == wib) {
+        const int w = rest > 32 * full ? full : c32_last_cb(rest);
+        s = (b / W) * max(nck, 2 * W) + 2 * (b % W);
+        if (b % W == wib) {
             for (; g < s; ++g) __syncthreads();
             if (w == 16) fwd32_band<16, PROF, true>(X, b0, t, vb, rb, cb);
             else if (w == 8) fwd32_band<8, PROF, true>(X, b0, t, vb, rb, cb);
@@ -258,8 +247,7 @@ __device__ void fwd32_coop(const Fwd32& X, int t, int wib, int& vb, int& rb, int
         }
         b0 += 32 * w;
     }
-    const int G = prev + nck;
-    for (; g < G; ++g) __syncthreads();
+    for (; g < s + nck; ++g) __syncthreads();
 }
 
 // Shared memory per warp: the forward profile (4 letters x 4 quads x 32
@@ -271,7 +259,7 @@ __host__ __device__ constexpr int c32_warp_smem_bytes(int K, int CT)
                                                                       : (4 * CT * 32 * 4 + K * 8);
 }
 
-// One pair: the forward pass (by this warp, or by the block's 4 warps when
+// One pair: the forward pass (by this warp, or by the block's warps when
 // coop), the best cell, the walk (this warp, or warp 0 of the block) and the
 // outputs.  wslot: the pair's checkpoint/tile memory (warp 0's slot when
 // coop); wsm: this warp's shared memory.  In coop every warp returns after
@@ -324,7 +312,7 @@ __device__ void c32_pair(const SwArgs& A, int p, bool coop, int wib, int t, uint
         if (ov > 0 && c32_better(ov, orr, oc, vb, rb, cb)) { vb = ov; rb = orr; cb = oc; }
     }
     if (coop) {
-        // the block's best: every warp reduces the four warps' bests in the same order
+        // the block's best: every warp reduces the warps' bests in the same order
         if (t == 0) { s_best[wib][0] = vb; s_best[wib][1] = rb; s_best[wib][2] = cb; }
         __syncthreads();
         vb = s_best[0][0]; rb = s_best[0][1]; cb = s_best[0][2];
@@ -569,28 +557,30 @@ __device__ void c32_pair(const SwArgs& A, int p, bool coop, int wib, int t, uint
     }
 }
 
-// Work items come largest first.  Items above A.coop_cells cells are taken by
-// a whole block (its 4 warps share the forward pass); from the first smaller
-// item on, each warp takes items of its own.
+// Work items come largest first.  The first ncoop (A.coop_cells >= 0: the leading
+// ones above that many cells) are taken by a whole block each (its warps share the
+// forward pass); from the next item on, each warp takes items of its own.
 // PLAN: items and per-warp memory from the device-built plan (plan_view),
 // the list and its length kept in shared memory; otherwise the launch's own.
 template <int K, int CT, bool PLAN>
-__global__ void __launch_bounds__(128, 4) sw32ck_kernel(SwArgs A)
+__global__ void __launch_bounds__(32 * COOP_MAX_WARPS, 1) sw32ck_kernel(SwArgs A)
 {
     constexpr int WSB = c32_warp_smem_bytes(K, CT);
     extern __shared__ int4 c32_smem[];
     __shared__ int s_item;
-    __shared__ int s_best[C32_MAX_WARPS][3];
+    __shared__ int s_best[COOP_MAX_WARPS][3];
     __shared__ const int32_t* s_work;
     __shared__ int s_nwork;
     const int t = threadIdx.x & 31;
     const int wib = threadIdx.x >> 5;
     int64_t dir_slot = A.dir_slot;
+    int ncoop = A.ncoop;
     if constexpr (PLAN) {
         const PlanView V = plan_view(A.plan, A.plan_list, A.work, A.nwork, A.nwork_dev, A.dir_slot, A.edge_slot,
                                      A.dir_cap, A.edge_cap, A.err);
         if (!V.run) return;
         dir_slot = V.dir_slot;
+        ncoop = V.ncoop;
         if (threadIdx.x == 0) { s_work = V.work; s_nwork = V.nwork; }
         __syncthreads();
     }
@@ -600,7 +590,7 @@ __global__ void __launch_bounds__(128, 4) sw32ck_kernel(SwArgs A)
     const int nwork = PLAN ? s_nwork : (A.nwork_dev ? *A.nwork_dev : A.nwork);
 #define SW32_WORK (PLAN ? s_work : A.work)
     // one call site of c32_pair, so its body is in the kernel once
-    bool block_phase = A.coop_cells >= 0;
+    bool block_phase = ncoop > 0 || A.coop_cells >= 0;
     for (;;) {
         int w = -1;
         bool coop = false;
@@ -611,7 +601,7 @@ __global__ void __launch_bounds__(128, 4) sw32ck_kernel(SwArgs A)
             __syncthreads();
             if (wb >= nwork) break;
             const int p = SW32_WORK[wb];
-            if ((int64_t)A.D.a_len[p] * A.D.b_len[p] > A.coop_cells) {
+            if (A.coop_cells >= 0 ? (int64_t)A.D.a_len[p] * A.D.b_len[p] > A.coop_cells : wb < ncoop) {
                 w = wb;
                 coop = true;
             } else {
@@ -634,29 +624,35 @@ __global__ void __launch_bounds__(128, 4) sw32ck_kernel(SwArgs A)
 template <int K, int CT>
 static size_t c32_smem(int warps = 4) { return (size_t)warps * c32_warp_smem_bytes(K, CT); }
 
-int sw32ck_max_slots(bool long_pairs, int sm_count)
+template <int K, int CT>
+static int c32_per_sm()
 {
-    if (long_pairs) {
-        // both variants launch with this shared memory: raise both limits
-        blocks_per_sm((const void*)sw32ck_kernel<512, 16, true>, 128, c32_smem<512, 16>());
-        return blocks_per_sm((const void*)sw32ck_kernel<512, 16, false>, 128, c32_smem<512, 16>()) * sm_count * 4;
+    // every variant's shared-memory limit is raised, to its widest block's
+    for (int w = 4; w <= COOP_MAX_WARPS; w *= 2) {
+        blocks_per_sm((const void*)sw32ck_kernel<K, CT, true>, 32 * w, c32_smem<K, CT>(w));
+        blocks_per_sm((const void*)sw32ck_kernel<K, CT, false>, 32 * w, c32_smem<K, CT>(w));
     }
-    blocks_per_sm((const void*)sw32ck_kernel<64, 2, true>, 128, c32_smem<64, 2>());
-    return blocks_per_sm((const void*)sw32ck_kernel<64, 2, false>, 128, c32_smem<64, 2>()) * sm_count * 4;
+    return blocks_per_sm((const void*)sw32ck_kernel<K, CT, false>, 128, c32_smem<K, CT>());
 }
 
-// slots: warp slots of A.dirs, a multiple of 4 (blocks of 4 warps).
-cudaError_t launch_sw32ck(const SwArgs& A, bool long_pairs, int slots, cudaStream_t st)
+int sw32ck_max_slots(bool long_pairs, int sm_count)
+{
+    return (long_pairs ? c32_per_sm<512, 16>() : c32_per_sm<64, 2>()) * sm_count * 4;
+}
+
+// slots: warp slots of A.dirs, a multiple of warps (per block).
+cudaError_t launch_sw32ck(const SwArgs& A, bool long_pairs, int slots, int warps, cudaStream_t st)
 {
     if (A.nwork <= 0 && !A.nwork_dev && !A.plan) return cudaSuccess;
-    if (slots < 4) return cudaErrorInvalidValue;
+    if (slots < warps || slots % warps != 0) return cudaErrorInvalidValue;
+    const int grid = slots / warps, threads = 32 * warps;
     launch_begin(K_SW32_TRACE, st);
     if (A.plan) {
-        if (long_pairs) sw32ck_kernel<512, 16, true><<<slots / 4, 128, c32_smem<512, 16>(), st>>>(A);
-        else sw32ck_kernel<64, 2, true><<<slots / 4, 128, c32_smem<64, 2>(), st>>>(A);
+        if (long_pairs) sw32ck_kernel<512, 16, true><<<grid, threads, c32_smem<512, 16>(warps), st>>>(A);
+        else sw32ck_kernel<64, 2, true><<<grid, threads, c32_smem<64, 2>(warps), st>>>(A);
     } else {
-        if (long_pairs) sw32ck_kernel<512, 16, false><<<slots / 4, 128, c32_smem<512, 16>(), st>>>(A);
-        else sw32ck_kernel<64, 2, false><<<slots / 4, 128, c32_smem<64, 2>(), st>>>(A);
+        if (long_pairs) sw32ck_kernel<512, 16, false><<<grid, threads, c32_smem<512, 16>(warps), st>>>(A);
+        else sw32ck_kernel<64, 2, false><<<grid, threads, c32_smem<64, 2>(warps), st>>>(A);
     }
     launch_end(K_SW32_TRACE, st);
     return cudaGetLastError();

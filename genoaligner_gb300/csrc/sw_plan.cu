@@ -34,6 +34,12 @@ __global__ void sp_classify_kernel(SwPlanArgs P)
     const int lane = threadIdx.x & 31;
     const int n = P.D.n;
     const int stride = gridDim.x * blockDim.x;
+    __shared__ unsigned long long s_cells[SP_LISTS], s_largest[SP_LISTS];
+    __shared__ int s_cols[SP_LISTS];
+    if (threadIdx.x < SP_LISTS) s_cells[threadIdx.x] = s_largest[threadIdx.x] = s_cols[threadIdx.x] = 0;
+    __syncthreads();
+    unsigned long long cells[SP_LISTS] = {0, 0, 0}, largest[SP_LISTS] = {0, 0, 0};
+    int cols[SP_LISTS] = {0, 0, 0};
     for (int p0 = blockIdx.x * blockDim.x + (threadIdx.x & ~31); p0 < n; p0 += stride) {
         const int p = p0 + lane;
         int it = -1;
@@ -58,11 +64,40 @@ __global__ void sp_classify_kernel(SwPlanArgs P)
                                      : ((!P.score_only && sw32ck_long(m, nn, P.long_log2)) ? SP_L32LONG : SP_L32);
                 it = list * SP_NB + (u16 ? sp_key16(m, nn) : sp_key(m, nn));
                 atomicMax(reinterpret_cast<unsigned long long*>(P.res + SP_EDGE), (unsigned long long)(2 * max(m, 0)));
+#pragma unroll
+                for (int l = 0; l < SP_LISTS; ++l)
+                    if (l == list) {
+                        const unsigned long long c = (unsigned long long)max(m, 0) * (unsigned long long)max(nn, 0);
+                        cells[l] += c;
+                        largest[l] = max(largest[l], c);
+                        cols[l] = max(cols[l], nn);
+                    }
             }
             P.item[p] = it;
         }
         const unsigned same = __match_any_sync(FULL, it);
         if (it >= 0 && lane == __ffs(same) - 1) atomicAdd(&P.counts[it], __popc(same));
+    }
+    if (P.coop_limit < 0) return;
+#pragma unroll
+    for (int l = 0; l < SP_LISTS; ++l) {
+        for (int o = 16; o > 0; o >>= 1) {
+            cells[l] += __shfl_xor_sync(FULL, cells[l], o);
+            largest[l] = max(largest[l], __shfl_xor_sync(FULL, largest[l], o));
+        }
+        const int c = __reduce_max_sync(FULL, cols[l]);
+        if (lane == 0 && cells[l]) {
+            atomicAdd(&s_cells[l], cells[l]);
+            atomicMax(&s_largest[l], largest[l]);
+            atomicMax(&s_cols[l], c);
+        }
+    }
+    __syncthreads();
+    if (threadIdx.x < SP_LISTS && s_cells[threadIdx.x]) {
+        unsigned long long* r = reinterpret_cast<unsigned long long*>(P.res + threadIdx.x);
+        atomicAdd(r + SP_CELLS, s_cells[threadIdx.x]);
+        atomicMax(r + SP_LARGEST, s_largest[threadIdx.x]);
+        atomicMax(r + SP_COLS, (unsigned long long)s_cols[threadIdx.x]);
     }
 }
 
@@ -101,6 +136,10 @@ __global__ void sp_scan_kernel(SwPlanArgs P)
             P.res[SP_INTS + l] = ints;
             P.res[SP_BASE + l] = base;
             base += ints;
+            P.res[SP_COOPW + l] = P.coop_block[l] ? P.coop_block[l]
+                                                  : sw_coop_block(P.res[SP_LARGEST + l], (int)P.res[SP_COLS + l],
+                                                                  l == SP_L16 ? P.res[SP_CELLS + l] / 2 : P.res[SP_CELLS + l],
+                                                                  P.sms);
         }
     }
 }
@@ -122,7 +161,10 @@ __global__ void sp_scatter_kernel(SwPlanArgs P)
     }
 }
 
-// Work items in launch order, and each list's largest per-warp memory.
+// Work items in launch order, each list's largest per-warp memory, and its leading
+// whole-block items: those up to the last item above sp_coop_cells.  The 32-bit lists
+// come by cells, the 16-bit list only among its widest pairs, so there only those
+// count, unless the items are so few that each can have a block.
 __global__ void sp_pack_kernel(SwPlanArgs P)
 {
     const int n = P.D.n;
@@ -133,35 +175,49 @@ __global__ void sp_pack_kernel(SwPlanArgs P)
         const int32_t* srt = P.sorted + (int64_t)l * n;
         int32_t* w = P.work + P.res[SP_BASE + l];
         unsigned long long* mx = reinterpret_cast<unsigned long long*>(P.res + SP_DIR + l);
-        unsigned long long local = 0, cmax = 0;
+        unsigned long long local = 0;
+        // (an item of the 16-bit list holds two pairs and costs a warp what one does)
+        const int64_t coop = sp_coop_cells(P.coop_limit, l == SP_L16 ? P.res[SP_CELLS + l] / 2 : P.res[SP_CELLS + l],
+                                           P.coop_warps[l]);
+        const int W = (int)P.res[SP_COOPW + l];
+        unsigned long long ncoop = 0;
         if (l == SP_L16) {
             const long long items = (cnt + 1) / 2;
+            const bool few = W * items <= P.coop_warps[l];
             for (long long q = blockIdx.x * blockDim.x + threadIdx.x; q < items; q += stride) {
                 const int a = srt[2 * q], b = 2 * q + 1 < cnt ? srt[2 * q + 1] : -1;
                 w[2 * q] = a;
                 w[2 * q + 1] = b;
                 const int M = max(P.D.a_len[a], b >= 0 ? P.D.a_len[b] : 0);
                 const int N = max(P.D.b_len[a], b >= 0 ? P.D.b_len[b] : 0);
-                local = max(local, (unsigned long long)(P.score_only ? sw16so_dir_words(M, N)
-                                                                     : sw16ck_dir_words(M, N, P.window)));
-                if (l == SP_L16) cmax = max(cmax, (unsigned long long)M * (unsigned long long)N);
+                int64_t words = P.score_only ? sw16so_dir_words(M, N) : sw16ck_dir_words(M, N, P.window);
+                if ((int64_t)M * N > coop && (few || sw16_by_cells(N))) {
+                    ncoop = q + 1;
+                    words = sw_coop_share(words, W, P.score_only ? SO_ROW_WORDS : 0);
+                }
+                local = max(local, (unsigned long long)words);
             }
         } else {
             for (long long q = blockIdx.x * blockDim.x + threadIdx.x; q < cnt; q += stride) {
                 const int a = srt[q];
                 w[q] = a;
-                if (!P.score_only)
-                    local = max(local, (unsigned long long)sw32ck_dir_words(P.D.a_len[a], P.D.b_len[a], P.long_log2));
+                if (P.score_only) continue;
+                int64_t words = sw32ck_dir_words(P.D.a_len[a], P.D.b_len[a], P.long_log2);
+                if ((int64_t)P.D.a_len[a] * P.D.b_len[a] > coop) {
+                    ncoop = q + 1;
+                    words = sw_coop_share(words, W);
+                }
+                local = max(local, (unsigned long long)words);
             }
         }
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) {
             local = max(local, __shfl_xor_sync(FULL, local, o));
-            cmax = max(cmax, __shfl_xor_sync(FULL, cmax, o));
+            ncoop = max(ncoop, __shfl_xor_sync(FULL, ncoop, o));
         }
+        if ((threadIdx.x & 31) == 0 && ncoop)
+            atomicMax(reinterpret_cast<unsigned long long*>(P.res + SP_NCOOP + l), ncoop);
         if ((threadIdx.x & 31) == 0 && local) atomicMax(mx, local);
-        if ((threadIdx.x & 31) == 0 && cmax)
-            atomicMax(reinterpret_cast<unsigned long long*>(P.res + SP_MAXC16), cmax);
     }
 }
 

@@ -83,6 +83,9 @@ __host__ __device__ inline int64_t sw16ck_dir_words(int M, int N, int window)
            (int64_t)CK_K * window * CK_TW;
 }
 
+// A 16-bit pair of n columns is listed by its cells, before those that are not.
+__host__ __device__ inline bool sw16_by_cells(int n) { return ck_ncol(n > 1 ? n : 1) >= 24 * 64; }
+
 // Bucket (0..4095, smallest first) of a 16-bit pair of m rows and n columns
 // in a list of the two-pairs-per-warp kernels: consecutive entries share a
 // warp and run with the larger of their row counts and forward column
@@ -95,7 +98,7 @@ __host__ __device__ inline int64_t sw16ck_dir_words(int M, int N, int window)
 __host__ __device__ inline int sw16_shape_key(int m, int n)
 {
     const int ncls = ck_ncol(n > 1 ? n : 1) / 64;
-    if (ncls >= 24) {
+    if (sw16_by_cells(n)) {
         const float lc = log2f((float)(m > 1 ? m : 1) * (float)(n > 1 ? n : 1));
         const int e = (int)(32.0f * (lc - 20.0f));
         return 1023 - (e < 0 ? 0 : (e > 1023 ? 1023 : e));
@@ -114,12 +117,60 @@ __host__ __device__ inline int64_t sw16so_dir_words(int M, int N)
     return SO_ROW_WORDS + (2 * (int64_t)(ck_ncol(N) / CK_TW) * M + 3) / 4 * 4 + 4;
 }
 
+// Items of a traceback list above this many cells run on a whole block: above
+// limit (the sw_coop_log2 setting, < 0: none), and above twice the list's cells per
+// resident warp.  An item past that share would keep its one warp busy when the
+// others have run out of work: 152 pairs of 8,000 x 8,000 take 28.8 ms on a warp
+// each and 8.2 ms on a block each, and batches with more items than warps stay
+// below the share.  Items under SW_COOP_MIN cells have too few bands to divide.
+constexpr int64_t SW_COOP_MIN = (int64_t)1 << 16;
+__host__ __device__ inline int64_t sp_coop_cells(int64_t limit, int64_t cells, int64_t warps)
+{
+    if (limit < 0 || warps <= 0) return INT64_MAX;
+    const int64_t share = 2 * cells / warps;
+    const int64_t t = share < SW_COOP_MIN ? SW_COOP_MIN : share;
+    return t < limit ? t : limit;
+}
+// Warps of a whole-block launch's blocks, 4, 8 or 16: enough that the largest item,
+// which gets W of a multiprocessor's 16 resident warps, ends no later than the
+// multiprocessors' common work, and no more than a quarter of the 64-column bands it
+// can be cut into.  152, 304 and 608 pairs of 8,000 x 8,000: 11.4, 13.1, 21.2 ms with
+// 4 warps, 8.9, 12.2, 24.6 with 8, 8.2, 16.2, 32.2 with 16; 1,024 pairs of 2 to 30 kb
+// (one pair holds 1/150 of the cells): 280, 217, 153 ms; 600 pairs of 200 to 1,000 x
+// 1,100 score-only: 0.61, 0.71, 1.54 ms.
+constexpr int COOP_MAX_WARPS = 16;
+__host__ __device__ inline int sw_coop_block(int64_t largest, int cols, int64_t cells, int sms)
+{
+    int W = 4;
+    while (W < COOP_MAX_WARPS && W * 512 <= cols && W * cells < 16 * largest * sms) W *= 2;
+    return W;
+}
+// Per-warp share of an item's memory when a block of W warps serves it (the
+// score-only kernel keeps SO_ROW_WORDS for each warp).
+__host__ __device__ inline int64_t sw_coop_share(int64_t words, int W, int64_t own = 0)
+{
+    return own + (words - own + 4 * W - 1) / (4 * W) * 4;
+}
+// Columns per lane of a whole-block item's full bands: those of 16, 8 and down to
+// `least` with the shortest schedule, of start(last band) + chunks chunks (fwd16_coop)
+// of CB + 4 units each.
+__host__ __device__ inline int coop_cb(int N, int W, int nck, int least)
+{
+    int best = 16;
+    int64_t t = INT64_MAX;
+    for (int cb = 16; cb >= least; cb >>= 1) {
+        const int last = (N - 1) / (32 * cb);
+        const int64_t g = (int64_t)(last / W) * (nck > 2 * W ? nck : 2 * W) + 2 * (last % W) + nck;
+        if (g * (cb + 4) < t) { t = g * (cb + 4); best = cb; }
+    }
+    return best;
+}
+
 // ---- 32-bit one-pair-per-warp checkpointed kernel (sw32ck.cu) ---------------
 constexpr int C32_C = 16;                // forward columns per lane, full bands
 constexpr int C32_BW = 32 * C32_C;
 constexpr int C32_LONG_LOG2 = 24;       // default: the long-pair shape above 2^24 cells
 constexpr int C32_COOP_LOG2 = 27;       // default: work items above 2^27 cells run on a whole block
-constexpr int C32_MAX_WARPS = 4;        // sw32ck: warps per block
 
 __host__ __device__ inline int c32_rows(int m, int K) { return m > 1 ? (m - 1) / K : 0; }
 __host__ __device__ inline int c32_last_cb(int rest) { return rest > 8 * 32 ? 16 : (rest > 4 * 32 ? 8 : 4); }

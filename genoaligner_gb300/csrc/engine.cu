@@ -712,16 +712,20 @@ static cudaError_t enqueue_wfa(const WfaScratch& S, PairDesc D, int smax, bool t
     WfaBlockArgs B;
     B.A = A;
     B.next = S.ctr + 3;
-    cudaError_t e = cudaMemsetAsync(S.ctr, 0, 64 * sizeof(int32_t), st);
-    if (e == cudaSuccess) e = launch_pack(D, S.seq_bytes, S.packed, S.pure, st);
+    const int NB = route_buckets();
+    Fills F;
+    F.add(S.ctr, 64, 0);
+    F.add(err, 1, 0);
+    if (route != 0) F.add(S.counts, 2 * NB + 4, 0);
+    cudaError_t e = launch_pack(D, S.seq_bytes, S.packed, route != 0 ? S.pure : nullptr, st, F);
     if (e != cudaSuccess) return e;
     if (route == 0) {
+        A.masks = packed_masks(S.packed, S.seq_bytes);
+        A.pure = S.pure;
         e = launch_wfa(A, S.slots, st);
         if (e == cudaSuccess && S.blocks > 0) e = launch_wfa_block(B, S.blocks, trace ? K_WFA_TRACE : K_WFA_SCORE, st);
         return e;
     }
-    const int NB = route_buckets();
-    if ((e = cudaMemsetAsync(S.counts, 0, sizeof(int32_t) * (2 * NB + 4), st)) != cudaSuccess) return e;
     if ((e = launch_route_model(D, smax, lane_smax, route == 1, S.item, S.lb, S.y, S.counts, score, len, st)) !=
         cudaSuccess)
         return e;
@@ -795,7 +799,8 @@ static cudaError_t run_wfa_graph(Ctx* c, const WfaScratch& S, const PairDesc& D,
                                        (uint64_t)trace | (uint64_t)lane_smax << 8 | (uint64_t)route << 16 |
                                            (uint64_t)S.group << 24,
                                        (uint64_t)(uintptr_t)score, (uint64_t)(uintptr_t)cig,
-                                       (uint64_t)(uintptr_t)D.a_off, (uint64_t)(uintptr_t)S.packed};
+                                       (uint64_t)(uintptr_t)D.a_off, (uint64_t)(uintptr_t)S.packed,
+                                       (uint64_t)(uintptr_t)err};
     return replay_graph(c->gexec, c->gkey, key, c->glaunches, st, [&]() {
         return enqueue_wfa(S, D, smax, trace, route, lane_smax, score, len, cig, err, st);
     });
@@ -1029,8 +1034,7 @@ int32_t wfa_batch(const ga_align_request* reqs, int32_t n, int32_t max_smax, int
         D.seq = dseq; D.packed = nullptr; D.pure = nullptr;
         D.a_off = da; D.a_len = dal; D.b_off = db; D.b_len = dbl; D.out_off = dout; D.n = nk;
         bool ok = !fail_here(2) &&
-                  cudaMemcpyAsync(c->dev, c->host, in_bytes, cudaMemcpyHostToDevice, c->stream) == cudaSuccess &&
-                  cudaMemsetAsync(der, 0, sizeof(int32_t), c->stream) == cudaSuccess;
+                  cudaMemcpyAsync(c->dev, c->host, in_bytes, cudaMemcpyHostToDevice, c->stream) == cudaSuccess;
         if (ok && span) {
             ok = (span_a == 0 || cudaMemcpyAsync(dspan_a, (const void*)spa.first, (size_t)span_a,
                                                  cudaMemcpyHostToDevice, c->stream) == cudaSuccess) &&
@@ -1050,8 +1054,7 @@ int32_t wfa_batch(const ga_align_request* reqs, int32_t n, int32_t max_smax, int
             le = run_wfa_graph(c, S, D, smax, trace, route, lane_smax, dsc, dln, dcg, der, c->stream);
         else le = enqueue_wfa(S, D, smax, trace, route, lane_smax, dsc, dln, dcg, der, c->stream);
         if (learned) note_route(c, S, nk);
-        if (le == cudaSuccess && trace) le = launch_wfa_validate(D, dsc, dln, dcg, dvf, c->stream);
-        if (le == cudaSuccess && trace) le = launch_cigar_pack(D, dln, dcg, dpo, dpk, c->stream);
+        if (le == cudaSuccess && trace) le = launch_wfa_validate(D, dsc, dln, dcg, dvf, c->stream, dpo, dpk);
         if (le != cudaSuccess) {
             cudaGetLastError();
             *rerr = E_LAUNCH;
@@ -1327,6 +1330,7 @@ struct SwSlots {
 static SwSlots size_sw(const SwPlan& P, bool trace, const ga_tune& T, int sm_count, int64_t budget)
 {
     SwSlots S;
+    sw_plan_prepare();
     for (int l = 0; l < SP_LISTS; ++l) {
         if (P.ints[l] <= 0) continue;
         // warp slots come in blocks of w; a whole-block item has a block to itself
@@ -1577,14 +1581,17 @@ static int32_t sw_batch_range(const ga_sw_request* reqs, int32_t n, int64_t base
     auto enqueue = [&]() -> cudaError_t {
         cudaStream_t st = c->stream;
         // sentinel: too-large pairs keep score -1 (never written by a kernel)
-        cudaError_t e = cudaMemsetAsync(dsc, 0xff, sizeof(int32_t) * (size_t)n, st);
-        if (e == cudaSuccess) e = cudaMemsetAsync(dpos, 0xff, sizeof(int32_t) * 4 * (size_t)n, st);
-        if (e == cudaSuccess) e = cudaMemsetAsync(dln, 0, sizeof(int32_t) * (size_t)n, st);
-        if (e == cudaSuccess) e = cudaMemsetAsync(der, 0, sizeof(int32_t), st);
-        if (e == cudaSuccess) e = cudaMemsetAsync(dctr, 0, sizeof(int32_t) * 8, st);
+        Fills F;
+        F.add(dsc, n, -1);
+        F.add(dpos, 4 * (int64_t)n, -1);
+        F.add(dln, n, 0);
+        F.add(der, 1, 0);
+        F.add(dctr, 8, 0);
+        sw_plan_fills(F, n, dscr, dres);
+        cudaError_t e = cudaSuccess;
         if (e == cudaSuccess && span) e = launch_gather_sides(D, dseq, dspan_a, dspan_b, dsa, dsb, st);
         if (e == cudaSuccess && span) e = cudaMemsetAsync(dseq + arena - 64, 0, 64, st);
-        if (e == cudaSuccess) e = launch_pack(D, arena, nullptr, dpure, st);
+        if (e == cudaSuccess) e = launch_pack(D, arena, nullptr, dpure, st, F);
         if (e == cudaSuccess && route) e = launch_sw_route(D, s0.match, s0.gap_open, dfeat, dy, dtry, st);
         if (e == cudaSuccess)
             e = enqueue_plan_sw(D, s0, trace, trace ? cell_limit : -1, -1, dsc, dwork, dscr, dres, T, st, dtry,
@@ -1593,8 +1600,7 @@ static int32_t sw_batch_range(const ga_sw_request* reqs, int32_t n, int64_t base
             e = launch_plan(P, S, D, s0, trace, T, dwork, dsc, dpos, dln, dcg, ddirs, dedge, dctr, der, st, dscr, dres);
         if (e == cudaSuccess && trace)
             e = launch_sw_validate(D, ga_sw_scoring_t{s0.match, s0.mismatch, s0.gap_open, s0.gap_extend}, dsc, dpos,
-                                   dln, dcg, dvf, st);
-        if (e == cudaSuccess && trace) e = launch_cigar_pack(D, dln, dcg, dpo, dpk, st);
+                                   dln, dcg, dvf, st, dpo, dpk);
         return e;
     };
     cudaError_t le = cudaErrorLaunchFailure;
@@ -2034,8 +2040,8 @@ int32_t ga_wfa_device_ex(const ga_device_batch* b, int32_t smax, int32_t trace, 
     D.a_off = b->a_off; D.a_len = b->a_len; D.b_off = b->b_off; D.b_len = b->b_len;
     D.out_off = b->out_off; D.n = b->n;
     int32_t rc = GA_OK;
-    cudaError_t le = cudaMemsetAsync(derr, 0, sizeof(int32_t), st);
-    if (le == cudaSuccess) {
+    cudaError_t le;
+    {
         const int lane_smax = tuned.wfa_lane_smax;
         if (learned && !profiling_on())
             le = run_wfa_graph(c, S, D, smax, trace != 0, route, lane_smax, out_score, out_len, out_cigar, derr, st);
@@ -2192,14 +2198,22 @@ int32_t ga_sw_device_ex(const ga_device_batch* b, ga_sw_scoring sc, int32_t trac
         }
     }
 
-    cudaMemsetAsync(out_score, 0xff, sizeof(int32_t) * n, st);
-    cudaMemsetAsync(out_pos, 0xff, sizeof(int32_t) * 4 * (size_t)n, st);
-    if (out_len) cudaMemsetAsync(out_len, 0, sizeof(int32_t) * n, st);
     SwPlan P;
+    // the purity pass, with the outputs' defaults and the planner's zeros
+    auto purity = [&](int32_t* counters) {
+        Fills F;
+        F.add(out_score, n, -1);
+        F.add(out_pos, 4 * (int64_t)n, -1);
+        if (out_len) F.add(out_len, n, 0);
+        if (counters) F.add(counters, 64, 0);
+        sw_plan_fills(F, n, dscr, dres);
+        return launch_pack(D, b->seq_bytes, nullptr, dpure, st, F);
+    };
+    sw_plan_prepare();
     auto plan = [&]() {
         plan_layout(c->dev, &dpure, &dscr, &dwork, &dres);
         D.pure = dpure;
-        if (launch_pack(D, b->seq_bytes, nullptr, dpure, st) != cudaSuccess) return false;
+        if (purity(nullptr) != cudaSuccess) return false;
         if (route && launch_sw_route(D, sc.match, sc.gap_open, dfeat, dy, dtry, st) != cudaSuccess) return false;
         return device_plan_sw(D, sc, trace != 0, cell_limit, -2, out_score, dwork, dscr, dres, hres, T, st, P, dtry) ==
                cudaSuccess;
@@ -2230,11 +2244,7 @@ int32_t ga_sw_device_ex(const ga_device_batch* b, ga_sw_scoring sc, int32_t trac
         // the launches of this shape in plan mode, captured with the memsets,
         // the purity pass and the planner, then replayed (this call included)
         auto enqueue = [&]() -> cudaError_t {
-            cudaError_t x = cudaMemsetAsync(out_score, 0xff, sizeof(int32_t) * n, st);
-            if (x == cudaSuccess) x = cudaMemsetAsync(out_pos, 0xff, sizeof(int32_t) * 4 * (size_t)n, st);
-            if (x == cudaSuccess) x = cudaMemsetAsync(out_len, 0, sizeof(int32_t) * n, st);
-            if (x == cudaSuccess) x = cudaMemsetAsync(dctr, 0, 64 * sizeof(int32_t), st);
-            if (x == cudaSuccess) x = launch_pack(D, b->seq_bytes, nullptr, dpure, st);
+            cudaError_t x = purity(dctr);
             if (x == cudaSuccess && route) x = launch_sw_route(D, sc.match, sc.gap_open, dfeat, dy, dtry, st);
             if (x == cudaSuccess)
                 x = enqueue_plan_sw(D, sc, true, cell_limit, -2, out_score, dwork, dscr, dres, T, st, dtry,

@@ -24,6 +24,8 @@ struct WfaArgs {
     int32_t cap;
     int32_t* blk = nullptr;
     int32_t* blk_count = nullptr;
+    const uint32_t* masks = nullptr;      // wfa_kernel: the arena's chunk masks (packed_masks); it sets pure of pairs in blk
+    uint8_t* pure = nullptr;
 };
 
 struct SwArgs {
@@ -109,9 +111,29 @@ struct WfaBlockArgs {
 };
 int wfa_block_slots(int smax, bool trace, int sm_count);
 cudaError_t launch_wfa_block(const WfaBlockArgs& B, int blocks, int kernel_id, cudaStream_t st);
+// Words that a batch's first kernel sets for the later ones: counters, records and
+// output defaults, for which a memset each would be a launch each.
+struct Fills {
+    int32_t* p[8];
+    int64_t n[8];
+    int32_t v[8];
+    int32_t count = 0;
+    void add(void* ptr, int64_t words, int32_t value)
+    {
+        p[count] = static_cast<int32_t*>(ptr);
+        n[count] = words;
+        v[count++] = value;
+    }
+};
 // Packs seq into the 2-bit arena `packed` (packed_arena_words(seq_bytes)
-// words; null: purity flags only) and sets pure[2n].
-cudaError_t launch_pack(const PairDesc& D, int64_t seq_bytes, uint64_t* packed, uint8_t* pure, cudaStream_t st);
+// words; null: purity flags only) and sets pure[2n] (null: the masks of the arena's
+// chunks, packed_masks, are left to the reader), and does the fills.
+cudaError_t launch_pack(const PairDesc& D, int64_t seq_bytes, uint64_t* packed, uint8_t* pure, cudaStream_t st,
+                        const Fills& fills = Fills());
+inline uint32_t* packed_masks(uint64_t* packed, int64_t seq_bytes)
+{
+    return reinterpret_cast<uint32_t*>(packed + seq_bytes / 32 + 2);
+}
 int64_t packed_arena_words(int64_t seq_bytes);
 cudaError_t launch_pack_arena(const uint8_t* seq, int64_t seq_bytes, uint64_t* packed, uint32_t* bad, cudaStream_t st);
 // Sequences copied to the device as the caller laid them out -- one span per
@@ -120,12 +142,21 @@ cudaError_t launch_pack_arena(const uint8_t* seq, int64_t seq_bytes, uint64_t* p
 // src_a[p] >= 0, side b likewise; seq is D.seq, writable (wfa.cu).
 cudaError_t launch_gather_sides(const PairDesc& D, uint8_t* seq, const uint8_t* span_a, const uint8_t* span_b,
                                 const int64_t* src_a, const int64_t* src_b, cudaStream_t st);
-// Each pair's CIGAR (end of its slot) packed 2 bits per op at pk + pk_off[p] (wfa.cu).
-cudaError_t launch_cigar_pack(const PairDesc& D, const int32_t* len, const char* cig, const int64_t* pk_off,
-                              uint8_t* pk, cudaStream_t st);
-// WFA result checks on the device (wfa.cu): flags[p] = rescore_ok | wellformed_ok << 1.
+// WFA result checks on the device (wfa.cu): flags[p] = rescore_ok | wellformed_ok << 1;
+// with pk, each pair's CIGAR also packed 2 bits per op at pk + pk_off[p] (pack_ops).
 cudaError_t launch_wfa_validate(const PairDesc& D, const int32_t* score, const int32_t* len, const char* cig,
-                                uint8_t* flags, cudaStream_t st);
+                                uint8_t* flags, cudaStream_t st, const int64_t* pk_off = nullptr, uint8_t* pk = nullptr);
+#ifdef __CUDACC__
+// Ops q0 + lane of a CIGAR of L ops packed for the copy back, 2 bits per op in op
+// order (M 0, X 1, I 2, D 3; op t at bits 2 (t % 4) of byte t / 4).
+__device__ __forceinline__ void pack_ops(uint8_t* dst, char op, int q, int L, int lane)
+{
+    uint32_t v = q < L ? (uint32_t)(op == 'M' ? 0 : (op == 'X' ? 1 : (op == 'I' ? 2 : 3))) << (2 * (lane & 3)) : 0u;
+    v |= __shfl_xor_sync(0xffffffffu, v, 1);
+    v |= __shfl_xor_sync(0xffffffffu, v, 2);
+    if ((lane & 3) == 0 && q < L) dst[q >> 2] = (uint8_t)v;
+}
+#endif
 // 3-mer sketch features [n][66]; sw: the scaling of the SW variant model.
 cudaError_t launch_sketch(const PairDesc& D, float* feat, int32_t* lb, cudaStream_t st, bool sw = false);
 cudaError_t launch_mlp_forward(const float* feat, int n, float* y, cudaStream_t st);
@@ -242,13 +273,18 @@ struct SwPlanArgs {
     long long* res;              // the record above
     int32_t *item, *counts, *starts, *sorted;   // scratch, set by launch_sw_plan
 };
+// Raises the planner's shared-memory limit (once, outside any capture).
+void sw_plan_prepare();
+// What launch_sw_plan finds zeroed for n pairs.
+void sw_plan_fills(Fills& F, int n, int32_t* scratch, long long* res);
 int64_t sw_plan_scratch_ints(int n);
 cudaError_t launch_sw_plan(SwPlanArgs P, int32_t* scratch, cudaStream_t st);
 // Result checks of every pair with a CIGAR (sw_plan.cu): flags[p] =
-// rescore_ok | wellformed_ok << 1.
+// rescore_ok | wellformed_ok << 1; with pk, the CIGARs packed too (pack_ops).
 struct ga_sw_scoring_t { int32_t match, mismatch, gap_open, gap_extend; };
 cudaError_t launch_sw_validate(const PairDesc& D, const ga_sw_scoring_t& sc, const int32_t* score, const int32_t* pos,
-                               const int32_t* len, const char* cig, uint8_t* flags, cudaStream_t st);
+                               const int32_t* len, const char* cig, uint8_t* flags, cudaStream_t st,
+                               const int64_t* pk_off = nullptr, uint8_t* pk = nullptr);
 
 // sw32ck has a short-pair shape and a long-pair shape (sw32ck_long); sizes
 // in sw_sizes.cuh.

@@ -30,9 +30,18 @@ namespace ga {
 // 64-bit word (A=0 C=1 G=2 T=3 under ((c>>1)^(c>>2))&3, little-endian).
 // Sequences start on 32-byte boundaries, so word index = byte offset / 32 and
 // no per-sequence bookkeeping is needed.
-__global__ void __launch_bounds__(256) pack_chunks_kernel(const uint8_t* __restrict__ seq, int64_t nchunks,
-                                                          uint64_t* __restrict__ packed, uint32_t* __restrict__ bad)
+__device__ __forceinline__ void fill_words(const Fills& F)
 {
+    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, stride = (int64_t)gridDim.x * blockDim.x;
+    for (int k = 0; k < F.count; ++k)
+        for (int64_t i = t; i < F.n[k]; i += stride) F.p[k][i] = F.v[k];
+}
+
+__global__ void __launch_bounds__(256) pack_chunks_kernel(const uint8_t* __restrict__ seq, int64_t nchunks,
+                                                          uint64_t* __restrict__ packed, uint32_t* __restrict__ bad,
+                                                          const Fills F)
+{
+    fill_words(F);
     for (int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; c < nchunks; c += (int64_t)gridDim.x * blockDim.x) {
         const uint4* src = reinterpret_cast<const uint4*>(seq + 32 * c);
         const uint4 x0 = __ldg(src), x1 = __ldg(src + 1);
@@ -82,8 +91,9 @@ __global__ void __launch_bounds__(256) purity_mask_kernel(PairDesc D, const uint
 // thread took length / 16 (600 pairs up to 1 kb: 31 -> 7.5 us; 200,000 uneven
 // pairs, 260 MB: 226 -> 154 us, bound by the latency of the few loads a warp has
 // in flight).
-__global__ void __launch_bounds__(256) purity_kernel(PairDesc D, uint8_t* __restrict__ pure)
+__global__ void __launch_bounds__(256) purity_kernel(PairDesc D, uint8_t* __restrict__ pure, const Fills F)
 {
+    fill_words(F);
     const int lane = threadIdx.x & 31;
     const int nw = (gridDim.x * blockDim.x) >> 5;
     for (int q = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; q < 2 * D.n; q += nw) {
@@ -116,6 +126,15 @@ __global__ void __launch_bounds__(256) purity_kernel(PairDesc D, uint8_t* __rest
 }
 
 // ------------------------------------------------------------------- WFA --
+// Whether a sequence of len bytes whose first chunk's mask is bad[0] is all A, C, G, T.
+__device__ __forceinline__ bool side_pure(const uint32_t* __restrict__ bad, int len, int lane)
+{
+    uint32_t acc = 0;
+    for (int w = lane; 32 * w < len; w += 32)
+        acc |= __ldg(bad + w) & (len - 32 * w >= 32 ? 0xffffffffu : (1u << (len - 32 * w)) - 1u);
+    return !__any_sync(FULL, acc != 0);
+}
+
 template <bool TRACE, int BITS>
 __device__ void wfa_pair(const WfaArgs& A, int p, const uint64_t* __restrict__ P, const uint64_t* __restrict__ T, int m,
                          int n, int32_t* wf0, int32_t* wf1, int32_t* stk, int lane)
@@ -170,7 +189,11 @@ __global__ void __launch_bounds__(128) wfa_kernel(WfaArgs A)
             }
             continue;
         }
-        const bool pure = A.D.pure[p] && A.D.pure[A.D.n + p];
+        // both sides pure ACGT: read from the chunk masks by the warp, where a kernel
+        // for the flags would be one more launch (48 reads: 60 -> 49 us a call, with the
+        // fills and the CIGAR packing in their neighbours' kernels)
+        const bool pure = side_pure(A.masks + (A.D.a_off[p] >> 5), m, lane) & side_pure(A.masks + (A.D.b_off[p] >> 5), n, lane);
+        if (A.blk && lane == 0) A.pure[p] = A.pure[A.D.n + p] = pure;
         if (pure) {
             const uint64_t* P = A.D.packed + (A.D.a_off[p] >> 5);
             const uint64_t* T = A.D.packed + (A.D.b_off[p] >> 5);
@@ -185,7 +208,8 @@ __global__ void __launch_bounds__(128) wfa_kernel(WfaArgs A)
 }
 
 // --------------------------------------------------------------- launchers --
-cudaError_t launch_pack(const PairDesc& D, int64_t seq_bytes, uint64_t* packed, uint8_t* pure, cudaStream_t st)
+cudaError_t launch_pack(const PairDesc& D, int64_t seq_bytes, uint64_t* packed, uint8_t* pure, cudaStream_t st,
+                        const Fills& fills)
 {
     if (D.n <= 0) return cudaSuccess;
     int blocks = (2 * D.n + 255) / 256;
@@ -194,12 +218,13 @@ cudaError_t launch_pack(const PairDesc& D, int64_t seq_bytes, uint64_t* packed, 
         // every sequence ends >= 64 bytes before the arena's end, so the whole
         // chunks cover them all and no read passes seq_bytes
         const int64_t nchunks = seq_bytes / 32;
-        uint32_t* bad = reinterpret_cast<uint32_t*>(packed + nchunks + 2);
+        uint32_t* bad = packed_masks(packed, seq_bytes);
         int64_t cblocks = (nchunks + 255) / 256;
         cblocks = std::min<int64_t>(cblocks, device_sms() * 32);
         launch_begin(K_PACK, st);
-        pack_chunks_kernel<<<(int)cblocks, 256, 0, st>>>(D.seq, nchunks, packed, bad);
+        pack_chunks_kernel<<<(int)std::max<int64_t>(cblocks, 1), 256, 0, st>>>(D.seq, nchunks, packed, bad, fills);
         launch_end(K_PACK, st);
+        if (!pure) return cudaGetLastError();
         launch_begin(K_PACK, st);
         purity_mask_kernel<<<blocks, 256, 0, st>>>(D, bad, pure);
         launch_end(K_PACK, st);
@@ -207,7 +232,7 @@ cudaError_t launch_pack(const PairDesc& D, int64_t seq_bytes, uint64_t* packed, 
     }
     launch_begin(K_PACK, st);
     blocks = (int)std::min<int64_t>(((int64_t)2 * D.n + 7) / 8, (int64_t)device_sms() * 32);      // a warp per sequence
-    purity_kernel<<<blocks, 256, 0, st>>>(D, pure);
+    purity_kernel<<<blocks, 256, 0, st>>>(D, pure, fills);
     launch_end(K_PACK, st);
     return cudaGetLastError();
 }
@@ -221,7 +246,7 @@ cudaError_t launch_pack_arena(const uint8_t* seq, int64_t seq_bytes, uint64_t* p
     int64_t cblocks = (nchunks + 255) / 256;
     cblocks = std::min<int64_t>(cblocks, device_sms() * 32);
     launch_begin(K_PACK, st);
-    pack_chunks_kernel<<<(int)cblocks, 256, 0, st>>>(seq, nchunks, packed, bad);
+    pack_chunks_kernel<<<(int)cblocks, 256, 0, st>>>(seq, nchunks, packed, bad, Fills());
     launch_end(K_PACK, st);
     return cudaGetLastError();
 }
@@ -236,25 +261,32 @@ cudaError_t launch_pack_arena(const uint8_t* seq, int64_t seq_bytes, uint64_t* p
 // flags[p] = rescore_ok | wellformed_ok << 1 for pairs with a CIGAR, 0 for
 // the others.
 __global__ void wfa_validate_kernel(PairDesc D, const int32_t* __restrict__ score, const int32_t* __restrict__ len,
-                                    const char* __restrict__ cig, uint8_t* __restrict__ flags)
+                                    const char* __restrict__ cig, uint8_t* __restrict__ flags,
+                                    const int64_t* __restrict__ pk_off, uint8_t* __restrict__ pk)
 {
     const int lane = threadIdx.x & 31;
     const int nw = (gridDim.x * blockDim.x) >> 5;
     for (int p = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; p < D.n; p += nw) {
         const int s = score[p], L = len[p];
-        if (s < 0 || L <= 0) {
+        if (L <= 0) {
             if (lane == 0) flags[p] = 0;
             continue;
         }
+        uint8_t* dst = pk ? pk + pk_off[p] : nullptr;
         const int m = D.a_len[p], n = D.b_len[p];
         const uint8_t* P = D.seq + D.a_off[p];
         const uint8_t* T = D.seq + D.b_off[p];
         const char* cg = cig + D.out_off[p] + (m + n) - L;
-        int pi0 = 0, ti0 = 0, cost = 0;
-        bool bad = false;
+        int pi0 = 0, ti0 = 0, cost = 0;                            // cost: this lane's ops
+        // the ops are loaded a step ahead and the bytes of an M or X compared a step
+        // behind, so a lone warp waits for neither
+        bool bad = false, chk = false, chk_m = false;
+        uint8_t cp = 0, ct = 0;
+        char next = lane < L ? cg[lane] : 'I';
         for (int q0 = 0; q0 < L; q0 += 32) {
             const int q = q0 + lane;
-            const char op = q < L ? cg[q] : 'I';
+            const char op = next;
+            next = q + 32 < L ? cg[q + 32] : 'I';
             const bool mx = op == 'M' || op == 'X';
             const int dp = (mx || op == 'D') && q < L, dt = (mx || op == 'I') && q < L;
             int v = dp << 16 | dt;                                 // inclusive prefix of both steps
@@ -264,47 +296,28 @@ __global__ void wfa_validate_kernel(PairDesc D, const int32_t* __restrict__ scor
                 if (lane >= o) v += y;
             }
             const int pi = pi0 + (v >> 16) - dp, ti = ti0 + (v & 0xffff) - dt;
-            bool b = false;
+            bad |= chk && (cp == ct) != chk_m;
+            chk = false;
             if (q < L) {
-                if (mx) b = pi >= m || ti >= n || ((P[pi] == T[ti]) != (op == 'M'));
-                else b = op != 'I' && op != 'D';
+                if (mx) {
+                    chk = pi < m && ti < n;
+                    bad |= !chk;
+                    chk_m = op == 'M';
+                    if (chk) { cp = P[pi]; ct = T[ti]; }
+                } else {
+                    bad |= op != 'I' && op != 'D';
+                }
+                cost += op == 'X' || op == 'I' || op == 'D';
             }
-            bad |= __any_sync(FULL, b);
-            cost += __popc(__ballot_sync(FULL, q < L && (op == 'X' || op == 'I' || op == 'D')));
+            if (pk) pack_ops(dst, op, q, L, lane);
             const int tot = __shfl_sync(FULL, v, 31);
             pi0 += tot >> 16;
             ti0 += tot & 0xffff;
         }
-        if (lane == 0) flags[p] = (uint8_t)((cost == s ? 1 : 0) | (!bad && pi0 == m && ti0 == n ? 2 : 0));
-    }
-}
-
-// Every pair's CIGAR (the last len[p] bytes of its slot of a_len + b_len) packed
-// for the copy back, 2 bits per op in op order (M 0, X 1, I 2, D 3; op t at
-// bits 2 (t % 4) of byte t / 4), at byte pk_off[p] of pk.  One warp per pair,
-// a lane per output byte: the slot is read and the packed bytes written
-// contiguously.
-__global__ void cigar_pack_kernel(PairDesc D, const int32_t* __restrict__ len, const char* __restrict__ cig,
-                                  const int64_t* __restrict__ pk_off, uint8_t* __restrict__ pk)
-{
-    const int lane = threadIdx.x & 31;
-    const int nw = (gridDim.x * blockDim.x) >> 5;
-    for (int p = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; p < D.n; p += nw) {
-        const int L = len[p];
-        if (L <= 0) continue;
-        const char* src = cig + D.out_off[p] + ((int64_t)D.a_len[p] + D.b_len[p]) - L;
-        uint8_t* dst = pk + pk_off[p];
-        for (int b = lane; 4 * b < L; b += 32) {
-            uint32_t v = 0;
-#pragma unroll
-            for (int t = 0; t < 4; ++t) {
-                if (4 * b + t < L) {
-                    const char c = src[4 * b + t];
-                    v |= (uint32_t)(c == 'M' ? 0 : (c == 'X' ? 1 : (c == 'I' ? 2 : 3))) << (2 * t);
-                }
-            }
-            dst[b] = (uint8_t)v;
-        }
+        bad |= chk && (cp == ct) != chk_m;
+        bad = __any_sync(FULL, bad);
+        cost = __reduce_add_sync(FULL, cost);
+        if (lane == 0) flags[p] = s < 0 ? 0 : (uint8_t)((cost == s ? 1 : 0) | (!bad && pi0 == m && ti0 == n ? 2 : 0));
     }
 }
 
@@ -340,25 +353,13 @@ cudaError_t launch_gather_sides(const PairDesc& D, uint8_t* seq, const uint8_t* 
     return cudaGetLastError();
 }
 
-cudaError_t launch_cigar_pack(const PairDesc& D, const int32_t* len, const char* cig, const int64_t* pk_off,
-                              uint8_t* pk, cudaStream_t st)
-{
-    if (D.n <= 0) return cudaSuccess;
-    int blocks = (D.n + 7) / 8;
-    blocks = std::min(blocks, device_sms() * 16);
-    launch_begin(K_VALIDATE, st);
-    cigar_pack_kernel<<<blocks, 256, 0, st>>>(D, len, cig, pk_off, pk);
-    launch_end(K_VALIDATE, st);
-    return cudaGetLastError();
-}
-
 cudaError_t launch_wfa_validate(const PairDesc& D, const int32_t* score, const int32_t* len, const char* cig,
-                                uint8_t* flags, cudaStream_t st)
+                                uint8_t* flags, cudaStream_t st, const int64_t* pk_off, uint8_t* pk)
 {
     if (D.n <= 0) return cudaSuccess;
     const int blocks = (int)std::min<int64_t>(((int64_t)D.n + 3) / 4, (int64_t)device_sms() * 16);   // a warp per pair
     launch_begin(K_VALIDATE, st);
-    wfa_validate_kernel<<<blocks, 128, 0, st>>>(D, score, len, cig, flags);
+    wfa_validate_kernel<<<blocks, 128, 0, st>>>(D, score, len, cig, flags, pk_off, pk);
     launch_end(K_VALIDATE, st);
     return cudaGetLastError();
 }

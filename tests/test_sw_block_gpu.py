@@ -102,3 +102,29 @@ def test_leading_items_only(with_cigar):
         ps = [p[:1500] for p in ps]
     want = oracle.sw_batch(ts, ps, scoring=SCORING, with_cigar=with_cigar)
     assert_sw_equal(sw_gpu(ts, ps, scoring=SCORING, with_cigar=with_cigar), want, "leading items")
+
+
+@pytest.mark.parametrize("n", [1, 31, 1025, 4095, 4096, 4097])
+def test_plan_by_one_block_and_by_many(n):
+    """Every list non-empty, at the sizes around what one block plans."""
+    rng = np.random.default_rng(n)
+    ts, ps = [], []
+    for k in range(n):
+        p = workloads.random_bases(rng, int(rng.integers(0, 70)))
+        t = np.concatenate([workloads.random_bases(rng, int(rng.integers(0, 9))), workloads.mutate_runs(rng, p, 0.1, (0.6, 0.2, 0.2))])
+        if k % 3 == 1 and p.shape[0]:
+            p[-1] = ord("y")
+        if k % 400 == 30:
+            p, t = workloads.random_bases(rng, 1100), workloads.random_bases(rng, 1000 + k % 7)
+            if k % 800 == 30:
+                p[3] = ord("-")
+        ts.append(t.tobytes())
+        ps.append(p.tobytes())
+    before = api.tune_get()
+    try:
+        api.tune_set(**{**before, "sw_long_log2": 20})
+        for with_cigar in (True, False):
+            want = oracle.sw_batch(ts, ps, scoring=SCORING, with_cigar=with_cigar)
+            assert_sw_equal(sw_gpu(ts, ps, scoring=SCORING, with_cigar=with_cigar), want, f"{n} pairs, {with_cigar}")
+    finally:
+        api.tune_set(**before)

@@ -1297,10 +1297,10 @@ static SwPlan bound_plan_sw(const ga_sw_request* reqs, int32_t n, bool trace, in
         // widest item's or the whole of one of coop16 cells (M rows, at most 255
         // padding columns, two words per 64 cells for rows and for edges each)
         const int W = P.w[SP_L16] = sw_coop_block(largest16, maxN16, cells16 / 2, device_sms());
-        const int64_t own = trace ? 0 : SO_ROW_WORDS, fix = trace ? CK_K * T.sw_window * CK_TW : SO_ROW_WORDS;
+        const int64_t own = sw16_own_words(trace, T.sw_window);
         if (W * ((n16 + 1) / 2) <= warps16)
             P.dir[SP_L16] = std::min(P.dir[SP_L16], std::max(sw_coop_share(P.dir[SP_L16], W, own),
-                                                             coop16 / 16 + 16 * (int64_t)maxM16 + fix + 8));
+                                                             coop16 / 16 + 16 * (int64_t)maxM16 + own + 8));
     }
     P.ints[SP_L32] = cnt[SP_L32];
     P.ints[SP_L32LONG] = cnt[SP_L32LONG];

@@ -171,7 +171,7 @@ __device__ __forceinline__ void sp_pack_list(const SwPlanArgs& P, const long lon
             int64_t words = P.score_only ? sw16so_dir_words(M, N) : sw16ck_dir_words(M, N, P.window);
             if ((int64_t)M * N > coop && (few || sw16_by_cells(N))) {
                 ncoop = q + 1;
-                words = sw_coop_share(words, W, P.score_only ? SO_ROW_WORDS : 0);
+                words = sw_coop_share(words, W, sw16_own_words(!P.score_only, P.window));
             }
             local = max(local, (unsigned long long)words);
         }

@@ -145,11 +145,15 @@ __host__ __device__ inline int sw_coop_block(int64_t largest, int cols, int64_t 
     while (W < COOP_MAX_WARPS && W * 512 <= cols && W * cells < 16 * largest * sms) W *= 2;
     return W;
 }
-// Per-warp share of an item's memory when a block of W warps serves it (the
-// score-only kernel keeps SO_ROW_WORDS for each warp).
+// Per-warp share of an item's memory when a block of W warps serves it, `own` words
+// of it for each warp: the score-only kernel's rows, the traceback kernels' table.
 __host__ __device__ inline int64_t sw_coop_share(int64_t words, int W, int64_t own = 0)
 {
     return own + (words - own + 4 * W - 1) / (4 * W) * 4;
+}
+__host__ __device__ inline int64_t sw16_own_words(bool trace, int window)
+{
+    return trace ? (int64_t)CK_K * window * CK_TW : SO_ROW_WORDS;
 }
 // Columns per lane of a whole-block item's full bands: those of 16, 8 and down to
 // `least` with the shortest schedule, of start(last band) + chunks chunks (fwd16_coop)

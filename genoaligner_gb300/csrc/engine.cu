@@ -1278,7 +1278,7 @@ static SwPlan bound_plan_sw(const ga_sw_request* reqs, int32_t n, bool trace, in
         if (trace) {
             int64_t words = sw32ck_dir_words(m, nn, T.sw_long_log2);
             const int64_t c = (int64_t)std::max(m, 0) * std::max(nn, 0);
-            if (c > coop[l]) words = sw_coop_share(words, W32);
+            if (c > coop[l]) words = sw_coop_share(words, W32, sw32_own_words(m, nn, T.sw_long_log2));
             if (c > std::min(limit, SW_COOP_MIN) && limit >= 0) {
                 P.ncoop[l] = 1;
                 P.w[l] = W32;

@@ -184,7 +184,7 @@ __device__ __forceinline__ void sp_pack_list(const SwPlanArgs& P, const long lon
         int64_t words = sw32ck_dir_words(P.D.a_len[a], P.D.b_len[a], P.long_log2);
         if ((int64_t)P.D.a_len[a] * P.D.b_len[a] > coop) {
             ncoop = q + 1;
-            words = sw_coop_share(words, W);
+            words = sw_coop_share(words, W, sw32_own_words(P.D.a_len[a], P.D.b_len[a], P.long_log2));
         }
         local = max(local, (unsigned long long)words);
     }

@@ -121,7 +121,7 @@ __host__ __device__ inline int64_t sw16so_dir_words(int M, int N)
 // limit (the sw_coop_log2 setting, < 0: none), and above twice the list's cells per
 // resident warp.  An item past that share would keep its one warp busy when the
 // others have run out of work: 152 pairs of 8,000 x 8,000 take 28.8 ms on a warp
-// each and 8.2 ms on a block each, and batches with more items than warps stay
+// each and 5.2 ms on a block each, and batches with more items than warps stay
 // below the share.  Items under SW_COOP_MIN cells have too few bands to divide.
 constexpr int64_t SW_COOP_MIN = (int64_t)1 << 16;
 __host__ __device__ inline int64_t sp_coop_cells(int64_t limit, int64_t cells, int64_t warps)
@@ -134,10 +134,10 @@ __host__ __device__ inline int64_t sp_coop_cells(int64_t limit, int64_t cells, i
 // Warps of a whole-block launch's blocks, 4, 8 or 16: enough that the largest item,
 // which gets W of a multiprocessor's 16 resident warps, ends no later than the
 // multiprocessors' common work, and no more than a quarter of the 64-column bands it
-// can be cut into.  152, 304 and 608 pairs of 8,000 x 8,000: 11.4, 13.1, 21.2 ms with
-// 4 warps, 8.9, 12.2, 24.6 with 8, 8.2, 16.2, 32.2 with 16; 1,024 pairs of 2 to 30 kb
-// (one pair holds 1/150 of the cells): 280, 217, 153 ms; 600 pairs of 200 to 1,000 x
-// 1,100 score-only: 0.61, 0.71, 1.54 ms.
+// can be cut into.  (With the walk still one warp's, 152, 304 and 608 pairs of 8,000 x
+// 8,000 took 11.4, 13.1, 21.2 ms with 4 warps, 8.9, 12.2, 24.6 with 8, 8.2, 16.2, 32.2
+// with 16; 1,024 pairs of 2 to 30 kb, one of them 1/150 of the cells, 280, 217, 153 ms;
+// 600 pairs of 200 to 1,000 x 1,100 score-only 0.61, 0.71, 1.54 ms.)
 constexpr int COOP_MAX_WARPS = 16;
 __host__ __device__ inline int sw_coop_block(int64_t largest, int cols, int64_t cells, int sms)
 {
@@ -198,6 +198,12 @@ __host__ __device__ inline int64_t sw32ck_dir_words(int m, int n, int long_log2)
     const int K = lg ? 512 : 64, CT = lg ? 16 : 2, TW = 32 * CT, NWT = CT >= 8 ? CT / 8 : 1;
     const int64_t stride = ((int64_t)c32_ncol(n) + TW - 1) / TW * TW;
     return 2 * (int64_t)c32_rows(m, K) * stride + 2 * (stride / TW) * (int64_t)m + (int64_t)(K + 31) * 32 * NWT;
+}
+
+// The tile table's part of them (sw_coop_share's own words).
+__host__ __device__ inline int64_t sw32_own_words(int m, int n, int long_log2)
+{
+    return sw32ck_long(m, n, long_log2) ? (512 + 31) * 32 * 2 : (64 + 31) * 32;
 }
 
 }  // namespace ga

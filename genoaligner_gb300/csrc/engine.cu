@@ -284,6 +284,8 @@ struct Ctx {
     int sm_count = 0;
     cudaStream_t stream = nullptr;
     cudaEvent_t done = nullptr;     // last work enqueued on a caller's stream
+    cudaStream_t side = nullptr;    // SW batches whose lists run beside each other (launch_plan), and its events
+    cudaEvent_t forked = nullptr, joined = nullptr;
     bool pending = false;
     char* dev = nullptr;
     size_t dev_cap = 0;
@@ -376,6 +378,18 @@ static Ctx* acquire_ctx(const char** err, int tag = -1)
         return nullptr;
     }
     return c;
+}
+
+// The context's second stream and its events, made on first use.
+static bool ensure_side(Ctx* c)
+{
+    if ((!c->side && cudaStreamCreateWithPriority(&c->side, cudaStreamNonBlocking, c->prio) != cudaSuccess) ||
+        (!c->forked && cudaEventCreateWithFlags(&c->forked, cudaEventDisableTiming) != cudaSuccess) ||
+        (!c->joined && cudaEventCreateWithFlags(&c->joined, cudaEventDisableTiming) != cudaSuccess)) {
+        cudaGetLastError();
+        return false;
+    }
+    return true;
 }
 
 static void release_ctx(Ctx* c)
@@ -1160,6 +1174,12 @@ struct SwPlan {
     int32_t w[SP_LISTS] = {4, 4, 4};                 // warps per block: the whole-block items', 4 without any
     int64_t edge_slot = 2;
     int64_t n_opt = 0, dir_opt = 0;
+    double share16 = 0;                              // fork: the 16-bit list's part of the work
+    // The 16-bit and the 32-bit lists run beside each other, on two streams.  Taken when
+    // both have whole-block items (few or uneven long pairs): each alone leaves
+    // multiprocessors idle at its end, 1,024 pairs of 2 to 30 kb 69 + 54 ms one after
+    // the other and 106 ms beside each other.  Needs the plan's own figures.
+    bool fork = false;
 };
 
 static int64_t sw_coop_limit(const ga_tune& T) { return T.sw_coop_log2 < 40 ? ((int64_t)1 << T.sw_coop_log2) : -1; }
@@ -1221,6 +1241,12 @@ static cudaError_t device_plan_sw(const PairDesc& D, const ga_sw_scoring& sc, bo
         P.w[l] = P.ncoop[l] > 0 ? (int32_t)hres[SP_COOPW + l] : 4;
     }
     P.edge_slot = std::max<int64_t>(2, hres[SP_EDGE]);
+    P.fork = trace && P.ncoop[SP_L16] > 0 && P.ncoop[SP_L32LONG] > 0;
+    // (whole-block items measured 12.7 Gcells/s a multiprocessor in 16 bits, 14.7 in 32:
+    // narrower pairs, shorter bands)
+    const double c16 = 1.2 * (double)hres[SP_CELLS + SP_L16],
+                 c32 = (double)(hres[SP_CELLS + SP_L32] + hres[SP_CELLS + SP_L32LONG]);
+    P.share16 = c16 / std::max(1.0, c16 + c32);
     P.n_opt = hres[SP_NOPT];
     P.dir_opt = (hres[SP_DIROPT] + 3) / 4 * 4;
     return cudaSuccess;
@@ -1332,12 +1358,14 @@ struct SwSlots {
     int s[SP_LISTS] = {0, 0, 0};
     int s_esc = 0;                                    // the 32-bit launch for pairs handed over by the 16-bit kernel
     int64_t dir_words = 0, max_slots = 4;
+    int64_t dir16 = 0;                                // fork: the words of the 16-bit list's stream, the table's first
 };
 
 static SwSlots size_sw(const SwPlan& P, bool trace, const ga_tune& T, int sm_count, int64_t budget)
 {
     SwSlots S;
     sw_plan_prepare();
+    if (P.fork) budget /= 2;
     for (int l = 0; l < SP_LISTS; ++l) {
         if (P.ints[l] <= 0) continue;
         // warp slots come in blocks of w; a whole-block item has a block to itself
@@ -1351,8 +1379,16 @@ static SwSlots size_sw(const SwPlan& P, bool trace, const ga_tune& T, int sm_cou
             s = (int)std::min<int64_t>(s, P.ncoop[l] > 0 ? P.ints[l] * w : (P.ints[l] + 3) / 4 * 4);
         }
         if (P.dir[l] > 0) s = (int)std::min<int64_t>(s, std::max<int64_t>(w, budget / (P.dir[l] * 4)));
+        if (P.fork && l != SP_L32) {
+            // lists that would not fit side by side get their parts of the device
+            const int all = sw16ck_max_slots(sm_count, T.sw_window);
+            const int64_t want = P.ints[SP_L16] / 2 * P.w[SP_L16] + P.ints[SP_L32LONG] * P.w[SP_L32LONG];
+            const double part = l == SP_L16 ? P.share16 : 1.0 - P.share16;
+            if (want > all) s = std::min(s, (int)(all * std::min(std::max(part, 0.05), 0.95)));
+        }
         s = std::max(w, s / w * w);
         S.s[l] = s;
+        if (P.fork && l == SP_L16) { S.dir16 = (int64_t)s * P.dir[l]; continue; }
         S.dir_words = std::max(S.dir_words, (int64_t)s * P.dir[l]);
         S.max_slots = std::max<int64_t>(S.max_slots, s);
     }
@@ -1361,9 +1397,11 @@ static SwSlots size_sw(const SwPlan& P, bool trace, const ga_tune& T, int sm_cou
         s = (int)std::min<int64_t>(s, (P.n_opt + 3) / 4 * 4);
         s = (int)std::min<int64_t>(s, std::max<int64_t>(4, budget / (P.dir_opt * 4) / 4 * 4));
         S.s_esc = s;
-        S.dir_words = std::max(S.dir_words, (int64_t)s * P.dir_opt);
+        (P.fork ? S.dir16 : S.dir_words) = std::max(P.fork ? S.dir16 : S.dir_words, (int64_t)s * P.dir_opt);
         S.max_slots = std::max<int64_t>(S.max_slots, s);
     }
+    S.dir16 = (S.dir16 + 63) / 64 * 64;
+    S.dir_words += S.dir16;
     return S;
 }
 
@@ -1376,9 +1414,32 @@ static SwSlots size_sw(const SwPlan& P, bool trace, const ga_tune& T, int sm_cou
 static cudaError_t launch_plan(const SwPlan& P, const SwSlots& S, const PairDesc& D, const ga_sw_scoring& sc,
                                bool trace, const ga_tune& T, const int32_t* dwork, int32_t* out_score, int32_t* out_pos,
                                int32_t* out_len, char* out_cigar, uint32_t* dirs, int32_t* edge, int32_t* ctr,
-                               int32_t* err, cudaStream_t st, int32_t* esc_list, const long long* dplan = nullptr)
+                               int32_t* err, cudaStream_t st0, int32_t* esc_list, const long long* dplan = nullptr,
+                               Ctx* c = nullptr)
 {
-    const int64_t dir_cap = S.dir_words, edge_cap = S.max_slots * P.edge_slot;
+    // with P.fork the 16-bit list, and what it hands over, run on the context's second
+    // stream with the first dir16 words of the table; st0 waits for them at the end
+    const bool fork = P.fork && c;
+    struct Join {
+        Ctx* c;
+        cudaStream_t st;
+        ~Join()
+        {
+            if (!c) return;
+            cudaEventRecord(c->joined, c->side);
+            cudaStreamWaitEvent(st, c->joined, 0);
+        }
+    } join{nullptr, st0};
+    cudaStream_t st = st0;
+    int64_t dir_cap = fork ? S.dir16 : S.dir_words;
+    if (fork) {
+        cudaError_t e = cudaEventRecord(c->forked, st0);
+        if (e == cudaSuccess) e = cudaStreamWaitEvent(c->side, c->forked, 0);
+        if (e != cudaSuccess) return e;
+        join.c = c;
+        st = c->side;
+    }
+    const int64_t edge_cap = S.max_slots * P.edge_slot;
     // ctr: [l] list l's item counter, [6] pairs handed over, [7] their counter
     const bool opt = trace && P.n_opt > 0 && esc_list && S.s_esc > 0;
     int64_t base = 0;
@@ -1414,6 +1475,11 @@ static cudaError_t launch_plan(const SwPlan& P, const SwSlots& S, const PairDesc
         }
     }
     base += P.ints[SP_L16];
+    if (fork) {
+        st = st0;
+        dirs += S.dir16;
+        dir_cap = S.dir_words - S.dir16;
+    }
     for (int l = SP_L32; l <= SP_L32LONG; ++l) {
         if (P.ints[l] > 0) {
             SwArgs A;
@@ -2241,6 +2307,7 @@ int32_t ga_sw_device_ex(const ga_device_batch* b, ga_sw_scoring sc, int32_t trac
     // little more, so it is sized again, with room to spare.
     for (int attempt = 0;; ++attempt) {
         if (!plan()) return fail(E_LAUNCH);
+        P.fork = P.fork && ensure_side(c);
         S = size_sw(P, trace != 0, T, c->sm_count, sw_dir_budget(c, 1));
         const size_t need = run_layout(nullptr, &dctr, &dedge, &ddirs);
         if (need <= c->dev_cap) break;
@@ -2258,7 +2325,7 @@ int32_t ga_sw_device_ex(const ga_device_batch* b, ga_sw_scoring sc, int32_t trac
                                     &P);
             if (x == cudaSuccess)
                 x = launch_plan(P, S, D, sc, true, T, dwork, out_score, out_pos, out_len, out_cigar, ddirs, dedge, dctr,
-                                dctr + 32, st, dscr, dres);
+                                dctr + 32, st, dscr, dres, c);
             return x;
         };
         std::vector<uint64_t> full = key;
@@ -2272,7 +2339,7 @@ int32_t ga_sw_device_ex(const ga_device_batch* b, ga_sw_scoring sc, int32_t trac
     }
     cudaMemsetAsync(dctr, 0, 64 * sizeof(int32_t), st);
     if (launch_plan(P, S, D, sc, trace != 0, T, dwork, out_score, out_pos, out_len, out_cigar, ddirs, dedge, dctr,
-                    dctr + 32, st, dscr) != cudaSuccess)
+                    dctr + 32, st, dscr, nullptr, c) != cudaSuccess)
         return fail(E_LAUNCH);
     if (stream) {
         cudaEventRecord(c->done, st);

@@ -128,3 +128,38 @@ def test_plan_by_one_block_and_by_many(n):
             assert_sw_equal(sw_gpu(ts, ps, scoring=SCORING, with_cigar=with_cigar), want, f"{n} pairs, {with_cigar}")
     finally:
         api.tune_set(**before)
+
+
+def test_device_entry_lists_side_by_side_after_the_arena_grew():
+    """Long pairs of both widths (two streams), three times the size of the call before:
+    the plan is made again in the grown arena and sized again."""
+    torch = pytest.importorskip("torch")
+    rng = np.random.default_rng(8)
+    for n in (2, 30, 90):
+        ts, ps = [], []
+        for k in range(n):
+            p = workloads.random_bases(rng, int(rng.integers(300, 1500)))
+            t = np.concatenate([workloads.mutate_runs(rng, p, 0.1, (0.6, 0.2, 0.2)),
+                                workloads.random_bases(rng, int(rng.integers(0, 400)))])
+            if k % 2:
+                p[p.shape[0] // 2] = ord("q")
+            ts.append(t.tobytes())
+            ps.append(p.tobytes())
+        want = oracle.sw_batch(ts, ps, scoring=SCORING, with_cigar=True)
+        q = packed(ts, ps)
+        batch = api.DeviceBatchT(q.a_buf, q.a_off, q.a_len, q.b_buf, q.b_off, q.b_len)
+        before = api.tune_get()
+        try:
+            api.tune_set(**{**before, "sw_long_log2": 20})
+            score, pos, length = (torch.zeros(k * n, dtype=torch.int32, device="cuda") for k in (1, 4, 1))
+            cigar = torch.zeros(batch.out_bytes, dtype=torch.uint8, device="cuda")
+            for limit in (-1, 1 << 26, 1 << 26, 1 << 26):           # as it is, then captured and replayed
+                score.zero_()
+                cigar.zero_()
+                api.sw_device(batch, SCORING, True, score, pos, length, cigar, trace_cell_limit=limit)
+                assert np.array_equal(score.cpu().numpy(), want.score)
+                got, ends = cigar.cpu().numpy(), (batch.out_off + batch.a_len + batch.b_len).cpu().numpy()
+                for k in range(n):
+                    assert got[int(ends[k]) - int(length[k]): int(ends[k])].tobytes() == want.cigars[k], (n, limit, k)
+        finally:
+            api.tune_set(**before)

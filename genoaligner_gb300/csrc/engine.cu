@@ -1281,9 +1281,10 @@ static SwPlan bound_plan_sw(const ga_sw_request* reqs, int32_t n, bool trace, in
     for (int32_t i = 0; i < n; ++i) {
         const int m = reqs[i].text_len, nn = reqs[i].pattern_len;
         if (cell_limit >= 0 && m > 0 && nn > 0 && ((int64_t)m + 1) * ((int64_t)nn + 1) > cell_limit) continue;
-        const bool strict = T.sw_pack16 && sw16_eligible(m, nn, sc.match, sc.mismatch, sc.gap_open, sc.gap_extend);
+        const bool rows16 = T.sw_pack16 && (!trace || m <= SW16_TRACE_ROWS);
+        const bool strict = rows16 && sw16_eligible(m, nn, sc.match, sc.mismatch, sc.gap_open, sc.gap_extend);
         // (the SW model may send any pair to the 16-bit kernel)
-        const bool u16 = strict || (trace && T.sw_pack16 &&
+        const bool u16 = strict || (trace && rows16 &&
                                     (learned ? (m > 0 && nn > 0 &&
                                                 sw16_scheme_ok(sc.match, sc.mismatch, sc.gap_open, sc.gap_extend))
                                              : sw16_eligible_opt(m, nn, sc.match, sc.mismatch, sc.gap_open,

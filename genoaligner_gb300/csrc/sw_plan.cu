@@ -44,7 +44,7 @@ __device__ __forceinline__ int sp_classify(const SwPlanArgs& P, int p, SpTally& 
         P.out_score[p] = P.too_large_score;
         return -1;
     }
-    const bool pure = P.use16 && P.D.pure[p] && P.D.pure[n + p];
+    const bool pure = P.use16 && P.D.pure[p] && P.D.pure[n + p] && (P.score_only || m <= SW16_TRACE_ROWS);
     const bool strict = pure && sw16_eligible(m, nn, P.match, P.mismatch, P.gap_open, P.gap_extend);
     const bool opt = P.try16 ? (P.try16[p] != 0 && m > 0 && nn > 0 &&
                                 sw16_scheme_ok(P.match, P.mismatch, P.gap_open, P.gap_extend))

@@ -23,6 +23,10 @@ __host__ __device__ inline bool sw16_eligible(int m, int n, int match, int misma
     return top < 32000;
 }
 
+// The 16-bit traceback kernel keeps a row number in 16 bits: longer texts are the
+// 32-bit kernels'.
+constexpr int SW16_TRACE_ROWS = 65535;
+
 // Optimistic 16-bit eligibility: the bound above with the all-match score
 // scaled by pct / 100 (pct 100: the bound itself).  A pair taken on this
 // rule alone may score past 16 bits; the kernel then sees a best value of at

@@ -163,3 +163,17 @@ def test_device_entry_lists_side_by_side_after_the_arena_grew():
                     assert got[int(ends[k]) - int(length[k]): int(ends[k])].tobytes() == want.cigars[k], (n, limit, k)
         finally:
             api.tune_set(**before)
+
+
+@pytest.mark.parametrize("rows", [65535, 65536, 70000])
+def test_texts_past_16_bit_rows(rows):
+    """The alignment ends in the last rows of a text that 16 bits just hold or do not."""
+    rng = np.random.default_rng(rows)
+    p = workloads.random_bases(rng, 60)
+    t = workloads.random_bases(rng, rows)
+    t[-70:-10] = p
+    t2 = workloads.random_bases(rng, 900)
+    ts, ps = [t.tobytes(), t2.tobytes()], [p.tobytes(), t2[100:700].tobytes()]
+    for with_cigar in (True, False):
+        want = oracle.sw_batch(ts, ps, scoring=SCORING, with_cigar=with_cigar)
+        assert_sw_equal(sw_gpu(ts, ps, scoring=SCORING, with_cigar=with_cigar), want, f"{rows} rows, {with_cigar}")

@@ -1651,7 +1651,7 @@ static int32_t sw_batch_range(const ga_sw_request* reqs, int32_t n, int64_t base
         return GA_DEVICE_ERROR;
     }
     // the device work: a fixed sequence for a given launch shape (no plan read
-    // back), so it is captured once per shape and replayed as a CUDA graph
+    // back), so it is captured and replayed as a CUDA graph when its shape repeats
     auto enqueue = [&]() -> cudaError_t {
         cudaStream_t st = c->stream;
         // sentinel: too-large pairs keep score -1 (never written by a kernel)

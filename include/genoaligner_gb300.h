@@ -197,8 +197,9 @@ int32_t ga_wfa_device(const ga_device_batch* batch, int32_t smax, int32_t trace,
 /* ga_wfa_device with extension options (opt may be NULL): opt->learned = 1
  * routes pairs by the cost model (loaded with ga_cost_model_set) into two
  * bucketed queues served by persistent kernels (one pair per lane for small
- * predicted distances, one pair per warp otherwise), replayed as one CUDA
- * graph; results are the same as without it. */
+ * predicted distances, one pair per warp otherwise, large distances on whole
+ * blocks), replayed as one CUDA graph when a launch shape repeats; results are
+ * the same as without it. */
 int32_t ga_wfa_device_ex(const ga_device_batch* batch, int32_t smax, int32_t trace, const ga_options* opt,
                          int32_t* out_score, int32_t* out_len, char* out_cigar, void* stream,
                          const char** err);
@@ -207,7 +208,7 @@ int32_t ga_wfa_device_ex(const ga_device_batch* batch, int32_t smax, int32_t tra
  * in the lane queue (one pair per lane), out[1] = pairs in the warp queue (one
  * pair per warp or per group of lanes), out[2] = pairs the lane queue escalated to the warp queue
  * (unresolved within their first smax, or handed over), out[3] = warp-queue
- * pairs run on a whole block (estimated distance >= 256); out[4..] = 0.  A
+ * pairs sent to whole blocks at once (estimated distance >= 256); out[4..] = 0.  A
  * host batch of 262,144 pairs or more runs in up to 4 ranges: the record is
  * then its last range's.  Synchronises the device. */
 int32_t ga_wfa_route_stats(int32_t* out, int32_t max);
@@ -232,7 +233,7 @@ int32_t ga_sw_device(const ga_device_batch* batch, ga_sw_scoring scoring, int32_
 
 /* ga_sw_device with extension options (opt may be NULL): opt->learned = 1
  * lets the SW variant model (model slot 1, ga_model_select) choose, pair by
- * pair, which pure-ACGT pairs beyond the proven 16-bit bound try the 16-bit
+ * pair, which pairs of A, C, G, T and N beyond the proven 16-bit bound try the 16-bit
  * two-pairs-per-warp kernel (one whose best reaches the 16-bit limit is
  * recomputed in 32 bits); results are the same as without it.  No reference
  * counterpart. */
@@ -388,7 +389,7 @@ int32_t ga_sw_qc_device(const ga_device_batch* batch, const int32_t* score, cons
  * used by every later call on that device (ga_sw_device, ga_align_sw_batch,
  * the learned WFA path). */
 typedef struct ga_tune {
-    int32_t sw_pack16;      /* SW traceback, pure-ACGT pairs whose scores fit 16 bits:
+    int32_t sw_pack16;      /* SW traceback, pairs of A, C, G, T, N whose scores fit 16 bits:
                                1 = two pairs per warp in 16-bit halves (inter-sequence),
                                0 = one pair per warp in 32 bits (intra-sequence) */
     int32_t sw_window;      /* 16-bit traceback: tiles of 64 columns recomputed per
@@ -398,11 +399,11 @@ typedef struct ga_tune {
                                the 512 x 512 tile shape, the rest 64 x 64; 16 .. 30 */
     int32_t wfa_lane_smax;  /* learned WFA: pairs whose first smax is <= this run one
                                per lane, 32 per warp (0 = none: one pair per warp); 0 .. 31 */
-    int32_t sw_coop_log2;   /* SW traceback: work items above 2^sw_coop_log2 cells (a 32-bit
-                               long-shape pair, or a 16-bit item of two pairs) run their forward
-                               pass on the 4 warps of a block (128 lanes) instead of one warp;
-                               16 .. 40 (40: never) */
-    int32_t sw_opt16_pct;   /* SW traceback: a pure-ACGT pair whose all-match score scaled by
+    int32_t sw_coop_log2;   /* SW: work items above 2^sw_coop_log2 cells (a 32-bit pair, or a
+                               16-bit item of two pairs) run on a block of 4, 8 or 16 warps
+                               instead of one warp, and so do smaller ones in batches that would
+                               leave warps idle; 16 .. 40 (40: none does) */
+    int32_t sw_opt16_pct;   /* SW traceback: a pair of A, C, G, T, N whose all-match score scaled by
                                sw_opt16_pct / 100 fits 16 bits runs on the 16-bit kernel; one
                                whose best then reaches the 16-bit limit is recomputed in 32 bits
                                (exact either way).  50 .. 100 (100: only pairs whose all-match

@@ -568,7 +568,8 @@ __global__ void __launch_bounds__(256) mlp_forward_tc_kernel(const __nv_bfloat16
 // ------------------------------------------ fused routing inference --
 // Sketch, lower bound, tensor-core forward pass and queue choice of every pair
 // of a WFA batch in one pass, one warp per 16 pairs: lane l < 16 counts the
-// 3-mers of side a of pair l of the tile, lane l + 16 those of side b, into a
+// 3-mers of side a of pair l of the tile, lane l + 16 those of side b (2^lg lanes a
+// side in batches too small for that to use every warp: 16 >> lg pairs), into a
 // private histogram column hist[bin][lane] (bin = c0 + 4 c1 + 16 c2, the 2-bit
 // window's own order); feature k = 16 c0 + 4 c1 + c2 of pair r is hist[bin][r] -
 // hist[bin][r + 16].  Features, bf16 rounding and the network
@@ -580,13 +581,15 @@ __global__ void __launch_bounds__(256) mlp_forward_tc_kernel(const __nv_bfloat16
 constexpr int RM_WARPS = 16;
 constexpr int RM_ROW = 44;        // words of a row of the feature tile: 80 features, rows on distinct banks by fours
 
-template <bool MODEL>
+template <bool MODEL, bool SPLIT>
 __global__ void __launch_bounds__(512) route_model_kernel(const __nv_bfloat16* __restrict__ w, PairDesc D, int smax,
                                                           int lane_smax,
                                                           int32_t* __restrict__ item, int32_t* __restrict__ lb_out,
                                                           float* __restrict__ y_out, int32_t* __restrict__ counts,
-                                                          int32_t* __restrict__ out_score, int32_t* __restrict__ out_len)
+                                                          int32_t* __restrict__ out_score, int32_t* __restrict__ out_len,
+                                                          int split_log2)
 {
+    const int lg = SPLIT ? split_log2 : 0;                     // 2^lg lanes to a side: 16 >> lg pairs to a tile
     extern __shared__ __align__(16) unsigned char rm_raw[];
     TcSmem& S = *reinterpret_cast<TcSmem*>(rm_raw);
     int* hist_all = reinterpret_cast<int*>(rm_raw + sizeof(TcSmem));
@@ -600,10 +603,10 @@ __global__ void __launch_bounds__(512) route_model_kernel(const __nv_bfloat16* _
     const int* Hw = hist_all + wib * 64 * 32;
     const int n = D.n;
     const int warps = (gridDim.x * blockDim.x) >> 5;
-    for (int tile = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; tile * 16 < n; tile += warps) {
+    for (int tile = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; tile * (16 >> lg) < n; tile += warps) {
 #pragma unroll 8
         for (int b = 0; b < 64; ++b) H[b * 32] = 0;
-        const int p = tile * 16 + sl;
+        const int p = tile * (16 >> lg) + (sl >> lg);
         int m = 0, nn = 0;
         if (p < n) {
             m = D.a_len[p];
@@ -612,7 +615,7 @@ __global__ void __launch_bounds__(512) route_model_kernel(const __nv_bfloat16* _
             const int L = side ? nn : m;
             // 256 symbols at a time: the 8 words that hold them and the next
             // one (3-mers straddle it) are loaded together, then counted
-            for (int q0 = 0; q0 + 2 < L; q0 += 256) {
+            for (int q0 = 256 * (sl & ((1 << lg) - 1)); q0 + 2 < L; q0 += 256 << lg) {
                 uint64_t wd[9];
                 const int wlast = ((L - 1) >> 5) - (q0 >> 5) + 1;     // words past this lie beyond the arena's spare
 #pragma unroll
@@ -627,6 +630,16 @@ __global__ void __launch_bounds__(512) route_model_kernel(const __nv_bfloat16* _
                     for (int i = 0; i < 16; ++i)
                         if (i < cnt) ++H[(int)((v >> (2 * i)) & 63u) * 32];   // the lane's own column: no atomic
                 }
+            }
+        }
+        if (SPLIT && __any_sync(FULL, max(m, nn) > 258)) {
+            // a side's lanes each take its counts (with no more than 256 3-mers a side
+            // they are its first lane's, the one whose outputs are kept)
+#pragma unroll 4
+            for (int b = 0; b < 64; ++b) {
+                int v = H[b * 32];
+                for (int o = 1; o < 1 << lg; o <<= 1) v += __shfl_xor_sync(FULL, v, o);
+                H[b * 32] = v;
             }
         }
         __syncwarp();
@@ -681,8 +694,8 @@ __global__ void __launch_bounds__(512) route_model_kernel(const __nv_bfloat16* _
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
                 const int r = h ? r1 : r0;
-                const int pr = tile * 16 + r;
-                if (pr >= n) continue;
+                const int pr = tile * (16 >> lg) + (r >> lg);
+                if (pr >= n || (r & ((1 << lg) - 1)) != 0) continue;
                 const int mr = h ? m1 : m0, nr = h ? n1 : n0, lbr = h ? lb1 : lb0;
                 const float y0 = h ? o[2] : o[0];
                 const int it = route_item(mr, nr, D.pure[pr] != 0, D.pure[n + pr] != 0, lbr, y0, smax, lane_smax);
@@ -714,15 +727,18 @@ cudaError_t launch_route_model(const PairDesc& D, int smax, int lane_smax, bool 
     const __nv_bfloat16* w = cost_model_weights();
     if (model && !w) return cudaErrorNotReady;
     if (D.n <= 0) return cudaSuccess;
-    int blocks = (D.n + 16 * RM_WARPS - 1) / (16 * RM_WARPS);
+    // Lanes to a side: as many as keep every tile a warp of its own.  One lane a side
+    // leaves the 2,000 long pairs' counting to 125 warps (2,000 of 2-10 kb: pass 256 us,
+    // with 16 lanes 47); the rows a tile then lacks cost nothing that waits.
+    int lg = 0;
+    while (lg < 4 && ((int64_t)D.n << (lg + 1)) <= (int64_t)16 * RM_WARPS * device_sms()) ++lg;
+    int blocks = (int)((((int64_t)D.n << lg) + 16 * RM_WARPS - 1) / (16 * RM_WARPS));
     blocks = std::min(blocks, device_sms());
     launch_begin(K_MLP, st);
-    if (model)
-        route_model_kernel<true><<<blocks, 32 * RM_WARPS, route_model_smem(), st>>>(w, D, smax, lane_smax, item, lb, y,
-                                                                                    counts, out_score, out_len);
-    else
-        route_model_kernel<false><<<blocks, 32 * RM_WARPS, route_model_smem(), st>>>(w, D, smax, lane_smax, item, lb,
-                                                                                     y, counts, out_score, out_len);
+    auto kernel = model ? (lg ? route_model_kernel<true, true> : route_model_kernel<true, false>)
+                        : (lg ? route_model_kernel<false, true> : route_model_kernel<false, false>);
+    kernel<<<blocks, 32 * RM_WARPS, route_model_smem(), st>>>(w, D, smax, lane_smax, item, lb, y, counts, out_score,
+                                                              out_len, lg);
     launch_end(K_MLP, st);
     return cudaGetLastError();
 }
@@ -785,10 +801,9 @@ void prepare_mlp()
         cudaFuncSetAttribute(mlp_forward_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(MlpSmem));
         cudaFuncSetAttribute(mlp_backward_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(MlpSmem));
         cudaFuncSetAttribute(mlp_forward_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(TcSmem));
-        cudaFuncSetAttribute(route_model_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)route_model_smem());
-        cudaFuncSetAttribute(route_model_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)route_model_smem());
+        for (auto kernel : {route_model_kernel<true, true>, route_model_kernel<true, false>,
+                            route_model_kernel<false, true>, route_model_kernel<false, false>})
+            cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)route_model_smem());
     });
 }
 

@@ -16,8 +16,8 @@ constexpr int LANE_MAXLEN = 256;
 // predicted distance bound, ROUTE_BUCKETS + s the lane queue with first smax s.
 constexpr int ROUTE_BUCKETS = 32;
 // Warp-queue items whose bucket key (bit length of the estimated distance) is
-// at least BLOCK_BITS -- estimated s >= 256 -- run first, each on a whole
-// block of the warp kernel (128 threads over the diagonals of one pair).
+// at least BLOCK_BITS -- estimated s >= 256 -- are the block kernel's (512
+// threads over the diagonals of one pair).
 constexpr int BLOCK_BITS = 9;
 
 __device__ __forceinline__ int bitlen(unsigned x) { return 32 - __clz(x); }

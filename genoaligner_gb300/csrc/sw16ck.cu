@@ -1035,7 +1035,7 @@ __device__ void ck_item(const Sw16Args& A, const int32_t* __restrict__ pwork, in
                 if (i <= 0 || j <= 0 || v == 0) fin = true;
             }
             if (fin || !coop) break;
-            // another window of this round, where the walk goes on inside it
+            // another window of this pass, where the walk goes on inside it
             k = (ti0[x] - 1) / CK_K - (i - 1) / CK_K;
             if (k < 1 || k >= nwin || s_win[k][x] < 0 || j <= TW * (s_win[k][x] - (TG - 1)) || j > TW * (s_win[k][x] + 1))
                 break;

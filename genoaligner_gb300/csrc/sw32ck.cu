@@ -565,7 +565,7 @@ __device__ void c32_pair(const SwArgs& A, int p, bool coop, int wib, int t, uint
             if (t == 0) slotc[pos] = op;
         }
             if (fin || !coop) break;
-            // another tile of this round, where the walk goes on
+            // another tile of this pass, where the walk goes on
             const int e0 = ((i - 1) / K) * K + 1, eb = (j - 1) / TW;
             const unsigned hit = __ballot_sync(FULL, t < nwin && s_win[t < nwin ? t : 0][0] == e0 && s_win[t < nwin ? t : 0][1] == eb);
             if (!hit) break;

@@ -284,7 +284,7 @@ struct Ctx {
     int sm_count = 0;
     cudaStream_t stream = nullptr;
     cudaEvent_t done = nullptr;     // last work enqueued on a caller's stream
-    cudaStream_t side = nullptr;    // SW batches whose lists run beside each other (launch_plan), and its events
+    cudaStream_t side = nullptr;    // launches that run beside the stream's (launch_plan, enqueue_wfa), and its events
     cudaEvent_t forked = nullptr, joined = nullptr;
     bool pending = false;
     char* dev = nullptr;
@@ -625,6 +625,8 @@ static const char* wfa_request_error(const ga_align_request& r, int32_t max_smax
 struct WfaScratch {
     uint64_t* packed = nullptr;
     uint8_t* pure = nullptr;
+    int32_t* block_stack = nullptr;  // the block kernel's stacks
+    bool beside = false;             // the learned path's block kernel beside its warp kernels
     int32_t* stack = nullptr;
     int32_t* ctr = nullptr;          // 64 ints: plain counter; learned: round counters
     int32_t* item = nullptr;         // queue item per pair (bucket | first smax << 8, or -1)
@@ -656,6 +658,7 @@ struct WfaScratch {
 // knows nothing of a pair, restarts the ones past 255 there (a 64th of the work
 // of a pair at 2048).
 constexpr int WFA_WARP_CAP = 511, WFA_PLAIN_CAP = 255;
+constexpr int64_t WFA_STACK_BYTES = (int64_t)16 << 30;     // stack memory cap
 // Below this no pair is estimated at the block kernel's distances.
 constexpr int WFA_BLOCK_MIN = 256;
 
@@ -678,7 +681,7 @@ static void size_wfa(WfaScratch& S, int n, int smax, bool trace, bool learned, i
     }
     if (blocks) S.blocks = std::min(wfa_block_slots(smax, trace, sm_count), std::max(n, 1));
     if (trace) {
-        const int64_t budget = (int64_t)16 << 30;     // stack memory cap
+        const int64_t budget = WFA_STACK_BYTES;
         S.slots = (int)std::min<int64_t>(S.slots, std::max<int64_t>(4, budget / (S.stack_slot * 4) / 4 * 4));
         S.blocks = (int)std::min<int64_t>(S.blocks, std::max<int64_t>(1, budget / ((int64_t)(smax + 1) * (smax + 1) * 4)));
     }
@@ -692,10 +695,14 @@ static void carve_wfa(Carve& k, WfaScratch& S, int n, int64_t arena, bool trace,
     S.packed = k.take<uint64_t>(packed_arena_words(arena));
     S.pure = k.take<uint8_t>(2 * (size_t)n);
     S.ctr = k.take<int32_t>(64, 256);
-    // the warp kernels and the block kernel run one after the other and share the stacks
-    S.stack = trace ? k.take<int32_t>((size_t)std::max<int64_t>((int64_t)S.slots * S.stack_slot,
-                                                                (int64_t)S.blocks * (S.smax + 1) * (S.smax + 1)))
+    // kernels that run one after the other share the stacks; the learned path's warp and
+    // block kernels run beside each other unless that takes more than one alone may
+    const int64_t warp_words = trace ? (int64_t)S.slots * S.stack_slot : 0;
+    const int64_t block_words = trace ? (int64_t)S.blocks * (S.smax + 1) * (S.smax + 1) : 0;
+    S.beside = learned && S.blocks > 0 && (warp_words + block_words) * 4 <= WFA_STACK_BYTES;
+    S.stack = trace ? k.take<int32_t>((size_t)(S.beside ? warp_words + block_words : std::max(warp_words, block_words)))
                     : nullptr;
+    S.block_stack = trace && S.beside ? S.stack + warp_words : S.stack;
     S.blk = k.take<int32_t>(S.blocks > 0 ? n : 0);
     if (learned) {
         S.item = k.take<int32_t>(n);
@@ -712,7 +719,9 @@ static void carve_wfa(Carve& k, WfaScratch& S, int n, int64_t arena, bool trace,
 
 // Every launch of one WFA batch on stream st (inputs already on the device).
 // route: 0 plain, 1 queues by the cost model, 2 queues by the lower bound alone.
-static cudaError_t enqueue_wfa(const WfaScratch& S, PairDesc D, int smax, bool trace, int route, int lane_smax,
+// c: the calling context, whose second stream the learned path's lane and warp kernels
+// take while the block kernel runs the pairs estimated to be its own (null: one stream).
+static cudaError_t enqueue_wfa(Ctx* c, const WfaScratch& S, PairDesc D, int smax, bool trace, int route, int lane_smax,
                                int32_t* score, int32_t* len, char* cig, int32_t* err, cudaStream_t st)
 {
     D.packed = S.packed;
@@ -725,6 +734,7 @@ static cudaError_t enqueue_wfa(const WfaScratch& S, PairDesc D, int smax, bool t
     A.cap = S.cap; A.blk = S.blk; A.blk_count = S.ctr + 33;
     WfaBlockArgs B;
     B.A = A;
+    B.A.stack = S.block_stack;
     B.next = S.ctr + 3;
     const int NB = route_buckets();
     Fills F;
@@ -745,7 +755,7 @@ static cudaError_t enqueue_wfa(const WfaScratch& S, PairDesc D, int smax, bool t
         return e;
     if ((e = launch_route(D.n, S.item, S.counts, S.starts, S.big, S.small, st)) != cudaSuccess) return e;
     // ctr layout: [0] warp-queue next, [1] lane-queue next, [2] escalation
-    // next, [3] whole-block next, [32] escalation count, [33] pairs left to
+    // next, [3] and [4] whole-block next, [32] escalation count, [33] pairs left to
     // whole blocks; counts[2 NB + 2]: whole-block items (the warp queue's first
     // ones)
     RoutedArgs R;
@@ -764,10 +774,29 @@ static cudaError_t enqueue_wfa(const WfaScratch& S, PairDesc D, int smax, bool t
     R.esc_next = S.ctr + 2;
     R.lane_rec = S.lane_rec;
     R.block_count = S.blocks > 0 ? S.counts + 2 * NB + 2 : nullptr;
-    e = launch_routed(R, S.lane_slots, S.slots, st);
-    if (e != cudaSuccess || S.blocks == 0) return e;
     B.big = S.big;
     B.big_count = R.block_count;
+    // Beside each other: the block kernel holds most of each multiprocessor and is bound
+    // by its steps' barriers, the few warps it leaves room for by their pairs' chains
+    // (2,000 pairs of 2-10 kb: 0.7 + 3.0 ms one after the other, 3.89 ms a call -> 3.48).
+    // What the warp kernels leave to blocks runs after both.
+    if (S.beside && c) {
+        if ((e = cudaEventRecord(c->forked, st)) != cudaSuccess ||
+            (e = cudaStreamWaitEvent(c->side, c->forked, 0)) != cudaSuccess) return e;
+        WfaBlockArgs first = B;
+        first.A.blk_count = nullptr;
+        e = launch_wfa_block(first, S.blocks, K_WFA_ROUTED, st);
+        const cudaError_t e2 = launch_routed(R, S.lane_slots, S.slots, c->side);
+        cudaEventRecord(c->joined, c->side);
+        cudaStreamWaitEvent(st, c->joined, 0);
+        if (e != cudaSuccess || e2 != cudaSuccess) return e != cudaSuccess ? e : e2;
+        if (S.cap >= smax) return cudaSuccess;
+        B.big_count = nullptr;
+        B.next = S.ctr + 4;
+        return launch_wfa_block(B, S.blocks, K_WFA_ROUTED, st);
+    }
+    e = launch_routed(R, S.lane_slots, S.slots, st);
+    if (e != cudaSuccess || S.blocks == 0) return e;
     return launch_wfa_block(B, S.blocks, K_WFA_ROUTED, st);
 }
 
@@ -823,7 +852,7 @@ static cudaError_t run_wfa_graph(Ctx* c, const WfaScratch& S, const PairDesc& D,
                                        (uint64_t)(uintptr_t)D.a_off, (uint64_t)(uintptr_t)S.packed,
                                        (uint64_t)(uintptr_t)err};
     return replay_graph(c->gexec, c->gkey, c->gseen, key, c->glaunches, st, [&]() {
-        return enqueue_wfa(S, D, smax, trace, route, lane_smax, score, len, cig, err, st);
+        return enqueue_wfa(c, S, D, smax, trace, route, lane_smax, score, len, cig, err, st);
     });
 }
 
@@ -1070,10 +1099,11 @@ int32_t wfa_batch(const ga_align_request* reqs, int32_t n, int32_t max_smax, int
             return GA_DEVICE_ERROR;
         }
         cudaError_t le;
+        S.beside = S.beside && ensure_side(c);
         if (fail_here(3)) le = cudaErrorLaunchFailure;
         else if (learned && !profiling_on())
             le = run_wfa_graph(c, S, D, smax, trace, route, lane_smax, dsc, dln, dcg, der, c->stream);
-        else le = enqueue_wfa(S, D, smax, trace, route, lane_smax, dsc, dln, dcg, der, c->stream);
+        else le = enqueue_wfa(c, S, D, smax, trace, route, lane_smax, dsc, dln, dcg, der, c->stream);
         if (learned) note_route(c, S, nk);
         if (le == cudaSuccess && trace) le = launch_wfa_validate(D, dsc, dln, dcg, dvf, c->stream, dpo, dpk);
         if (le != cudaSuccess) {
@@ -2117,9 +2147,10 @@ int32_t ga_wfa_device_ex(const ga_device_batch* b, int32_t smax, int32_t trace, 
     cudaError_t le;
     {
         const int lane_smax = tuned.wfa_lane_smax;
+        S.beside = S.beside && ensure_side(c);
         if (learned && !profiling_on())
             le = run_wfa_graph(c, S, D, smax, trace != 0, route, lane_smax, out_score, out_len, out_cigar, derr, st);
-        else le = enqueue_wfa(S, D, smax, trace != 0, route, lane_smax, out_score, out_len, out_cigar, derr, st);
+        else le = enqueue_wfa(c, S, D, smax, trace != 0, route, lane_smax, out_score, out_len, out_cigar, derr, st);
         if (learned) note_route(c, S, b->n);
     }
     if (le != cudaSuccess) {

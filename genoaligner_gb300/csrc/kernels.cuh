@@ -101,7 +101,7 @@ struct RoutedArgs {
 };
 
 // Pairs on whole blocks (wfa_block.cu): the first *big_count of the warp queue
-// (null: none), then the warp kernels' unresolved ones (A.blk).  A.stack: per
+// (null: none), then the warp kernels' unresolved ones (A.blk, A.blk_count null: none).  A.stack: per
 // block (A.smax + 1)^2 offsets.
 struct WfaBlockArgs {
     WfaArgs A;

@@ -91,7 +91,7 @@ __global__ void __launch_bounds__(BLK_T, 2) wfa_block_kernel(WfaBlockArgs B)
     __shared__ int s_q, s_at[3];
     const WfaArgs& A = B.A;
     const int t = threadIdx.x, smax = A.smax;
-    const int nbig = B.big_count ? *B.big_count : 0, cnt = nbig + *A.blk_count;
+    const int nbig = B.big_count ? *B.big_count : 0, cnt = nbig + (A.blk_count ? *A.blk_count : 0);
     int32_t* const wf0 = bsmem;
     int32_t* const wf1 = bsmem + 2 * smax + 3;
     int32_t* const stk = TRACE ? A.stack + blockIdx.x * ((int64_t)(smax + 1) * (smax + 1)) : nullptr;

@@ -40,3 +40,17 @@ def test_block_pairs_match_oracle(pairs, smax, learned):
     assert_wfa_equal(got, want, f"smax {smax}, learned {learned}")
     score = wfa_gpu(ps, ts, smax=smax, with_cigar=False, max_smax=4096, learned=learned)
     assert np.array_equal(score.res["score"], want.score)
+
+
+@pytest.mark.parametrize("copies", [1, 64])
+def test_block_kernel_beside_the_warps_and_after_them(pairs, copies):
+    """The largest smax: the stacks of few pairs fit for both kernels at once, those of
+    2,432 pairs do not, so there the kernels run one after the other."""
+    assert cost_model.load_default()
+    ps, ts = pairs
+    want = oracle.wfa_batch(ps, ts, smax=3500, with_cigar=True, max_smax=4096)
+    got = wfa_gpu(ps * copies, ts * copies, smax=3500, max_smax=4096, learned=True)
+    assert np.array_equal(got.res["score"], np.tile(want.score, copies))
+    for k in range(len(ps)):
+        for c in (0, copies - 1):
+            assert got.cigar(c * len(ps) + k) == want.cigars[k], (copies, c, k)

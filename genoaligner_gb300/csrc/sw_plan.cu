@@ -190,32 +190,63 @@ __device__ __forceinline__ void sp_pack_list(const SwPlanArgs& P, const long lon
     }
 }
 
-// One warp per list: exclusive scan of its bucket counts (bucket order is
-// largest first), then sp_lay_out.
-__global__ void sp_scan_kernel(SwPlanArgs P)
+// Exclusive scan of each list's bucket counts (bucket order is largest first) by one
+// block of SP_SCAN_T threads: start[l][b] for list l's bucket b, in cnt's place or in
+// another array (flat: counted on from list to list); the lists' totals.
+constexpr int SP_SCAN_T = 1024;
+__device__ __forceinline__ void sp_scan(const int32_t* cnt, int32_t* start, bool flat, int32_t (*warp_sum)[32],
+                                        long long* total)
 {
-    __shared__ long long total[SP_LISTS];
-    const int lane = threadIdx.x & 31, L = threadIdx.x >> 5;
-    if (L < SP_LISTS) {
-        const int per = SP_NB / 32;
-        const int32_t* cnt = P.counts + L * SP_NB + lane * per;
-        int32_t* st = P.starts + L * SP_NB + lane * per;
-        int sum = 0;
-        for (int b = 0; b < per; ++b) sum += cnt[b];
-        int incl = sum;
+    constexpr int BPT = SP_NB / SP_SCAN_T;
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    int own[SP_LISTS], incl[SP_LISTS];
+#pragma unroll
+    for (int l = 0; l < SP_LISTS; ++l) {
+        own[l] = 0;
+#pragma unroll
+        for (int k = 0; k < BPT; ++k) own[l] += cnt[l * SP_NB + tid * BPT + k];
+        incl[l] = own[l];
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
-            const int v = __shfl_up_sync(FULL, incl, o);
-            if (lane >= o) incl += v;
+            const int v = __shfl_up_sync(FULL, incl[l], o);
+            if (lane >= o) incl[l] += v;
         }
-        int acc = incl - sum;
-        for (int b = 0; b < per; ++b) {
-            st[b] = acc;
-            acc += cnt[b];
-        }
-        if (lane == 31) total[L] = incl;
+        if (lane == 31) warp_sum[l][wid] = incl[l];
     }
     __syncthreads();
+    if (wid < SP_LISTS) {
+        const int v = warp_sum[wid][lane];
+        int s = v;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int u = __shfl_up_sync(FULL, s, o);
+            if (lane >= o) s += u;
+        }
+        warp_sum[wid][lane] = s - v;
+        if (lane == 31) total[wid] = s;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int l = 0; l < SP_LISTS; ++l) {
+        int acc = warp_sum[l][wid] + incl[l] - own[l];
+        if (flat)                                      // one array for all lists: behind the lists before
+            for (int k = 0; k < l; ++k) acc += (int)total[k];
+#pragma unroll
+        for (int k = 0; k < BPT; ++k) {
+            const int c = cnt[l * SP_NB + tid * BPT + k];
+            start[l * SP_NB + tid * BPT + k] = acc;
+            acc += c;
+        }
+    }
+}
+
+// (A warp per list, 128 buckets a lane, took 30 us of a 200,000-pair plan; this
+// 7.)
+__global__ void __launch_bounds__(SP_SCAN_T) sp_scan_kernel(SwPlanArgs P)
+{
+    __shared__ long long total[SP_LISTS];
+    __shared__ int32_t warp_sum[SP_LISTS][32];
+    sp_scan(P.counts, P.starts, false, warp_sum, total);
     if (threadIdx.x == 0) sp_lay_out(P, P.res, total);
 }
 
@@ -253,10 +284,10 @@ __global__ void sp_pack_kernel(SwPlanArgs P)
 
 // The same plan by one block, for at most SP_SMALL pairs: the four kernels' launches
 // and the trips through memory between them cost a small batch more than the work
-// (plan of one pair 51 -> 13 us, of 4,096 pairs 55 -> 20; a call of 4,096 pairs 423 ->
-// 401 us, of 8,192 pairs 561 and 558, of 16,384 pairs 909 -> 933).  A
+// (plan of one pair 51 -> 11 us; a call of 4,096 pairs 399 us either way, of 8,192 pairs
+// 558 us by one block and 541 by four kernels, of 16,384 pairs 933 and 886).  A
 // pair's place in its bucket is what its count's atomic returns.
-constexpr int SP_SMALL = 4096, SP_SMALL_T = 1024;
+constexpr int SP_SMALL = 4096, SP_SMALL_T = SP_SCAN_T;
 __global__ void __launch_bounds__(SP_SMALL_T) sp_small_kernel(SwPlanArgs P)
 {
     extern __shared__ int32_t sp_smem[];
@@ -266,7 +297,7 @@ __global__ void __launch_bounds__(SP_SMALL_T) sp_small_kernel(SwPlanArgs P)
     __shared__ int32_t warp_sum[SP_LISTS][32];
     __shared__ long long total[SP_LISTS];
     const int n = P.D.n, tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-    constexpr int PER = SP_SMALL / SP_SMALL_T, BPT = SP_NB / SP_SMALL_T;
+    constexpr int PER = SP_SMALL / SP_SMALL_T;
     for (int k = tid; k < SP_LISTS * SP_NB; k += SP_SMALL_T) cnt[k] = 0;
     if (tid < SP_RES) rec[tid] = 0;
     __syncthreads();
@@ -280,41 +311,7 @@ __global__ void __launch_bounds__(SP_SMALL_T) sp_small_kernel(SwPlanArgs P)
     }
     if (wid * 32 < n) sp_add_tally(T, rec, lane);
     __syncthreads();
-    int own[SP_LISTS], incl[SP_LISTS];
-#pragma unroll
-    for (int l = 0; l < SP_LISTS; ++l) {
-        own[l] = 0;
-        for (int k = 0; k < BPT; ++k) own[l] += cnt[l * SP_NB + tid * BPT + k];
-        incl[l] = own[l];
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int v = __shfl_up_sync(FULL, incl[l], o);
-            if (lane >= o) incl[l] += v;
-        }
-        if (lane == 31) warp_sum[l][wid] = incl[l];
-    }
-    __syncthreads();
-    if (wid < SP_LISTS) {
-        int v = warp_sum[wid][lane], s = v;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int u = __shfl_up_sync(FULL, s, o);
-            if (lane >= o) s += u;
-        }
-        warp_sum[wid][lane] = s - v;
-        if (lane == 31) total[wid] = s;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int l = 0; l < SP_LISTS; ++l) {
-        int acc = warp_sum[l][wid] + incl[l] - own[l];
-        for (int k = 0; k < l; ++k) acc += (int)total[k];
-        for (int k = 0; k < BPT; ++k) {
-            const int c = cnt[l * SP_NB + tid * BPT + k];
-            cnt[l * SP_NB + tid * BPT + k] = acc;
-            acc += c;
-        }
-    }
+    sp_scan(cnt, cnt, true, warp_sum, total);
     if (tid == 0) sp_lay_out(P, reinterpret_cast<long long*>(rec), total);
     __syncthreads();
 #pragma unroll
@@ -468,7 +465,7 @@ cudaError_t launch_sw_plan(SwPlanArgs P, int32_t* scratch, cudaStream_t st)
     sp_classify_kernel<<<blocks, 256, 0, st>>>(P);
     launch_end(K_SWPLAN, st);
     launch_begin(K_SWPLAN, st);
-    sp_scan_kernel<<<1, 32 * SP_LISTS, 0, st>>>(P);
+    sp_scan_kernel<<<1, SP_SCAN_T, 0, st>>>(P);
     launch_end(K_SWPLAN, st);
     launch_begin(K_SWPLAN, st);
     sp_scatter_kernel<<<blocks, 256, 0, st>>>(P);

@@ -847,10 +847,12 @@ static cudaError_t run_wfa_graph(Ctx* c, const WfaScratch& S, const PairDesc& D,
 {
     const std::vector<uint64_t> key = {c->dev_gen, (uint64_t)D.n, (uint64_t)(uintptr_t)D.seq, (uint64_t)smax,
                                        (uint64_t)trace | (uint64_t)lane_smax << 8 | (uint64_t)route << 16 |
-                                           (uint64_t)S.group << 24,
-                                       (uint64_t)(uintptr_t)score, (uint64_t)(uintptr_t)cig,
-                                       (uint64_t)(uintptr_t)D.a_off, (uint64_t)(uintptr_t)S.packed,
-                                       (uint64_t)(uintptr_t)err};
+                                           (uint64_t)S.group << 24 | (uint64_t)S.beside << 32,
+                                       (uint64_t)(uintptr_t)score, (uint64_t)(uintptr_t)len, (uint64_t)(uintptr_t)cig,
+                                       (uint64_t)(uintptr_t)D.a_off, (uint64_t)(uintptr_t)D.a_len,
+                                       (uint64_t)(uintptr_t)D.b_off, (uint64_t)(uintptr_t)D.b_len,
+                                       (uint64_t)(uintptr_t)D.out_off, (uint64_t)S.seq_bytes,
+                                       (uint64_t)(uintptr_t)S.packed, (uint64_t)(uintptr_t)err};
     return replay_graph(c->gexec, c->gkey, c->gseen, key, c->glaunches, st, [&]() {
         return enqueue_wfa(c, S, D, smax, trace, route, lane_smax, score, len, cig, err, st);
     });

@@ -1,0 +1,84 @@
+"""A CUDA graph is replayed only for the call it was captured for: every value
+the captured launches hold is in the key (on a runtime that records, no GPU)."""
+import numpy as np
+import pytest
+
+import fake_cuda
+from genoaligner_gb300 import api, cost_model, workloads
+
+
+@pytest.fixture(scope="module")
+def fake_path(tmp_path_factory):
+    return fake_cuda.build(tmp_path_factory.mktemp("fake"))
+
+
+@pytest.fixture
+def rt(fake_path, tmp_path):
+    with fake_cuda.library(fake_path, tmp_path) as r:
+        yield r
+
+
+def _batch(torch, ps):
+    b = api.DeviceBatchT(ps.a_buf, ps.a_off, ps.a_len, ps.b_buf, ps.b_off, ps.b_len, device="cpu")
+    out = (torch.zeros(b.n, dtype=torch.int32), torch.zeros(b.n, dtype=torch.int32),
+           torch.zeros(max(b.out_bytes, 1), dtype=torch.uint8))
+    return b, out
+
+
+def test_equal_learned_calls_replay_one_graph(rt):
+    torch = pytest.importorskip("torch")
+    assert cost_model.load_default()
+    b, out = _batch(torch, workloads.wfa_mixed(n=300, seed=1))
+    for call, want in enumerate(((0, 0), (1, 1), (0, 1), (0, 1))):
+        rt.clear()
+        api.wfa_device(b, 64, True, *out, learned=True)
+        assert (rt.count("capture"), rt.count("replay")) == want, call
+
+
+@pytest.mark.parametrize("changed", ["a_off", "a_len", "b_off", "b_len", "out_off", "out_score", "out_len", "out_cigar",
+                                     "seq", "seq_bytes"])
+def test_learned_call_with_another_buffer_is_no_replay(rt, changed):
+    torch = pytest.importorskip("torch")
+    assert cost_model.load_default()
+    b, out = _batch(torch, workloads.wfa_mixed(n=300, seed=1))
+    for _ in range(3):
+        api.wfa_device(b, 64, True, *out, learned=True)
+    out = list(out)
+    keep = []
+    if changed.startswith("out_") and changed != "out_off":
+        k = ("out_score", "out_len", "out_cigar").index(changed)
+        keep.append(out[k])
+        out[k] = out[k].clone()
+    elif changed == "seq_bytes":
+        b.c.seq_bytes -= 32                       # (every sequence still ends 32 bytes before the end)
+    else:
+        t = getattr(b, changed)
+        keep.append(t)
+        t = t.clone()
+        keep.append(t)
+        setattr(b.c, changed, t.data_ptr())
+    rt.clear()
+    api.wfa_device(b, 64, True, *out, learned=True)
+    assert rt.count("replay") == 0 and rt.count("launch") > 0
+
+
+def test_host_batches_whose_arenas_share_a_256_byte_step_are_no_replay(rt):
+    """Score-only host batches of equal n, arenas 128 bytes apart: each carved
+    buffer starts where the other batch's does."""
+    assert cost_model.load_default()
+    rng = np.random.default_rng(3)
+
+    def call(length):
+        a = workloads.random_bases(rng, 32 * 40)
+        off = np.arange(40, dtype=np.int64) * 32
+        lens = np.full(40, 32, np.int32)
+        lens[0] = length                                    # (the second sequence's bytes again)
+        got = api.align_batch_packed(a, off, lens, a, off, lens, smax=31, with_cigar=False, learned=True)
+        assert got.status == api.Status.ok, got.error
+
+    for _ in range(3):
+        call(32)
+    for length in (64, 96, 128, 160, 192, 224, 256):
+        rt.clear()
+        call(length)
+        assert rt.count("replay") == 0, length

@@ -1224,14 +1224,21 @@ static int sw_coop_warps(int l, bool trace, const ga_tune& T)
 }
 
 // The plan, built on the device (sw_plan.cu) into `dwork`, its record into dres.
-// launched: when set, the launches' block sizes are its (and the 16-bit launch has
-// the whole-block phase only if it counts such items); otherwise the device's choice.
+// launched: when set, the launches are those of launch_plan for it -- the block sizes are
+// its, the 16-bit launch has the whole-block phase only if it counts such items, and
+// pairs that no launch of its takes set ERR_SCRATCH at err; otherwise the device's choice.
 static cudaError_t enqueue_plan_sw(const PairDesc& D, const ga_sw_scoring& sc, bool trace, int64_t cell_limit,
                                    int32_t too_large_score, int32_t* out_score, int32_t* dwork, int32_t* scratch,
                                    long long* dres, const ga_tune& T, cudaStream_t st, const uint8_t* try16 = nullptr,
-                                   const SwPlan* launched = nullptr)
+                                   const SwPlan* launched = nullptr, int32_t* err = nullptr)
 {
     SwPlanArgs A;
+    if (launched) {
+        A.launched = 0;
+        for (int l = 0; l < SP_LISTS; ++l) A.launched |= (launched->ints[l] > 0) << l;
+        A.handover = launched->n_opt > 0;
+        A.err = err;
+    }
     A.coop_limit = sw_coop_limit(T);
     for (int l = 0; l < SP_LISTS; ++l) {
         A.coop_warps[l] = l == SP_L16 && launched && launched->ncoop[l] <= 0 ? 0 : sw_coop_warps(l, trace, T);
@@ -1701,7 +1708,7 @@ static int32_t sw_batch_range(const ga_sw_request* reqs, int32_t n, int64_t base
         if (e == cudaSuccess && route) e = launch_sw_route(D, s0.match, s0.gap_open, dfeat, dy, dtry, st);
         if (e == cudaSuccess)
             e = enqueue_plan_sw(D, s0, trace, trace ? cell_limit : -1, -1, dsc, dwork, dscr, dres, T, st, dtry,
-                                &P);
+                                &P, der);
         if (e == cudaSuccess)
             e = launch_plan(P, S, D, s0, trace, T, dwork, dsc, dpos, dln, dcg, ddirs, dedge, dctr, der, st, dscr, dres);
         if (e == cudaSuccess && trace)
@@ -2276,9 +2283,10 @@ int32_t ga_sw_device_ex(const ga_device_batch* b, ga_sw_scoring sc, int32_t trac
     // A synchronous traceback call with a cell limit replays the CUDA graph of
     // its launch shape: the first call of a shape reads the plan back to size
     // the per-warp memory and captures the launches in plan mode (sizes read
-    // on the device); a replay whose plan needs more memory than that (the
-    // pairs behind the same pointers grew) is flagged by the kernels
-    // (ERR_SCRATCH) and runs again through the read-back path.
+    // on the device); a replay whose plan needs more memory than that, or a
+    // launch that the graph lacks (the pairs behind the same pointers grew, or
+    // moved to a list that was empty), is flagged by the kernels and the
+    // planner (ERR_SCRATCH) and runs again through the read-back path.
     const bool graph = !stream && trace && cell_limit >= 0 && !profiling_on();
     std::vector<uint64_t> key;
     if (graph) {
@@ -2356,7 +2364,7 @@ int32_t ga_sw_device_ex(const ga_device_batch* b, ga_sw_scoring sc, int32_t trac
             if (x == cudaSuccess && route) x = launch_sw_route(D, sc.match, sc.gap_open, dfeat, dy, dtry, st);
             if (x == cudaSuccess)
                 x = enqueue_plan_sw(D, sc, true, cell_limit, -2, out_score, dwork, dscr, dres, T, st, dtry,
-                                    &P);
+                                    &P, dctr + 32);
             if (x == cudaSuccess)
                 x = launch_plan(P, S, D, sc, true, T, dwork, out_score, out_pos, out_len, out_cigar, ddirs, dedge, dctr,
                                 dctr + 32, st, dscr, dres, c);

@@ -268,6 +268,13 @@ struct SwPlanArgs {
     int32_t coop_block[SP_LISTS];     // ... and the warps of such a block, 0: chosen here (sw_coop_block)
     int32_t sms;
     int32_t score_only;          // 1: lists of the score-only kernels (sw16so, sw_kernel)
+    // The launches that follow were chosen before this plan: the lists they take (a bit
+    // each), and whether pairs handed over by the 16-bit kernel have one to go to (without
+    // it none is taken on the optimistic rule).  Pairs that need another launch set
+    // ERR_SCRATCH at err.
+    int32_t launched = (1 << SP_LISTS) - 1;
+    int32_t handover = 1;
+    int32_t* err = nullptr;
     int32_t* out_score;
     int32_t* work;               // flattened work lists (2n + 8 ints)
     long long* res;              // the record above

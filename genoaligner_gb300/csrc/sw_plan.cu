@@ -49,8 +49,8 @@ __device__ __forceinline__ int sp_classify(const SwPlanArgs& P, int p, SpTally& 
     const bool opt = P.try16 ? (P.try16[p] != 0 && m > 0 && nn > 0 &&
                                 sw16_scheme_ok(P.match, P.mismatch, P.gap_open, P.gap_extend))
                              : sw16_eligible_opt(m, nn, P.match, P.mismatch, P.gap_open, P.gap_extend, P.opt16_pct);
-    const bool u16 = strict || (!P.score_only && pure && opt);
-    if (u16 && !strict) {           // may be handed to the 32-bit long-shape kernel
+    const bool tried = !P.score_only && pure && opt && !strict, u16 = strict || (tried && P.handover);
+    if (tried) {                    // may be handed to the 32-bit long-shape kernel
         ++T.nopt;
         T.diropt = max(T.diropt, (unsigned long long)sw32ck_dir_words(m, nn, 0));
     }
@@ -128,12 +128,15 @@ __global__ void sp_classify_kernel(SwPlanArgs P)
 }
 
 // Lists' lengths in the flattened work array and their offsets there (16-bit lists
-// hold two entries per work item), and the warps of their whole-block launches.
+// hold two entries per work item), the warps of their whole-block launches, and
+// whether the launches that follow serve these lists.
 __device__ __forceinline__ void sp_lay_out(const SwPlanArgs& P, long long* res, const long long* total)
 {
     long long base = 0;
+    bool served = res[SP_NOPT] == 0 || P.handover;
     for (int l = 0; l < SP_LISTS; ++l) {
         const long long ints = l == SP_L16 ? 2 * ((total[l] + 1) / 2) : total[l];
+        served = served && (total[l] == 0 || (P.launched >> l & 1));
         res[SP_COUNT + l] = total[l];
         res[SP_INTS + l] = ints;
         res[SP_BASE + l] = base;
@@ -142,6 +145,7 @@ __device__ __forceinline__ void sp_lay_out(const SwPlanArgs& P, long long* res, 
                                             : sw_coop_block(res[SP_LARGEST + l], (int)res[SP_COLS + l],
                                                             l == SP_L16 ? res[SP_CELLS + l] / 2 : res[SP_CELLS + l], P.sms);
     }
+    if (!served && P.err) atomicOr(P.err, ERR_SCRATCH);
 }
 
 // Work items first, first + step, ... of list l in launch order; their largest

@@ -800,24 +800,35 @@ static cudaError_t enqueue_wfa(Ctx* c, const WfaScratch& S, PairDesc D, int smax
     return launch_wfa_block(B, S.blocks, K_WFA_ROUTED, st);
 }
 
+// Whether a capture can begin on the stream: not on the legacy one, nor on one
+// that the caller is capturing.
+static bool can_capture(cudaStream_t st)
+{
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    if (st == cudaStreamLegacy) return false;
+    if (cudaStreamIsCapturing(st, &status) != cudaSuccess) { cudaGetLastError(); return false; }
+    return status == cudaStreamCaptureStatusNone;
+}
+
 // Replays `exec` when `key` (everything the enqueued launches bake in) is the
 // one it was captured for.  Another key's launches are enqueued as they are the
-// first time, and captured when the same key comes again at once (`seen`): batches
-// whose sizes differ from call to call, which no graph serves twice, do not pay for
-// one (SW batches of 1 to 3,558 pairs in turn: 40 to 70 us a call).  `launches` keeps
+// first time, and captured when the same key comes again at once (`seen`: the call
+// before's): batches whose sizes differ from call to call, which no graph serves twice,
+// do not pay for one (SW batches of 1 to 3,558 pairs in turn: 40 to 70 us a call).  A
+// stream on which no capture can begin takes the key of the call before alone, by its
+// graph or, not yet captured, as it is.  `launches` keeps
 // the number of library kernels the graph holds (counted once per replay).
 static cudaError_t replay_graph(cudaGraphExec_t& exec, std::vector<uint64_t>& have, std::vector<uint64_t>& seen,
                                 const std::vector<uint64_t>& key, int& launches, cudaStream_t st,
                                 const std::function<cudaError_t()>& enqueue)
 {
+    const bool again = seen == key, can = can_capture(st);
+    if (!again && !can) return cudaErrorStreamCaptureUnsupported;
+    seen = key;
     if (!exec || have != key) {
-        if (seen != key) {
-            seen = key;
-            return enqueue();
-        }
+        if (!again || !can) return enqueue();
         // one capture at a time in the process (the ranges of a ranged call
-        // capture their first calls from their own threads); a capture is
-        // made once per launch shape, so this costs nothing on replays
+        // capture from their own threads)
         static std::mutex capture_mu;
         std::lock_guard<std::mutex> lk(capture_mu);
         if (exec) { cudaGraphExecDestroy(exec); exec = nullptr; }
@@ -2301,6 +2312,7 @@ int32_t ga_sw_device_ex(const ga_device_batch* b, ga_sw_scoring sc, int32_t trac
         if (c->swexec && c->swkey.size() == key.size() + 2 && std::equal(key.begin(), key.end(), c->swkey.begin()) &&
             c->swkey[key.size()] == c->dev_gen) {
             int32_t* derr = reinterpret_cast<int32_t*>(c->swkey[key.size() + 1]);
+            c->swseen = c->swkey;
             note_graph_launches(c->swlaunches);
             if (cudaGraphLaunch(c->swexec, st) != cudaSuccess ||
                 cudaMemcpyAsync(herr, derr, sizeof(int32_t), cudaMemcpyDeviceToHost, st) != cudaSuccess ||

@@ -1,5 +1,7 @@
-"""A CUDA graph is replayed only for the call it was captured for: every value
-the captured launches hold is in the key (on a runtime that records, no GPU)."""
+"""Which calls run as CUDA graphs (on a runtime that records, no GPU).  A graph is
+replayed only for the call it was captured for: every value the captured launches
+hold is in the key.  A call is captured when it repeats the one before; a stream
+that cannot be captured takes what that one did, and nothing else."""
 import numpy as np
 import pytest
 
@@ -82,3 +84,58 @@ def test_host_batches_whose_arenas_share_a_256_byte_step_are_no_replay(rt):
         rt.clear()
         call(length)
         assert rt.count("replay") == 0, length
+
+
+def test_a_shape_between_two_others_is_not_captured(rt):
+    torch = pytest.importorskip("torch")
+    assert cost_model.load_default()
+    a, b = (_batch(torch, workloads.wfa_mixed(n=n, seed=1)) for n in (300, 200))
+    for x in (a, a, b, a, b, a, b):
+        api.wfa_device(x[0], 64, True, *x[1], learned=True)
+    assert rt.count("capture") == 1                     # a's two in a row
+
+
+LEGACY = 1                                              # cudaStreamLegacy
+
+
+@pytest.mark.parametrize("legacy", [True, False])
+def test_streams_that_cannot_be_captured(rt, legacy):
+    torch = pytest.importorskip("torch")
+    assert cost_model.load_default()
+    b, out = _batch(torch, workloads.wfa_mixed(n=300, seed=1))
+    other, other_out = _batch(torch, workloads.wfa_mixed(n=200, seed=2))
+    s = LEGACY if legacy else rt.stream()
+
+    def refused(batch, outs):
+        rt.clear()
+        if not legacy:
+            rt.capturing(s, True)
+        try:
+            api.wfa_device(batch, 64, True, *outs, stream=s, learned=True)
+            return False
+        except RuntimeError:
+            assert not rt.log()                         # nothing was enqueued
+            return True
+        finally:
+            if not legacy:
+                rt.capturing(s, False)
+
+    assert refused(b, out) and refused(b, out)          # a new shape: every time
+    api.wfa_device(b, 64, True, *out, learned=True)
+    assert not refused(b, out)                          # the shape of the call before
+    assert refused(other, other_out)
+    for _ in range(2):
+        api.wfa_device(b, 64, True, *out, learned=True)
+    assert not refused(b, out) and rt.count("replay") == 1
+    api.wfa_device(other, 64, True, *other_out, learned=True)
+    assert refused(b, out) and not refused(other, other_out)
+
+
+def test_plain_calls_take_any_stream(rt):
+    torch = pytest.importorskip("torch")
+    b, out = _batch(torch, workloads.wfa_mixed(n=300, seed=1))
+    s = rt.stream()
+    rt.capturing(s, True)
+    for stream in (s, LEGACY):
+        api.wfa_device(b, 64, True, *out, stream=stream)
+    rt.capturing(s, False)

@@ -96,7 +96,9 @@ template <typename Run>
 static int32_t time_candidate(const ga_tune& cand, int reps, const Run& run, double* ms, const char** err)
 {
     t_candidate = &cand;
-    int32_t rc = run(err);                                      // untimed: allocations, graph capture
+    // untimed: the first call allocates, the second, which repeats it, is captured as a graph
+    int32_t rc = run(err);
+    if (rc == GA_OK) rc = run(err);
     double total = 0.0;
     for (int r = 0; r < reps && rc == GA_OK; ++r) {
         const auto t0 = std::chrono::steady_clock::now();

@@ -429,8 +429,8 @@ int32_t ga_tune_set(const ga_tune* t);
 
 /* Time candidate settings on an SW traceback batch (arguments and outputs as
  * ga_sw_device with trace = 1) and keep the fastest for the current device.
- * Each candidate runs once untimed, then `reps` timed calls (reps <= 0: 2) on
- * the library's own stream.  Coordinate search: sw_pack16, then sw_window
+ * Each candidate runs twice untimed (the second call may build a CUDA graph),
+ * then `reps` timed calls (reps <= 0: 2) on the library's own stream.  Coordinate search: sw_pack16, then sw_window
  * (when pack16 is chosen), then sw_long_log2 (when the batch has pairs above
  * 2^20 cells), then sw_coop_log2 (when it has pairs above 2^24 cells), then
  * sw_opt16_pct (when it has pure pairs whose all-match score passes 16 bits).  chosen (may be NULL) gets the setting kept; trials[0 ..

@@ -1,12 +1,14 @@
 """The library linked to a CUDA runtime that only records (fake_cudart.cpp), for
-tests of the host engine without a GPU: `with fake_cuda.library(tmp) as rt` makes
-genoaligner_gb300.api call a fresh copy of it, with host tensors for device
-memory, and rt.log() gives the lines that runtime wrote."""
+tests of the host engine without a GPU: under the `rt` fixture genoaligner_gb300.api
+calls a fresh copy of it, with host tensors for device memory, and rt.log() gives
+the lines that runtime wrote."""
 import contextlib
 import ctypes
 import os
 import shutil
 import subprocess
+
+import pytest
 
 from genoaligner_gb300 import _build, api
 
@@ -64,3 +66,14 @@ def library(path, folder):
         yield Runtime(api.load())
     finally:
         api._lib, _build.build = kept, kept_build
+
+
+@pytest.fixture(scope="module")
+def fake_path(tmp_path_factory):
+    return build(tmp_path_factory.mktemp("fake"))
+
+
+@pytest.fixture
+def rt(fake_path, tmp_path):
+    with library(fake_path, tmp_path) as r:
+        yield r

@@ -5,19 +5,8 @@ that cannot be captured takes what that one did, and nothing else."""
 import numpy as np
 import pytest
 
-import fake_cuda
+from fake_cuda import fake_path, rt  # noqa: F401
 from genoaligner_gb300 import api, cost_model, workloads
-
-
-@pytest.fixture(scope="module")
-def fake_path(tmp_path_factory):
-    return fake_cuda.build(tmp_path_factory.mktemp("fake"))
-
-
-@pytest.fixture
-def rt(fake_path, tmp_path):
-    with fake_cuda.library(fake_path, tmp_path) as r:
-        yield r
 
 
 def _batch(torch, ps):

@@ -828,6 +828,8 @@ static cudaError_t run_backward(const __nv_bfloat16* w, const float* feat, const
     cudaMemsetAsync(grad, 0, GRAD_COPIES * GRAD_STRIDE * sizeof(float), st);
     launch_begin(K_MLP, st);
     mlp_backward_kernel<<<mlp_blocks(n), MLP_T, sizeof(MlpSmem), st>>>(w, feat, target, n, 1.0f / (float)n, grad);
+    launch_end(K_MLP, st);
+    launch_begin(K_MLP, st);
     fold_grad_kernel<<<(NPARAM + 256) / 256, 256, 0, st>>>(grad);
     launch_end(K_MLP, st);
     return cudaGetLastError();
@@ -930,7 +932,9 @@ int32_t ga_cost_model_set(const float* params, int32_t n)
         cudaGetLastError();
         return GA_DEVICE_ERROR;
     }
+    launch_begin(K_MLP, nullptr);
     to_bf16_kernel<<<64, 256>>>(M->master, M->w, NPARAM);
+    launch_end(K_MLP, nullptr);
     if (cudaDeviceSynchronize() != cudaSuccess) { cudaGetLastError(); return GA_DEVICE_ERROR; }
     M->step = 0;
     M->ready = true;

@@ -162,7 +162,7 @@ cudaError_t launch_sketch(const PairDesc& D, float* feat, int32_t* lb, cudaStrea
 cudaError_t launch_mlp_forward(const float* feat, int n, float* y, cudaStream_t st);
 bool cost_model_loaded();
 bool sw_model_loaded();
-void prepare_mlp();
+cudaError_t prepare_mlp();
 // SW variant routing by the SW model: try16[p] = 1 for pairs the 16-bit
 // kernel should try (feat [n][66] and y [n][2] are scratch).
 cudaError_t launch_sw_route(const PairDesc& D, int match, int go, float* feat, float* y, uint8_t* try16,

@@ -17,6 +17,7 @@
 // computed in fp32 (fp32 master copy for Adam).  Outputs: log2(d + 1) and
 // log2(wavefront cells + 1) with wavefront cells = (d + 1)^2.  It is a tiny
 // GEMM (25k multiply-adds per pair); training runs it as register-tiled fp32 FMA.
+#include <atomic>
 #include <mutex>
 #include <vector>
 
@@ -31,7 +32,7 @@ constexpr int NF = 66, NH1 = 128, NH2 = 128, NO = 2;
 constexpr int OFF_W1 = 0, OFF_B1 = OFF_W1 + NH1 * NF, OFF_W2 = OFF_B1 + NH1, OFF_B2 = OFF_W2 + NH2 * NH1,
               OFF_W3 = OFF_B2 + NH2, OFF_B3 = OFF_W3 + NO * NH2, NPARAM = OFF_B3 + NO;
 
-void prepare_mlp();
+cudaError_t prepare_mlp();
 const __nv_bfloat16* cost_model_weights();
 
 // ------------------------------------------------------------------ sketch --
@@ -727,6 +728,7 @@ cudaError_t launch_route_model(const PairDesc& D, int smax, int lane_smax, bool 
     const __nv_bfloat16* w = cost_model_weights();
     if (model && !w) return cudaErrorNotReady;
     if (D.n <= 0) return cudaSuccess;
+    if (const cudaError_t e = prepare_mlp()) return e;
     // Lanes to a side: as many as keep every tile a warp of its own.  One lane a side
     // leaves the 2,000 long pairs' counting to 125 warps (2,000 of 2-10 kb: pass 256 us,
     // with 16 lanes 47); the rows a tile then lacks cost nothing that waits.
@@ -746,7 +748,7 @@ cudaError_t launch_route_model(const PairDesc& D, int smax, int lane_smax, bool 
 static cudaError_t run_forward_tc(const __nv_bfloat16* w, const float* feat, int n, float* y, cudaStream_t st)
 {
     if (n <= 0) return cudaSuccess;
-    prepare_mlp();
+    if (const cudaError_t e = prepare_mlp()) return e;
     int blocks = (n + 127) / 128;
     blocks = std::min(blocks, device_sms() * 2);
     launch_begin(K_MLP, st);
@@ -792,19 +794,30 @@ static Model* model_for(int slot, bool create)
     return M.master ? &M : nullptr;
 }
 
-// Kernel attributes are set outside any stream capture (prepare_mlp is called
-// while planning a batch).
-void prepare_mlp()
+// The shared-memory limits of this file's kernels, per device and outside any stream
+// capture (prepare_mlp is called while planning a batch).
+cudaError_t prepare_mlp()
 {
-    static std::once_flag once;
-    std::call_once(once, [] {
-        cudaFuncSetAttribute(mlp_forward_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(MlpSmem));
-        cudaFuncSetAttribute(mlp_backward_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(MlpSmem));
-        cudaFuncSetAttribute(mlp_forward_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(TcSmem));
-        for (auto kernel : {route_model_kernel<true, true>, route_model_kernel<true, false>,
-                            route_model_kernel<false, true>, route_model_kernel<false, false>})
-            cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)route_model_smem());
-    });
+    constexpr int MAX_DEV = 64;
+    static std::mutex mu;
+    static std::atomic<bool> ready[MAX_DEV];
+    int dev = 0;
+    const cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    const bool known = dev >= 0 && dev < MAX_DEV;
+    if (known && ready[dev].load(std::memory_order_acquire)) return cudaSuccess;
+    std::lock_guard<std::mutex> lk(mu);
+    auto limit = [](auto kernel, size_t bytes) {
+        return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    };
+    cudaError_t r = limit(mlp_forward_kernel, sizeof(MlpSmem));
+    if (r == cudaSuccess) r = limit(mlp_backward_kernel, sizeof(MlpSmem));
+    if (r == cudaSuccess) r = limit(mlp_forward_tc_kernel, sizeof(TcSmem));
+    for (auto kernel : {route_model_kernel<true, true>, route_model_kernel<true, false>,
+                        route_model_kernel<false, true>, route_model_kernel<false, false>})
+        if (r == cudaSuccess) r = limit(kernel, route_model_smem());
+    if (known && r == cudaSuccess) ready[dev].store(true, std::memory_order_release);
+    return r;
 }
 
 // A tile a block, no more blocks than multiprocessors (a block's shared memory fills one).
@@ -813,7 +826,7 @@ static int mlp_blocks(int n) { return std::min((int)(((int64_t)n + TILE - 1) / T
 static cudaError_t run_forward(const __nv_bfloat16* w, const float* feat, int n, float* y, cudaStream_t st)
 {
     if (n <= 0) return cudaSuccess;
-    prepare_mlp();
+    if (const cudaError_t e = prepare_mlp()) return e;
     launch_begin(K_MLP, st);
     mlp_forward_kernel<<<mlp_blocks(n), MLP_T, sizeof(MlpSmem), st>>>(w, feat, n, y);
     launch_end(K_MLP, st);
@@ -824,7 +837,7 @@ static cudaError_t run_forward(const __nv_bfloat16* w, const float* feat, int n,
 static cudaError_t run_backward(const __nv_bfloat16* w, const float* feat, const float* target, int n, float* grad,
                                 cudaStream_t st)
 {
-    prepare_mlp();
+    if (const cudaError_t e = prepare_mlp()) return e;
     cudaMemsetAsync(grad, 0, GRAD_COPIES * GRAD_STRIDE * sizeof(float), st);
     launch_begin(K_MLP, st);
     mlp_backward_kernel<<<mlp_blocks(n), MLP_T, sizeof(MlpSmem), st>>>(w, feat, target, n, 1.0f / (float)n, grad);

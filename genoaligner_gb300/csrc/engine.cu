@@ -285,6 +285,7 @@ struct Ctx {
     cudaStream_t stream = nullptr;
     cudaEvent_t done = nullptr;     // last work enqueued on a caller's stream
     cudaStream_t side = nullptr;    // launches that run beside the stream's (launch_plan, enqueue_wfa), and its events
+    int side_prio = 0;
     cudaEvent_t forked = nullptr, joined = nullptr;
     bool pending = false;
     char* dev = nullptr;
@@ -380,15 +381,34 @@ static Ctx* acquire_ctx(const char** err, int tag = -1)
     return c;
 }
 
-// The context's second stream and its events, made on first use.
-static bool ensure_side(Ctx* c)
+// Priority of the stream a call runs on: the caller's or the context's.
+static int call_priority(const Ctx* c, cudaStream_t st)
 {
-    if ((!c->side && cudaStreamCreateWithPriority(&c->side, cudaStreamNonBlocking, c->prio) != cudaSuccess) ||
+    int prio = c->prio;
+    if (st != c->stream && cudaStreamGetPriority(st, &prio) != cudaSuccess) {
+        cudaGetLastError();
+        prio = c->prio;
+    }
+    return prio;
+}
+
+// The context's second stream, at the priority of the call's stream `st`, and its
+// events, made on first use.  (A stream of another priority gives way: what it still
+// runs is the calls' before, which they wait for.)
+static bool ensure_side(Ctx* c, cudaStream_t st)
+{
+    const int prio = call_priority(c, st);
+    if (c->side && c->side_prio != prio) {
+        cudaStreamDestroy(c->side);
+        c->side = nullptr;
+    }
+    if ((!c->side && cudaStreamCreateWithPriority(&c->side, cudaStreamNonBlocking, prio) != cudaSuccess) ||
         (!c->forked && cudaEventCreateWithFlags(&c->forked, cudaEventDisableTiming) != cudaSuccess) ||
         (!c->joined && cudaEventCreateWithFlags(&c->joined, cudaEventDisableTiming) != cudaSuccess)) {
         cudaGetLastError();
         return false;
     }
+    c->side_prio = prio;
     return true;
 }
 
@@ -863,7 +883,8 @@ static cudaError_t run_wfa_graph(Ctx* c, const WfaScratch& S, const PairDesc& D,
                                        (uint64_t)(uintptr_t)D.a_off, (uint64_t)(uintptr_t)D.a_len,
                                        (uint64_t)(uintptr_t)D.b_off, (uint64_t)(uintptr_t)D.b_len,
                                        (uint64_t)(uintptr_t)D.out_off, (uint64_t)S.seq_bytes,
-                                       (uint64_t)(uintptr_t)S.packed, (uint64_t)(uintptr_t)err};
+                                       (uint64_t)(uintptr_t)S.packed, (uint64_t)(uintptr_t)err,
+                                       (uint64_t)(int64_t)call_priority(c, st)};
     return replay_graph(c->gexec, c->gkey, c->gseen, key, c->glaunches, st, [&]() {
         return enqueue_wfa(c, S, D, smax, trace, route, lane_smax, score, len, cig, err, st);
     });
@@ -1112,7 +1133,7 @@ int32_t wfa_batch(const ga_align_request* reqs, int32_t n, int32_t max_smax, int
             return GA_DEVICE_ERROR;
         }
         cudaError_t le;
-        S.beside = S.beside && ensure_side(c);
+        S.beside = S.beside && ensure_side(c, c->stream);
         if (fail_here(3)) le = cudaErrorLaunchFailure;
         else if (learned && !profiling_on())
             le = run_wfa_graph(c, S, D, smax, trace, route, lane_smax, dsc, dln, dcg, der, c->stream);
@@ -1743,6 +1764,7 @@ static int32_t sw_batch_range(const ga_sw_request* reqs, int32_t n, int64_t base
                 (uint64_t)P.ints[0], (uint64_t)P.ints[1], (uint64_t)P.ints[2], (uint64_t)P.dir[0],
                 (uint64_t)P.dir[1], (uint64_t)P.dir[2], (uint64_t)P.edge_slot,
                 (uint64_t)P.w[0] | (uint64_t)P.w[1] << 8 | (uint64_t)P.w[2] << 16 | (uint64_t)(P.ncoop[0] > 0) << 24,
+                (uint64_t)(int64_t)c->prio,
                 (uint64_t)P.n_opt, (uint64_t)P.dir_opt, (uint64_t)S.dir_words, (uint64_t)S.max_slots,
                 (uint64_t)S.s[0] | (uint64_t)S.s[1] << 32, (uint64_t)S.s[2] | (uint64_t)S.s_esc << 32};
             le = replay_graph(c->swexec, c->swkey, c->swseen, key, c->swlaunches, c->stream, enqueue);
@@ -2167,7 +2189,7 @@ int32_t ga_wfa_device_ex(const ga_device_batch* b, int32_t smax, int32_t trace, 
     cudaError_t le;
     {
         const int lane_smax = tuned.wfa_lane_smax;
-        S.beside = S.beside && ensure_side(c);
+        S.beside = S.beside && ensure_side(c, st);
         if (learned && !profiling_on())
             le = run_wfa_graph(c, S, D, smax, trace != 0, route, lane_smax, out_score, out_len, out_cigar, derr, st);
         else le = enqueue_wfa(c, S, D, smax, trace != 0, route, lane_smax, out_score, out_len, out_cigar, derr, st);
@@ -2301,7 +2323,7 @@ int32_t ga_sw_device_ex(const ga_device_batch* b, ga_sw_scoring sc, int32_t trac
     const bool graph = !stream && trace && cell_limit >= 0 && !profiling_on();
     std::vector<uint64_t> key;
     if (graph) {
-        key = {0x5357445645ull, (uint64_t)n, (uint64_t)(uintptr_t)b->seq, (uint64_t)b->seq_bytes,
+        key = {0x5357445645ull, (uint64_t)(int64_t)c->prio, (uint64_t)n, (uint64_t)(uintptr_t)b->seq, (uint64_t)b->seq_bytes,
                (uint64_t)(uintptr_t)b->a_off, (uint64_t)(uintptr_t)b->a_len, (uint64_t)(uintptr_t)b->b_off,
                (uint64_t)(uintptr_t)b->b_len, (uint64_t)(uintptr_t)b->out_off, (uint64_t)(uintptr_t)out_score,
                (uint64_t)(uintptr_t)out_pos, (uint64_t)(uintptr_t)out_len, (uint64_t)(uintptr_t)out_cigar,
@@ -2361,7 +2383,7 @@ int32_t ga_sw_device_ex(const ga_device_batch* b, ga_sw_scoring sc, int32_t trac
     // little more, so it is sized again, with room to spare.
     for (int attempt = 0;; ++attempt) {
         if (!plan()) return fail(E_LAUNCH);
-        P.fork = P.fork && ensure_side(c);
+        P.fork = P.fork && ensure_side(c, st);
         S = size_sw(P, trace != 0, T, c->sm_count, sw_dir_budget(c, 1));
         const size_t need = run_layout(nullptr, &dctr, &dedge, &ddirs);
         if (need <= c->dev_cap) break;

@@ -114,12 +114,15 @@ cudaError_t launch_wfa_block(const WfaBlockArgs& B, int blocks, int kernel_id, c
 // Words that a batch's first kernel sets for the later ones: counters, records and
 // output defaults, for which a memset each would be a launch each.
 struct Fills {
-    int32_t* p[8];
-    int64_t n[8];
-    int32_t v[8];
+    static constexpr int MAX = 8;
+    int32_t* p[MAX];
+    int64_t n[MAX];
+    int32_t v[MAX];
     int32_t count = 0;
+    bool over = false;           // more than MAX were added: launch_pack refuses them
     void add(void* ptr, int64_t words, int32_t value)
     {
+        if (count == MAX) { over = true; return; }
         p[count] = static_cast<int32_t*>(ptr);
         n[count] = words;
         v[count++] = value;

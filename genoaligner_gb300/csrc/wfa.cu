@@ -211,6 +211,7 @@ __global__ void __launch_bounds__(128) wfa_kernel(WfaArgs A)
 cudaError_t launch_pack(const PairDesc& D, int64_t seq_bytes, uint64_t* packed, uint8_t* pure, cudaStream_t st,
                         const Fills& fills)
 {
+    if (fills.over) return cudaErrorInvalidValue;
     if (D.n <= 0) return cudaSuccess;
     int blocks = (2 * D.n + 255) / 256;
     blocks = std::min(blocks, device_sms() * 32);

@@ -358,7 +358,7 @@ __global__ void sw_validate_kernel(PairDesc D, int match, int mismatch, int go, 
     const int nw = (gridDim.x * blockDim.x) >> 5;
     for (int p = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; p < D.n; p += nw) {
         const int s = score[p], L = len[p];
-        if (L <= 0) {
+        if (s <= 0 || L <= 0) {                        // no CIGAR: len and pos may hold anything
             if (lane == 0) flags[p] = 0;
             continue;
         }
@@ -419,7 +419,7 @@ __global__ void sw_validate_kernel(PairDesc D, int match, int mismatch, int go, 
         bad |= chk && (ct == cp) != chk_m;
         total = __reduce_add_sync(FULL, total);
         const bool ok = !__any_sync(FULL, bad) && i0 == ei + 1 && j0 == ej + 1;
-        if (lane == 0) flags[p] = s <= 0 ? 0 : (uint8_t)((ok && total == s ? 1 : 0) | (ok ? 2 : 0));
+        if (lane == 0) flags[p] = (uint8_t)((ok && total == s ? 1 : 0) | (ok ? 2 : 0));
     }
 }
 

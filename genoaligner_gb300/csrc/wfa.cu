@@ -269,7 +269,7 @@ __global__ void wfa_validate_kernel(PairDesc D, const int32_t* __restrict__ scor
     const int nw = (gridDim.x * blockDim.x) >> 5;
     for (int p = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; p < D.n; p += nw) {
         const int s = score[p], L = len[p];
-        if (L <= 0) {
+        if (s < 0 || L <= 0) {                         // no CIGAR: len may hold anything
             if (lane == 0) flags[p] = 0;
             continue;
         }
@@ -318,7 +318,7 @@ __global__ void wfa_validate_kernel(PairDesc D, const int32_t* __restrict__ scor
         bad |= chk && (cp == ct) != chk_m;
         bad = __any_sync(FULL, bad);
         cost = __reduce_add_sync(FULL, cost);
-        if (lane == 0) flags[p] = s < 0 ? 0 : (uint8_t)((cost == s ? 1 : 0) | (!bad && pi0 == m && ti0 == n ? 2 : 0));
+        if (lane == 0) flags[p] = (uint8_t)((cost == s ? 1 : 0) | (!bad && pi0 == m && ti0 == n ? 2 : 0));
     }
 }
 

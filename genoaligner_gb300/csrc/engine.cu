@@ -723,7 +723,7 @@ static void carve_wfa(Carve& k, WfaScratch& S, int n, int64_t arena, bool trace,
     S.stack = trace ? k.take<int32_t>((size_t)(S.beside ? warp_words + block_words : std::max(warp_words, block_words)))
                     : nullptr;
     S.block_stack = trace && S.beside ? S.stack + warp_words : S.stack;
-    S.blk = k.take<int32_t>(S.blocks > 0 ? n : 0);
+    S.blk = S.blocks > 0 ? k.take<int32_t>(n) : nullptr;
     if (learned) {
         S.item = k.take<int32_t>(n);
         S.lb = k.take<int32_t>(n);

@@ -664,6 +664,10 @@ struct WfaScratch {
     int cap = 0;                     // edits the warp kernels search; the pairs left below smax go to the block kernel
     int blocks = 0;                  // blocks of the block kernel (0: not launched)
     int32_t* blk = nullptr;          // the pairs left to it
+    // plain: the warps' second pass over the pairs left, when there are more than few (cap2 0: none), the
+    // pairs that are not for it, and its warp slots
+    int cap2 = 0, few = 0, slots2 = 0;
+    int32_t* far = nullptr;
     int smax = 0;
     int warp_smem = 0;
     int group = 32;                  // learned: lanes per warp-queue pair
@@ -672,12 +676,20 @@ struct WfaScratch {
 };
 
 // Edits the warp kernels search before a pair moves to a whole block
-// (wfa_block.cu).  Their shared memory and stacks are sized for it: at 511, 27
+// (wfa_block.cu).  Their shared memory and stacks are sized for it: at 511, 24
 // warps of 8 KB share an SM where 4 fitted at smax 2048.  The learned path sends
-// pairs estimated at 256 edits and more to blocks at once; the plain path, which
-// knows nothing of a pair, restarts the ones past 255 there (a 64th of the work
-// of a pair at 2048).
-constexpr int WFA_WARP_CAP = 511, WFA_PLAIN_CAP = 255;
+// pairs estimated at 256 edits and more to blocks at once.
+constexpr int WFA_WARP_CAP = 511;
+// The plain path knows nothing of a pair: above smax 511 its warps search 255 edits,
+// which leaves room for 55 of them on an SM, and the pairs they leave start again.  Up to
+// four of those a resident block run on blocks, which are soonest done with a pair.  More
+// of them are bound by throughput, and there a warp's wavefront cell costs half a
+// block's below some 500 diagonals: the ones that look to be within 511 edits then run
+// on warps once more, the others on blocks (20,000 pairs at distance 260-430, smax 512,
+// CIGARs: 14.2 ms on blocks, 7.4 with the second pass; 1,500 of them 1.5 and 1.4; 20,000
+// at 520-720, smax 1024: 34.8 on blocks, 42.2 if the second pass takes them all).
+// Score-only blocks have no walk to wait for and win up to eight a resident block.
+constexpr int WFA_PLAIN_CAP = 255, WFA_FEW_TRACE = 4, WFA_FEW_SCORE = 8;
 constexpr int64_t WFA_STACK_BYTES = (int64_t)16 << 30;     // stack memory cap
 // Below this no pair is estimated at the block kernel's distances.
 constexpr int WFA_BLOCK_MIN = 256;
@@ -686,7 +698,10 @@ constexpr int WFA_BLOCK_MIN = 256;
 static void size_wfa(WfaScratch& S, int n, int smax, bool trace, bool learned, int sm_count, int group)
 {
     S.smax = smax;
+    const int block_slots = smax >= WFA_BLOCK_MIN ? wfa_block_slots(smax, trace, sm_count) : 0;
     S.cap = smax <= WFA_WARP_CAP ? smax : (learned ? WFA_WARP_CAP : WFA_PLAIN_CAP);
+    S.few = (trace ? WFA_FEW_TRACE : WFA_FEW_SCORE) * block_slots;
+    if (!learned && S.cap < smax && n > S.few) S.cap2 = WFA_WARP_CAP;
     const bool blocks = S.cap < smax || (learned && smax >= WFA_BLOCK_MIN);
     if (learned) {
         prepare_mlp();
@@ -696,14 +711,17 @@ static void size_wfa(WfaScratch& S, int n, int smax, bool trace, bool learned, i
         S.stack_slot = routed_stack_slot(S.cap, S.group);
         S.warp_smem = routed_warp_smem(S.cap, S.group);
     } else {
-        S.slots = (int)std::min<int64_t>(wfa_max_slots(S.cap, trace, sm_count), ((int64_t)n + 3) / 4 * 4);
+        const int pass = S.cap2 ? FIRST_PASS : ONLY_PASS;
+        S.slots = (int)std::min<int64_t>(wfa_max_slots(S.cap, trace, sm_count, pass), ((int64_t)n + 3) / 4 * 4);
         S.stack_slot = (int64_t)(S.cap + 1) * (S.cap + 1);
+        if (S.cap2) S.slots2 = std::min(wfa_max_slots(S.cap2, trace, sm_count, SECOND_PASS), S.slots);
     }
-    if (blocks) S.blocks = std::min(wfa_block_slots(smax, trace, sm_count), std::max(n, 1));
+    if (blocks) S.blocks = std::min(block_slots, std::max(n, 1));
     if (trace) {
         const int64_t budget = WFA_STACK_BYTES;
         S.slots = (int)std::min<int64_t>(S.slots, std::max<int64_t>(4, budget / (S.stack_slot * 4) / 4 * 4));
         S.blocks = (int)std::min<int64_t>(S.blocks, std::max<int64_t>(1, budget / ((int64_t)(smax + 1) * (smax + 1) * 4)));
+        S.slots2 = (int)std::min<int64_t>(S.slots2, budget / ((int64_t)(S.cap2 + 1) * (S.cap2 + 1) * 4) / 4 * 4);
     }
     // pairs per counter increment: keep >= 8 grabs per warp
     S.chunk = (int)std::max<int64_t>(1, std::min<int64_t>(16, (int64_t)n / ((int64_t)S.slots * 8)));
@@ -717,13 +735,15 @@ static void carve_wfa(Carve& k, WfaScratch& S, int n, int64_t arena, bool trace,
     S.ctr = k.take<int32_t>(64, 256);
     // kernels that run one after the other share the stacks; the learned path's warp and
     // block kernels run beside each other unless that takes more than one alone may
-    const int64_t warp_words = trace ? (int64_t)S.slots * S.stack_slot : 0;
+    const int64_t warp_words =
+        trace ? std::max((int64_t)S.slots * S.stack_slot, (int64_t)S.slots2 * (S.cap2 + 1) * (S.cap2 + 1)) : 0;
     const int64_t block_words = trace ? (int64_t)S.blocks * (S.smax + 1) * (S.smax + 1) : 0;
     S.beside = learned && S.blocks > 0 && (warp_words + block_words) * 4 <= WFA_STACK_BYTES;
     S.stack = trace ? k.take<int32_t>((size_t)(S.beside ? warp_words + block_words : std::max(warp_words, block_words)))
                     : nullptr;
     S.block_stack = trace && S.beside ? S.stack + warp_words : S.stack;
     S.blk = S.blocks > 0 ? k.take<int32_t>(n) : nullptr;
+    S.far = S.cap2 ? k.take<int32_t>(n) : nullptr;
     if (learned) {
         S.item = k.take<int32_t>(n);
         S.lb = k.take<int32_t>(n);
@@ -766,7 +786,21 @@ static cudaError_t enqueue_wfa(Ctx* c, const WfaScratch& S, PairDesc D, int smax
     if (route == 0) {
         A.masks = packed_masks(S.packed, S.seq_bytes);
         A.pure = S.pure;
+        if (S.cap2) {
+            A.far = B.A.far = S.far;
+            A.far_count = B.A.far_count = S.ctr + 34;
+            A.far_edits = S.cap2;
+            B.few = S.few;
+        }
         e = launch_wfa(A, S.slots, st);
+        if (e == cudaSuccess && S.cap2) {
+            WfaArgs A2 = A;
+            A2.list = A.blk; A2.list_count = A.blk_count; A2.list_few = S.few;
+            A2.cap = S.cap2; A2.stack_slot = (int64_t)(S.cap2 + 1) * (S.cap2 + 1);
+            A2.blk = S.far; A2.blk_count = S.ctr + 34; A2.far = nullptr;
+            A2.counter = S.ctr + 5; A2.chunk = 1;
+            e = launch_wfa(A2, S.slots2, st);
+        }
         if (e == cudaSuccess && S.blocks > 0) e = launch_wfa_block(B, S.blocks, trace ? K_WFA_TRACE : K_WFA_SCORE, st);
         return e;
     }

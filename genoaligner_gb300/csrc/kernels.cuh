@@ -24,8 +24,16 @@ struct WfaArgs {
     int32_t cap;
     int32_t* blk = nullptr;
     int32_t* blk_count = nullptr;
-    const uint32_t* masks = nullptr;      // wfa_kernel: the arena's chunk masks (packed_masks); it sets pure of pairs in blk
+    const uint32_t* masks = nullptr;      // wfa_kernel: the arena's chunk masks (packed_masks); it sets pure of the pairs it leaves
     uint8_t* pure = nullptr;
+    // SECOND_PASS: its pairs, taken when there are more than list_few.  FIRST_PASS: where the
+    // pairs go that are left but look to be past far_edits.
+    const int32_t* list = nullptr;
+    const int32_t* list_count = nullptr;
+    int32_t list_few = 0;
+    int32_t* far = nullptr;
+    int32_t* far_count = nullptr;
+    int32_t far_edits = 0;
 };
 
 struct SwArgs {
@@ -101,13 +109,15 @@ struct RoutedArgs {
 };
 
 // Pairs on whole blocks (wfa_block.cu): the first *big_count of the warp queue
-// (null: none), then the warp kernels' unresolved ones (A.blk, A.blk_count null: none).  A.stack: per
-// block (A.smax + 1)^2 offsets.
+// (null: none), then the warp kernels' unresolved ones (A.blk, A.blk_count null: none)
+// unless they are more than few, which the warps take once more, then those of A.far
+// (A.far_count null: none).  A.stack: per block (A.smax + 1)^2 offsets.
 struct WfaBlockArgs {
     WfaArgs A;
     const int2* big = nullptr;
     const int32_t* big_count = nullptr;
     int32_t* next;
+    int32_t few = INT32_MAX;
 };
 int wfa_block_slots(int smax, bool trace, int sm_count);
 cudaError_t launch_wfa_block(const WfaBlockArgs& B, int blocks, int kernel_id, cudaStream_t st);
@@ -189,7 +199,11 @@ cudaError_t launch_route(int n, const int32_t* item, int32_t* counts, int32_t* s
 cudaError_t launch_routed(const RoutedArgs& R, int lane_slots, int slots, cudaStream_t st);
 
 size_t wfa_smem_bytes(int smax);
-int wfa_max_slots(int smax, bool trace, int sm_count);
+// Passes of wfa_kernel over a batch: the only one before the block kernel, or the first of
+// two, which sends the pairs that look to be past A.far_edits to A.far, or the second,
+// over the pairs of A.list.
+enum { ONLY_PASS, FIRST_PASS, SECOND_PASS };
+int wfa_max_slots(int smax, bool trace, int sm_count, int pass = ONLY_PASS);
 cudaError_t launch_wfa(const WfaArgs& A, int slots, cudaStream_t st);
 
 // Score-only 32-bit kernel (sw.cu): SW_SCORE_C columns per lane.

@@ -135,13 +135,19 @@ __device__ __forceinline__ bool side_pure(const uint32_t* __restrict__ bad, int 
     return !__any_sync(FULL, acc != 0);
 }
 
-template <bool TRACE, int BITS>
+template <bool TRACE, int BITS, int PASS>
 __device__ void wfa_pair(const WfaArgs& A, int p, const uint64_t* __restrict__ P, const uint64_t* __restrict__ T, int m,
                          int n, int32_t* wf0, int32_t* wf1, int32_t* stk, int lane)
 {
-    const int score = wfa_forward<TRACE, BITS, 32>(P, T, m, n, A.cap, wf0, wf1, stk, lane, FULL);
-    if (score < 0 && A.cap < A.smax) {                      // left to the block kernel
-        if (lane == 0) A.blk[atomicAdd(A.blk_count, 1)] = p;
+    const int score = wfa_forward<TRACE, BITS, 32, false, PASS == FIRST_PASS>(P, T, m, n, A.cap, wf0, wf1, stk, lane, FULL);
+    if (score < 0 && A.cap < A.smax) {                      // left to another pass or the block kernel
+        // past A.far_edits at the rate at which cap edits went through both sides' bases?
+        const bool far = PASS == FIRST_PASS && (int64_t)A.cap * (m + n) > (int64_t)A.far_edits * (2 * (-1 - score) - (n - m));
+        if (lane == 0) {
+            A.pure[p] = A.pure[A.D.n + p] = BITS == 2;
+            if (far) A.far[atomicAdd(A.far_count, 1)] = p;
+            else A.blk[atomicAdd(A.blk_count, 1)] = p;
+        }
         return;
     }
     int len = 0;
@@ -155,7 +161,7 @@ __device__ void wfa_pair(const WfaArgs& A, int p, const uint64_t* __restrict__ P
     }
 }
 
-template <bool TRACE>
+template <bool TRACE, int PASS>
 __global__ void __launch_bounds__(128) wfa_kernel(WfaArgs A)
 {
     extern __shared__ int32_t smem[];
@@ -166,14 +172,17 @@ __global__ void __launch_bounds__(128) wfa_kernel(WfaArgs A)
     int32_t* wf1 = wf0 + WS;
     const int64_t slot = (int64_t)blockIdx.x * (blockDim.x >> 5) + wib;
     int32_t* stk = TRACE ? A.stack + slot * A.stack_slot : nullptr;
+    const int cnt = PASS == SECOND_PASS ? *A.list_count : A.D.n;
+    if (PASS == SECOND_PASS && cnt <= A.list_few) return;    // the block kernel's
     for (;;) {
         int p0 = 0;
         if (lane == 0) p0 = atomicAdd(A.counter, A.chunk);
         p0 = __shfl_sync(FULL, p0, 0);
-        if (p0 >= A.D.n) break;
-        const int pend = min(p0 + A.chunk, A.D.n);
-        for (int p = p0; p < pend; ++p) {
+        if (p0 >= cnt) break;
+        const int pend = min(p0 + A.chunk, cnt);
+        for (int q = p0; q < pend; ++q) {
         __syncwarp();
+        const int p = PASS == SECOND_PASS ? A.list[q] : q;
         const int m = A.D.a_len[p];       // pattern
         const int n = A.D.b_len[p];       // text
         if (m <= 0 || n <= 0) {
@@ -193,15 +202,14 @@ __global__ void __launch_bounds__(128) wfa_kernel(WfaArgs A)
         // for the flags would be one more launch (48 reads: 60 -> 49 us a call, with the
         // fills and the CIGAR packing in their neighbours' kernels)
         const bool pure = side_pure(A.masks + (A.D.a_off[p] >> 5), m, lane) & side_pure(A.masks + (A.D.b_off[p] >> 5), n, lane);
-        if (A.blk && lane == 0) A.pure[p] = A.pure[A.D.n + p] = pure;
         if (pure) {
             const uint64_t* P = A.D.packed + (A.D.a_off[p] >> 5);
             const uint64_t* T = A.D.packed + (A.D.b_off[p] >> 5);
-            wfa_pair<TRACE, 2>(A, p, P, T, m, n, wf0, wf1, stk, lane);
+            wfa_pair<TRACE, 2, PASS>(A, p, P, T, m, n, wf0, wf1, stk, lane);
         } else {
             const uint64_t* P = reinterpret_cast<const uint64_t*>(A.D.seq + A.D.a_off[p]);
             const uint64_t* T = reinterpret_cast<const uint64_t*>(A.D.seq + A.D.b_off[p]);
-            wfa_pair<TRACE, 8>(A, p, P, T, m, n, wf0, wf1, stk, lane);
+            wfa_pair<TRACE, 8, PASS>(A, p, P, T, m, n, wf0, wf1, stk, lane);
         }
         }
     }
@@ -375,12 +383,17 @@ int64_t packed_arena_words(int64_t seq_bytes)
 
 size_t wfa_smem_bytes(int smax) { return (size_t)4 * 2 * (2 * smax + 3) * sizeof(int32_t); }
 
-int wfa_max_slots(int smax, bool trace, int sm_count)
+using WfaKernel = void (*)(WfaArgs);
+static WfaKernel wfa_kernel_of(bool trace, int pass)
 {
-    const size_t smem = wfa_smem_bytes(smax);
-    const int per_sm = trace ? blocks_per_sm((const void*)wfa_kernel<true>, 128, smem)
-                             : blocks_per_sm((const void*)wfa_kernel<false>, 128, smem);
-    return per_sm * sm_count * 4;
+    if (pass == FIRST_PASS) return trace ? wfa_kernel<true, FIRST_PASS> : wfa_kernel<false, FIRST_PASS>;
+    if (pass == SECOND_PASS) return trace ? wfa_kernel<true, SECOND_PASS> : wfa_kernel<false, SECOND_PASS>;
+    return trace ? wfa_kernel<true, ONLY_PASS> : wfa_kernel<false, ONLY_PASS>;
+}
+
+int wfa_max_slots(int smax, bool trace, int sm_count, int pass)
+{
+    return blocks_per_sm((const void*)wfa_kernel_of(trace, pass), 128, wfa_smem_bytes(smax)) * sm_count * 4;
 }
 
 cudaError_t launch_wfa(const WfaArgs& A, int slots, cudaStream_t st)
@@ -390,8 +403,8 @@ cudaError_t launch_wfa(const WfaArgs& A, int slots, cudaStream_t st)
     const size_t smem = wfa_smem_bytes(A.cap);
     const int id = A.trace ? K_WFA_TRACE : K_WFA_SCORE;
     launch_begin(id, st);
-    if (A.trace) wfa_kernel<true><<<blocks, 128, smem, st>>>(A);
-    else         wfa_kernel<false><<<blocks, 128, smem, st>>>(A);
+    const WfaKernel kernel = wfa_kernel_of(A.trace, A.list ? SECOND_PASS : (A.far ? FIRST_PASS : ONLY_PASS));
+    kernel<<<blocks, 128, smem, st>>>(A);
     launch_end(id, st);
     return cudaGetLastError();
 }

@@ -10,7 +10,7 @@
 // blocks of 128 threads, 4.2 ms with these blocks and the warps' cap.
 //
 // Items: the router's pairs estimated at s >= 256 (largest first), then the
-// pairs the warp kernels left unresolved at their cap.
+// pairs the warp kernels left unresolved at their last cap.
 #include "wfa_step.cuh"
 
 namespace ga {
@@ -91,7 +91,9 @@ __global__ void __launch_bounds__(BLK_T, 2) wfa_block_kernel(WfaBlockArgs B)
     __shared__ int s_q, s_at[3];
     const WfaArgs& A = B.A;
     const int t = threadIdx.x, smax = A.smax;
-    const int nbig = B.big_count ? *B.big_count : 0, cnt = nbig + (A.blk_count ? *A.blk_count : 0);
+    const int left = A.blk_count ? *A.blk_count : 0;
+    const int nbig = B.big_count ? *B.big_count : 0, nblk = nbig + (left > B.few ? 0 : left);
+    const int cnt = nblk + (A.far_count ? *A.far_count : 0);
     int32_t* const wf0 = bsmem;
     int32_t* const wf1 = bsmem + 2 * smax + 3;
     int32_t* const stk = TRACE ? A.stack + blockIdx.x * ((int64_t)(smax + 1) * (smax + 1)) : nullptr;
@@ -101,7 +103,7 @@ __global__ void __launch_bounds__(BLK_T, 2) wfa_block_kernel(WfaBlockArgs B)
         const int q = s_q;
         __syncthreads();
         if (q >= cnt) break;
-        const int p = q < nbig ? B.big[q].x : A.blk[q - nbig];
+        const int p = q < nbig ? B.big[q].x : (q < nblk ? A.blk[q - nbig] : A.far[q - nblk]);
         const int m = A.D.a_len[p], n = A.D.b_len[p];
         if (m <= 0 || n <= 0) {
             const int len = m <= 0 ? max(n, 0) : m;

@@ -116,7 +116,8 @@ __device__ __forceinline__ int wave_hi(int s, int n, int kfinal, int smax) { ret
 // by that chain, gains (the warps' 669 pairs of the 2,000-pair long batch: 1.0 ->
 // 0.73 ms), a full device, bound by instruction issue, loses (20,000 x 2 kb: 656 ->
 // 695 us).
-template <bool TRACE, int BITS, int G, bool AHEAD = false>
+// REACH: a pair above smax returns -1 less the offset it has reached on its final diagonal.
+template <bool TRACE, int BITS, int G, bool AHEAD = false, bool REACH = false>
 __device__ int wfa_forward(const uint64_t* __restrict__ P, const uint64_t* __restrict__ T, int m, int n, int smax,
                            int32_t* wf0, int32_t* wf1, int32_t* stk, int gl, unsigned gmask)
 {
@@ -134,6 +135,7 @@ __device__ int wfa_forward(const uint64_t* __restrict__ P, const uint64_t* __res
         if (TRACE) stk[0] = off0;
     }
     gsync<G>(gmask);
+    int reach = 0;
     for (int s = 1; s <= smax; ++s) {
         const int hi = wave_hi(s, n, kfinal, smax);
         int32_t* const row = TRACE ? stk + (int64_t)s * s + s : nullptr;
@@ -157,10 +159,11 @@ __device__ int wfa_forward(const uint64_t* __restrict__ P, const uint64_t* __res
             }
         }
         gsync<G>(gmask);
-        if (cur[kfinal] >= n) return s;
+        reach = cur[kfinal];
+        if (reach >= n) return s;
         int32_t* t = prev; prev = cur; cur = t;
     }
-    return -1;
+    return REACH ? -1 - max(reach, 0) : -1;
 }
 
 // The walk's choice at a cell from the wavefront before: the offset it came from

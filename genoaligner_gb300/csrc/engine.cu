@@ -781,10 +781,11 @@ static cudaError_t enqueue_wfa(Ctx* c, const WfaScratch& S, PairDesc D, int smax
     F.add(S.ctr, 64, 0);
     F.add(err, 1, 0);
     if (route != 0) F.add(S.counts, 2 * NB + 4, 0);
-    cudaError_t e = launch_pack(D, S.seq_bytes, S.packed, route != 0 ? S.pure : nullptr, st, F);
+    const bool flags = route != 0 || purity_pass(D.n);
+    cudaError_t e = launch_pack(D, S.seq_bytes, S.packed, flags ? S.pure : nullptr, st, F);
     if (e != cudaSuccess) return e;
     if (route == 0) {
-        A.masks = packed_masks(S.packed, S.seq_bytes);
+        if (!flags) A.masks = packed_masks(S.packed, S.seq_bytes);
         A.pure = S.pure;
         if (S.cap2) {
             A.far = B.A.far = S.far;

@@ -24,7 +24,7 @@ struct WfaArgs {
     int32_t cap;
     int32_t* blk = nullptr;
     int32_t* blk_count = nullptr;
-    const uint32_t* masks = nullptr;      // wfa_kernel: the arena's chunk masks (packed_masks); it sets pure of the pairs it leaves
+    const uint32_t* masks = nullptr;      // wfa_kernel: the arena's chunk masks (packed_masks; null: D.pure is set); it sets pure of the pairs it leaves
     uint8_t* pure = nullptr;
     // SECOND_PASS: its pairs, taken when there are more than list_few.  FIRST_PASS: where the
     // pairs go that are left but look to be past far_edits.
@@ -147,6 +147,12 @@ inline uint32_t* packed_masks(uint64_t* packed, int64_t seq_bytes)
 {
     return reinterpret_cast<uint32_t*>(packed + seq_bytes / 32 + 2);
 }
+// Plain WFA batches of this many pairs set the purity flags in a kernel of their own,
+// smaller ones read the masks in each warp.  The kernel is one more launch (48 reads: 34
+// us a call against 30), the warp's dependent load of each mask 70 ns a pair whose work
+// is small (1M pairs of 30-60 bases: 554 us with the kernel, 637 without; 1M of 150-250:
+// 1,435 and 1,511; 65,000 pairs: equal).
+inline bool purity_pass(int n) { return n >= 65536; }
 int64_t packed_arena_words(int64_t seq_bytes);
 cudaError_t launch_pack_arena(const uint8_t* seq, int64_t seq_bytes, uint64_t* packed, uint32_t* bad, cudaStream_t st);
 // Sequences copied to the device as the caller laid them out -- one span per

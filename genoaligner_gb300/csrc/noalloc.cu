@@ -115,7 +115,7 @@ extern "C" int32_t ga_wfa_device_noalloc(const ga_device_batch* b, int32_t smax,
     }
     if (b->n == 0) return GA_OK;
 
-    // scratch layout: [counter, error word | 2 n spare bytes | 2-bit arena | wavefront stacks]
+    // scratch layout: [counter, error word | purity flags (purity_pass) | 2-bit arena | wavefront stacks]
     const size_t head = 256;
     const size_t pure_bytes = round256(2 * (size_t)b->n);
     const size_t packed_bytes = round256((size_t)packed_arena_words(b->seq_bytes) * sizeof(uint64_t));
@@ -139,6 +139,7 @@ extern "C" int32_t ga_wfa_device_noalloc(const ga_device_batch* b, int32_t smax,
         return GA_DEVICE_ERROR;
     }
     int32_t* ctr = reinterpret_cast<int32_t*>(base);
+    uint8_t* pure = purity_pass(b->n) ? base + head : nullptr;
     uint64_t* packed = reinterpret_cast<uint64_t*>(base + head + pure_bytes);
     int32_t* stk = trace ? reinterpret_cast<int32_t*>(base + fixed) : nullptr;
 
@@ -157,7 +158,7 @@ extern "C" int32_t ga_wfa_device_noalloc(const ga_device_batch* b, int32_t smax,
         return GA_DEVICE_ERROR;
     }
     PairDesc D;
-    D.seq = b->seq; D.packed = packed; D.pure = nullptr;
+    D.seq = b->seq; D.packed = packed; D.pure = pure;
     D.a_off = b->a_off; D.a_len = b->a_len; D.b_off = b->b_off; D.b_len = b->b_len;
     D.out_off = b->out_off; D.n = b->n;
     WfaArgs A;
@@ -166,8 +167,8 @@ extern "C" int32_t ga_wfa_device_noalloc(const ga_device_batch* b, int32_t smax,
     A.stack = stk; A.stack_slot = ((int64_t)smax + 1) * ((int64_t)smax + 1);
     A.counter = ctr; A.err = ctr + 1;
     A.chunk = chunk;
-    A.masks = packed_masks(packed, b->seq_bytes);
-    if (launch_pack(D, b->seq_bytes, packed, nullptr, st) != cudaSuccess || launch_wfa(A, slots, st) != cudaSuccess) {
+    if (!pure) A.masks = packed_masks(packed, b->seq_bytes);
+    if (launch_pack(D, b->seq_bytes, packed, pure, st) != cudaSuccess || launch_wfa(A, slots, st) != cudaSuccess) {
         cudaGetLastError();
         if (err) *err = "kernel launch failed";
         return GA_DEVICE_ERROR;

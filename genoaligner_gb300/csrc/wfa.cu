@@ -198,10 +198,15 @@ __global__ void __launch_bounds__(128) wfa_kernel(WfaArgs A)
             }
             continue;
         }
-        // both sides pure ACGT: read from the chunk masks by the warp, where a kernel
-        // for the flags would be one more launch (48 reads: 60 -> 49 us a call, with the
-        // fills and the CIGAR packing in their neighbours' kernels)
-        const bool pure = side_pure(A.masks + (A.D.a_off[p] >> 5), m, lane) & side_pure(A.masks + (A.D.b_off[p] >> 5), n, lane);
+        // both sides pure ACGT: in small batches read from the chunk masks by the warp, where
+        // a kernel for the flags would be one more launch (purity_pass; with the fills and
+        // the CIGAR packing in their neighbours' kernels, 48 reads took 60 -> 49 us a call)
+        bool pure;
+        if (A.masks) {
+            pure = side_pure(A.masks + (A.D.a_off[p] >> 5), m, lane) & side_pure(A.masks + (A.D.b_off[p] >> 5), n, lane);
+        } else {
+            pure = A.D.pure[p] && A.D.pure[A.D.n + p];
+        }
         if (pure) {
             const uint64_t* P = A.D.packed + (A.D.a_off[p] >> 5);
             const uint64_t* T = A.D.packed + (A.D.b_off[p] >> 5);

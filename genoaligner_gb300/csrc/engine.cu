@@ -1297,9 +1297,10 @@ static int sw_coop_warps(int l, bool trace, const ga_tune& T)
 static cudaError_t enqueue_plan_sw(const PairDesc& D, const ga_sw_scoring& sc, bool trace, int64_t cell_limit,
                                    int32_t too_large_score, int32_t* out_score, int32_t* dwork, int32_t* scratch,
                                    long long* dres, const ga_tune& T, cudaStream_t st, const uint8_t* try16 = nullptr,
-                                   const SwPlan* launched = nullptr, int32_t* err = nullptr)
+                                   const SwPlan* launched = nullptr, int32_t* err = nullptr, int parts = 1)
 {
     SwPlanArgs A;
+    A.parts = parts;
     if (launched) {
         A.launched = 0;
         for (int l = 0; l < SP_LISTS; ++l) A.launched |= (launched->ints[l] > 0) << l;
@@ -1364,8 +1365,11 @@ static cudaError_t device_plan_sw(const PairDesc& D, const ga_sw_scoring& sc, bo
 // in its 32-bit list as well; per-warp memory is the largest any of those
 // pairs (or items) can need.  The kernels take the exact figures from the
 // plan on the device (plan_view); these only size the grids and the memory.
+// parts: ranges like this one run at once, and an item's share is one of them all
+// (sp_coop_cells).  (Against its range alone, every item of 12 ranges of 1,600 pairs of
+// 1,000 to 1,400 bases was above it: 20,000 pairs took 15.2 ms on blocks, 12.9 on warps.)
 static SwPlan bound_plan_sw(const ga_sw_request* reqs, int32_t n, bool trace, int64_t cell_limit, const ga_tune& T,
-                            bool learned)
+                            bool learned, int parts)
 {
     SwPlan P;
     const ga_sw_scoring sc = reqs[0].scoring;
@@ -1381,6 +1385,7 @@ static SwPlan bound_plan_sw(const ga_sw_request* reqs, int32_t n, bool trace, in
         largest = std::max(largest, c);
         cols = std::max(cols, (int)reqs[i].pattern_len);
     }
+    cells *= parts;
     const int W32 = sw_coop_block(largest, cols, cells, device_sms());
     int64_t coop[SP_LISTS];
     for (int l = SP_L32; l < SP_LISTS; ++l) coop[l] = sp_coop_cells(limit, cells, sw_coop_warps(l, trace, T));
@@ -1423,15 +1428,16 @@ static SwPlan bound_plan_sw(const ga_sw_request* reqs, int32_t n, bool trace, in
     P.ints[SP_L16] = 2 * ((n16 + 1) / 2);
     P.dir[SP_L16] = n16 ? (trace ? sw16ck_dir_words(maxM16, maxN16, T.sw_window) : sw16so_dir_words(maxM16, maxN16)) : 0;
     // the 16-bit list has its whole-block phase when the widest possible item is above its share of them all
-    const int64_t warps16 = sw_coop_warps(SP_L16, trace, T), coop16 = sp_coop_cells(limit, cells16 / 2, warps16);
+    cells16 = parts * (cells16 / 2);
+    const int64_t warps16 = sw_coop_warps(SP_L16, trace, T), coop16 = sp_coop_cells(limit, cells16, warps16);
     if ((int64_t)maxM16 * maxN16 > coop16) {
         P.ncoop[SP_L16] = 1;
         // with a block for each item, the largest per-warp memory is a share of the
         // widest item's or the whole of one of coop16 cells (M rows, at most 255
         // padding columns, two words per 64 cells for rows and for edges each)
-        const int W = P.w[SP_L16] = sw_coop_block(largest16, maxN16, cells16 / 2, device_sms());
+        const int W = P.w[SP_L16] = sw_coop_block(largest16, maxN16, cells16, device_sms());
         const int64_t own = sw16_own_words(trace, T.sw_window);
-        if (W * ((n16 + 1) / 2) <= warps16)
+        if (W * ((n16 + 1) / 2) * parts <= warps16)
             P.dir[SP_L16] = std::min(P.dir[SP_L16], std::max(sw_coop_share(P.dir[SP_L16], W, own),
                                                              coop16 / 16 + 16 * (int64_t)maxM16 + own + 8));
     }
@@ -1655,7 +1661,7 @@ static int32_t sw_batch_range(const ga_sw_request* reqs, int32_t n, int64_t base
     // Launch sizes from the lengths (bounds of the plan the device builds):
     // every launch is enqueued without reading the plan back.
     const bool route = learned && trace;                 // the SW model picks the 16-bit pairs
-    const SwPlan P = bound_plan_sw(reqs, n, trace, trace ? cell_limit : -1, T, route);
+    const SwPlan P = bound_plan_sw(reqs, n, trace, trace ? cell_limit : -1, T, route, parts);
     SwSlots S = size_sw(P, trace, T, c->sm_count, sw_dir_budget(c, parts));
     // Ranges that run beside others give their 16-bit persistent kernel three
     // quarters of the device's blocks: the next range's pack and plan kernels
@@ -1775,7 +1781,7 @@ static int32_t sw_batch_range(const ga_sw_request* reqs, int32_t n, int64_t base
         if (e == cudaSuccess && route) e = launch_sw_route(D, s0.match, s0.gap_open, dfeat, dy, dtry, st);
         if (e == cudaSuccess)
             e = enqueue_plan_sw(D, s0, trace, trace ? cell_limit : -1, -1, dsc, dwork, dscr, dres, T, st, dtry,
-                                &P, der);
+                                &P, der, parts);
         if (e == cudaSuccess)
             e = launch_plan(P, S, D, s0, trace, T, dwork, dsc, dpos, dln, dcg, ddirs, dedge, dctr, der, st, dscr, dres);
         if (e == cudaSuccess && trace)
@@ -1799,7 +1805,7 @@ static int32_t sw_batch_range(const ga_sw_request* reqs, int32_t n, int64_t base
                 (uint64_t)P.ints[0], (uint64_t)P.ints[1], (uint64_t)P.ints[2], (uint64_t)P.dir[0],
                 (uint64_t)P.dir[1], (uint64_t)P.dir[2], (uint64_t)P.edge_slot,
                 (uint64_t)P.w[0] | (uint64_t)P.w[1] << 8 | (uint64_t)P.w[2] << 16 | (uint64_t)(P.ncoop[0] > 0) << 24,
-                (uint64_t)(int64_t)c->prio,
+                (uint64_t)(int64_t)c->prio, (uint64_t)parts,
                 (uint64_t)P.n_opt, (uint64_t)P.dir_opt, (uint64_t)S.dir_words, (uint64_t)S.max_slots,
                 (uint64_t)S.s[0] | (uint64_t)S.s[1] << 32, (uint64_t)S.s[2] | (uint64_t)S.s_esc << 32};
             le = replay_graph(c->swexec, c->swkey, c->swseen, key, c->swlaunches, c->stream, enqueue);

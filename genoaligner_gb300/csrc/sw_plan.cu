@@ -127,6 +127,13 @@ __global__ void sp_classify_kernel(SwPlanArgs P)
     }
 }
 
+// Cells that the list's items cost the device's warps: an item of the 16-bit list holds
+// two pairs and costs a warp what one does, and the ranges beside this one cost the same.
+__device__ __forceinline__ int64_t sp_item_cells(const SwPlanArgs& P, const long long* res, int l)
+{
+    return (int64_t)P.parts * (l == SP_L16 ? res[SP_CELLS + l] / 2 : res[SP_CELLS + l]);
+}
+
 // Lists' lengths in the flattened work array and their offsets there (16-bit lists
 // hold two entries per work item), the warps of their whole-block launches, and
 // whether the launches that follow serve these lists.
@@ -143,7 +150,7 @@ __device__ __forceinline__ void sp_lay_out(const SwPlanArgs& P, long long* res, 
         base += ints;
         res[SP_COOPW + l] = P.coop_block[l] ? P.coop_block[l]
                                             : sw_coop_block(res[SP_LARGEST + l], (int)res[SP_COLS + l],
-                                                            l == SP_L16 ? res[SP_CELLS + l] / 2 : res[SP_CELLS + l], P.sms);
+                                                            sp_item_cells(P, res, l), P.sms);
     }
     if (!served && P.err) atomicOr(P.err, ERR_SCRATCH);
 }
@@ -159,13 +166,11 @@ __device__ __forceinline__ void sp_pack_list(const SwPlanArgs& P, const long lon
 {
     const long long cnt = res[SP_COUNT + l];
     int32_t* w = P.work + res[SP_BASE + l];
-    // (an item of the 16-bit list holds two pairs and costs a warp what one does)
-    const int64_t coop =
-        sp_coop_cells(P.coop_limit, l == SP_L16 ? res[SP_CELLS + l] / 2 : res[SP_CELLS + l], P.coop_warps[l]);
+    const int64_t coop = sp_coop_cells(P.coop_limit, sp_item_cells(P, res, l), P.coop_warps[l]);
     const int W = (int)res[SP_COOPW + l];
     if (l == SP_L16) {
         const long long items = (cnt + 1) / 2;
-        const bool few = W * items <= P.coop_warps[l];
+        const bool few = W * items * P.parts <= P.coop_warps[l];
         for (long long q = first; q < items; q += step) {
             const int a = srt[2 * q], b = 2 * q + 1 < cnt ? srt[2 * q + 1] : -1;
             w[2 * q] = a;

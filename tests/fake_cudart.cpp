@@ -113,7 +113,11 @@ cudaError_t cudaFuncSetAttribute(const void* f, cudaFuncAttribute a, int v)
     if (a == cudaFuncAttributeMaxDynamicSharedMemorySize) smem_limit[{device, f}] = v;
     return cudaSuccess;
 }
-cudaError_t cudaOccupancyMaxActiveBlocksPerMultiprocessor(int* n, const void*, int, size_t) { *n = 1; return cudaSuccess; }
+cudaError_t cudaOccupancyMaxActiveBlocksPerMultiprocessor(int* n, const void*, int threads, size_t)
+{
+    *n = threads < 512 ? 512 / threads : 1;
+    return cudaSuccess;
+}
 cudaError_t cudaGetSymbolAddress(void**, const void*) { return set(cudaErrorInvalidSymbol); }
 cudaError_t cudaGetDriverEntryPointByVersion(const char*, void** f, unsigned, unsigned long long,
                                              enum cudaDriverEntryPointQueryResult*)

@@ -1,0 +1,25 @@
+"""How the ranges of a host SW batch that run at once launch their work (on a runtime
+that records, no GPU)."""
+import numpy as np
+import pytest
+
+from fake_cuda import fake_path, rt  # noqa: F401
+from genoaligner_gb300 import api, workloads
+
+BLOCKS, WARPS = "sw16ck_kernelILi2ELb1E", "sw16ck_kernelILi2ELb0E"      # with, without whole-block items
+
+
+def _call(n, length):
+    """n pairs of one length, each side one buffer that every request shares."""
+    a = workloads.random_bases(np.random.default_rng(1), length)
+    off, lens = np.zeros(n, np.int64), np.full(n, length, np.int32)
+    got = api.align_sw_batch_packed(a, off, lens, a, off, lens, scoring=(2, -3, 3, 1))
+    assert got.status == api.Status.ok, got.error
+
+
+def test_an_items_share_is_of_all_ranges(rt):
+    _call(600, 1300)                                  # alone: few items, each on a block
+    assert rt.count(BLOCKS) > 0 and rt.count(WARPS) == 0
+    rt.clear()
+    _call(20000, 1300)                                # 12 ranges: more items than the device has warps
+    assert rt.count(WARPS) > 1 and rt.count(BLOCKS) == 0

@@ -1773,7 +1773,7 @@ static int32_t sw_batch_range(const ga_sw_request* reqs, int32_t n, int64_t base
         F.add(dln, n, 0);
         F.add(der, 1, 0);
         F.add(dctr, 8, 0);
-        sw_plan_fills(F, n, dscr, dres);
+        sw_plan_fills(F, n, parts, dscr, dres);
         cudaError_t e = cudaSuccess;
         if (e == cudaSuccess && span) e = launch_gather_sides(D, dseq, dspan_a, dspan_b, dsa, dsb, st);
         if (e == cudaSuccess && span) e = cudaMemsetAsync(dseq + arena - 64, 0, 64, st);
@@ -2396,7 +2396,7 @@ int32_t ga_sw_device_ex(const ga_device_batch* b, ga_sw_scoring sc, int32_t trac
         F.add(out_pos, 4 * (int64_t)n, -1);
         if (out_len) F.add(out_len, n, 0);
         if (counters) F.add(counters, 64, 0);
-        sw_plan_fills(F, n, dscr, dres);
+        sw_plan_fills(F, n, 1, dscr, dres);
         return launch_pack(D, b->seq_bytes, nullptr, dpure, st, F);
     };
     sw_plan_prepare();

@@ -306,8 +306,8 @@ struct SwPlanArgs {
 };
 // Raises the planner's shared-memory limit (once, outside any capture).
 void sw_plan_prepare();
-// What launch_sw_plan finds zeroed for n pairs.
-void sw_plan_fills(Fills& F, int n, int32_t* scratch, long long* res);
+// What launch_sw_plan finds zeroed for n pairs (parts: SwPlanArgs).
+void sw_plan_fills(Fills& F, int n, int parts, int32_t* scratch, long long* res);
 int64_t sw_plan_scratch_ints(int n);
 cudaError_t launch_sw_plan(SwPlanArgs P, int32_t* scratch, cudaStream_t st);
 // Result checks of every pair with a CIGAR (sw_plan.cu): flags[p] =

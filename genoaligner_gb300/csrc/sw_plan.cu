@@ -200,13 +200,13 @@ __device__ __forceinline__ void sp_pack_list(const SwPlanArgs& P, const long lon
 }
 
 // Exclusive scan of each list's bucket counts (bucket order is largest first) by one
-// block of SP_SCAN_T threads: start[l][b] for list l's bucket b, in cnt's place or in
+// block of NT threads: start[l][b] for list l's bucket b, in cnt's place or in
 // another array (flat: counted on from list to list); the lists' totals.
-constexpr int SP_SCAN_T = 1024;
+template <int NT>
 __device__ __forceinline__ void sp_scan(const int32_t* cnt, int32_t* start, bool flat, int32_t (*warp_sum)[32],
                                         long long* total)
 {
-    constexpr int BPT = SP_NB / SP_SCAN_T;
+    constexpr int BPT = SP_NB / NT;
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     int own[SP_LISTS], incl[SP_LISTS];
 #pragma unroll
@@ -224,7 +224,7 @@ __device__ __forceinline__ void sp_scan(const int32_t* cnt, int32_t* start, bool
     }
     __syncthreads();
     if (wid < SP_LISTS) {
-        const int v = warp_sum[wid][lane];
+        const int v = lane < NT / 32 ? warp_sum[wid][lane] : 0;
         int s = v;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
@@ -249,13 +249,14 @@ __device__ __forceinline__ void sp_scan(const int32_t* cnt, int32_t* start, bool
     }
 }
 
-// (A warp per list, 128 buckets a lane, took 30 us of a 200,000-pair plan; this
-// 7.)
-__global__ void __launch_bounds__(SP_SCAN_T) sp_scan_kernel(SwPlanArgs P)
+// (A warp per list, 128 buckets a lane, took 30 us of a 200,000-pair plan; 1,024
+// threads 7.)
+template <int NT>
+__global__ void __launch_bounds__(NT) sp_scan_kernel(SwPlanArgs P)
 {
     __shared__ long long total[SP_LISTS];
     __shared__ int32_t warp_sum[SP_LISTS][32];
-    sp_scan(P.counts, P.starts, false, warp_sum, total);
+    sp_scan<NT>(P.counts, P.starts, false, warp_sum, total);
     if (threadIdx.x == 0) sp_lay_out(P, P.res, total);
 }
 
@@ -296,7 +297,7 @@ __global__ void sp_pack_kernel(SwPlanArgs P)
 // (plan of one pair 51 -> 11 us; a call of 4,096 pairs 399 us either way, of 8,192 pairs
 // 558 us by one block and 541 by four kernels, of 16,384 pairs 933 and 886).  A
 // pair's place in its bucket is what its count's atomic returns.
-constexpr int SP_SMALL = 4096, SP_SMALL_T = SP_SCAN_T;
+constexpr int SP_SMALL = 4096, SP_SMALL_T = 1024;
 __global__ void __launch_bounds__(SP_SMALL_T) sp_small_kernel(SwPlanArgs P)
 {
     extern __shared__ int32_t sp_smem[];
@@ -320,7 +321,7 @@ __global__ void __launch_bounds__(SP_SMALL_T) sp_small_kernel(SwPlanArgs P)
     }
     if (wid * 32 < n) sp_add_tally(T, rec, lane);
     __syncthreads();
-    sp_scan(cnt, cnt, true, warp_sum, total);
+    sp_scan<SP_SMALL_T>(cnt, cnt, true, warp_sum, total);
     if (tid == 0) sp_lay_out(P, reinterpret_cast<long long*>(rec), total);
     __syncthreads();
 #pragma unroll
@@ -447,9 +448,15 @@ constexpr size_t SP_SMALL_SMEM = sizeof(int32_t) * (SP_LISTS * SP_NB + SP_SMALL)
 
 void sw_plan_prepare() { blocks_per_sm((const void*)sp_small_kernel, SP_SMALL_T, SP_SMALL_SMEM); }
 
-void sw_plan_fills(Fills& F, int n, int32_t* scratch, long long* res)
+// A range that runs beside others plans while their persistent kernels hold three
+// blocks of 128 threads a multiprocessor and 48 of its 64 K registers: a block of 1,024
+// threads finds no room there before one of them ends (5 ranges of 4,000 pairs: 170 us
+// a launch of four, 520 for the one block), so its plan is made of blocks of 256.
+static bool sp_one_block(int n, int parts) { return n <= SP_SMALL && parts == 1; }
+
+void sw_plan_fills(Fills& F, int n, int parts, int32_t* scratch, long long* res)
 {
-    if (n <= SP_SMALL) return;                         // sp_small_kernel keeps its own
+    if (sp_one_block(n, parts)) return;                // sp_small_kernel keeps its own
     F.add(scratch + n, SP_LISTS * SP_NB, 0);           // the buckets' counts
     F.add(res, 2 * SP_RES, 0);
 }
@@ -462,7 +469,7 @@ cudaError_t launch_sw_plan(SwPlanArgs P, int32_t* scratch, cudaStream_t st)
     P.starts = P.counts + SP_LISTS * SP_NB;
     P.sorted = P.starts + SP_LISTS * SP_NB;
     if (n <= 0) return cudaSuccess;
-    if (n <= SP_SMALL) {
+    if (sp_one_block(n, P.parts)) {
         launch_begin(K_SWPLAN, st);
         sp_small_kernel<<<1, SP_SMALL_T, SP_SMALL_SMEM, st>>>(P);
         launch_end(K_SWPLAN, st);
@@ -474,7 +481,8 @@ cudaError_t launch_sw_plan(SwPlanArgs P, int32_t* scratch, cudaStream_t st)
     sp_classify_kernel<<<blocks, 256, 0, st>>>(P);
     launch_end(K_SWPLAN, st);
     launch_begin(K_SWPLAN, st);
-    sp_scan_kernel<<<1, SP_SCAN_T, 0, st>>>(P);
+    if (P.parts > 1) sp_scan_kernel<256><<<1, 256, 0, st>>>(P);
+    else sp_scan_kernel<1024><<<1, 1024, 0, st>>>(P);
     launch_end(K_SWPLAN, st);
     launch_begin(K_SWPLAN, st);
     sp_scatter_kernel<<<blocks, 256, 0, st>>>(P);

@@ -23,3 +23,16 @@ def test_an_items_share_is_of_all_ranges(rt):
     rt.clear()
     _call(20000, 1300)                                # 12 ranges: more items than the device has warps
     assert rt.count(WARPS) > 1 and rt.count(BLOCKS) == 0
+
+
+def test_a_range_plans_in_small_blocks(rt):
+    """Beside other ranges' persistent kernels a block of 1,024 threads finds no room."""
+    _call(20000, 800)                                   # 6 ranges of 3,333 pairs
+    assert rt.count("sp_scan_kernelILi256E") > 1
+    assert rt.count("sp_small_kernel") == 0 and rt.count("sp_scan_kernelILi1024E") == 0
+    rt.clear()
+    _call(3333, 800)
+    assert rt.count("sp_small_kernel") == 1 and rt.count("sp_scan_kernel") == 0
+    rt.clear()
+    _call(5000, 100)
+    assert rt.count("sp_small_kernel") == 0 and rt.count("sp_scan_kernelILi1024E") == 1

@@ -86,23 +86,25 @@ __global__ void __launch_bounds__(256) purity_mask_kernel(PairDesc D, const uint
 
 // Letters of each sequence straight from the bytes (the Smith-Waterman paths,
 // which build no 2-bit arena): 1 every byte is A, C, G or T; 2 some are N; 0
-// some are neither.  A warp per sequence, 512 bytes a step: the loads of a
-// sequence are contiguous, and a sequence takes length / 512 steps where a
-// thread took length / 16 (600 pairs up to 1 kb: 31 -> 7.5 us; 200,000 uneven
-// pairs, 260 MB: 226 -> 154 us, bound by the latency of the few loads a warp has
-// in flight).
+// some are neither.  G lanes per sequence (purity_lanes), 16 G bytes a step: the
+// loads of a sequence are contiguous, and with a warp it takes length / 512 steps
+// where a thread takes length / 16 (600 pairs up to 1 kb: 31 -> 7.5 us; 200,000
+// uneven pairs, 260 MB: 226 -> 154 us, bound by the latency of the few loads a
+// warp has in flight).
+template <int G>
 __global__ void __launch_bounds__(256) purity_kernel(PairDesc D, uint8_t* __restrict__ pure, const Fills F)
 {
     fill_words(F);
-    const int lane = threadIdx.x & 31;
-    const int nw = (gridDim.x * blockDim.x) >> 5;
-    for (int q = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; q < 2 * D.n; q += nw) {
+    const int lane = threadIdx.x & (G - 1);
+    const unsigned gmask = (0xffffffffu >> (32 - G)) << (threadIdx.x & 31 & ~(G - 1));
+    const int ng = gridDim.x * blockDim.x / G;
+    for (int q = (blockIdx.x * blockDim.x + threadIdx.x) / G; q < 2 * D.n; q += ng) {
         const bool is_a = q < D.n;
         const int p = is_a ? q : q - D.n;
         const uint8_t* s = D.seq + (is_a ? D.a_off[p] : D.b_off[p]);
         const int len = is_a ? D.a_len[p] : D.b_len[p];
         uint32_t other = 0, n_seen = 0;                 // bits 0, 8, 16, 24: a byte outside ACGT; an N
-        for (int o = 16 * lane; o < len; o += 512) {
+        for (int o = 16 * lane; o < len; o += 16 * G) {
             const uint4 v = __ldg(reinterpret_cast<const uint4*>(s + o));
             const uint32_t w[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
@@ -120,7 +122,7 @@ __global__ void __launch_bounds__(256) purity_kernel(PairDesc D, uint8_t* __rest
                 n_seen |= not_a & ~not_n;
             }
         }
-        const bool bad = __any_sync(FULL, other != 0), some_n = __any_sync(FULL, n_seen != 0);
+        const bool bad = __any_sync(gmask, other != 0), some_n = __any_sync(gmask, n_seen != 0);
         if (lane == 0) pure[q] = bad ? 0 : (some_n ? 2 : 1);
     }
 }
@@ -221,6 +223,16 @@ __global__ void __launch_bounds__(128) wfa_kernel(WfaArgs A)
 }
 
 // --------------------------------------------------------------- launchers --
+// Lanes per sequence of purity_kernel: a warp, unless the batch then has more threads
+// than the device and a smaller group still reads its mean sequence in four steps.
+static int purity_lanes(int n, int64_t seq_bytes)
+{
+    const int64_t mean = seq_bytes / (2 * (int64_t)n), threads = (int64_t)device_sms() * 2048;
+    int g = 32;
+    while (g > 1 && 2 * (int64_t)n * g > threads && 32 * g >= mean) g /= 2;
+    return g;
+}
+
 cudaError_t launch_pack(const PairDesc& D, int64_t seq_bytes, uint64_t* packed, uint8_t* pure, cudaStream_t st,
                         const Fills& fills)
 {
@@ -245,8 +257,11 @@ cudaError_t launch_pack(const PairDesc& D, int64_t seq_bytes, uint64_t* packed, 
         return cudaGetLastError();
     }
     launch_begin(K_PACK, st);
-    blocks = (int)std::min<int64_t>(((int64_t)2 * D.n + 7) / 8, (int64_t)device_sms() * 32);      // a warp per sequence
-    purity_kernel<<<blocks, 256, 0, st>>>(D, pure, fills);
+    const int g = purity_lanes(D.n, seq_bytes);
+    blocks = (int)std::min<int64_t>((2 * (int64_t)D.n * g + 255) / 256, (int64_t)device_sms() * 32);
+    auto kernel = g == 32 ? purity_kernel<32> : g == 16 ? purity_kernel<16> : g == 8 ? purity_kernel<8>
+                : g == 4  ? purity_kernel<4>  : g == 2  ? purity_kernel<2>  : purity_kernel<1>;
+    kernel<<<blocks, 256, 0, st>>>(D, pure, fills);
     launch_end(K_PACK, st);
     return cudaGetLastError();
 }

@@ -1435,18 +1435,23 @@ static SwPlan bound_plan_sw(const ga_sw_request* reqs, int32_t n, bool trace, in
     }
     P.ints[SP_L16] = 2 * ((n16 + 1) / 2);
     P.dir[SP_L16] = n16 ? (trace ? sw16ck_dir_words(maxM16, maxN16, T.sw_window) : sw16so_dir_words(maxM16, maxN16)) : 0;
-    // the 16-bit list has its whole-block phase when the widest possible item is above its share of them all
+    // the 16-bit list has its whole-block phase when the widest possible item is above its
+    // share of them all, and is one that the planner counts (sp_pack_list): the kernel with
+    // the phase runs the other items slower (2,000 pairs of 200 to 600 bases, none on a
+    // block: 1,140 us without the phase, 1,525 with it)
     cells16 = parts * (cells16 / 2);
     const int64_t warps16 = sw_coop_warps(SP_L16, trace, T), coop16 = sp_coop_cells(limit, cells16, warps16);
-    if ((int64_t)maxM16 * maxN16 > coop16) {
+    const int W16 = sw_coop_block(largest16, maxN16, cells16, device_sms());
+    const bool few16 = W16 * ((n16 + 1) / 2) * parts <= warps16;
+    if ((int64_t)maxM16 * maxN16 > coop16 && (few16 || sw16_by_cells(maxN16))) {
         P.ncoop[SP_L16] = 1;
+        P.w[SP_L16] = W16;
         // with a block for each item, the largest per-warp memory is a share of the
         // widest item's or the whole of one of coop16 cells (M rows, at most 255
         // padding columns, two words per 64 cells for rows and for edges each)
-        const int W = P.w[SP_L16] = sw_coop_block(largest16, maxN16, cells16, device_sms());
         const int64_t own = sw16_own_words(trace, T.sw_window);
-        if (W * ((n16 + 1) / 2) * parts <= warps16)
-            P.dir[SP_L16] = std::min(P.dir[SP_L16], std::max(sw_coop_share(P.dir[SP_L16], W, own),
+        if (few16)
+            P.dir[SP_L16] = std::min(P.dir[SP_L16], std::max(sw_coop_share(P.dir[SP_L16], W16, own),
                                                              coop16 / 16 + 16 * (int64_t)maxM16 + own + 8));
     }
     P.ints[SP_L32] = cnt[SP_L32];

@@ -1,4 +1,4 @@
-"""How the ranges of a host SW batch that run at once launch their work (on a runtime
+"""How a host SW batch, and its ranges that run at once, launch their work (on a runtime
 that records, no GPU)."""
 import numpy as np
 import pytest
@@ -36,3 +36,18 @@ def test_a_range_plans_in_small_blocks(rt):
     rt.clear()
     _call(5000, 100)
     assert rt.count("sp_small_kernel") == 0 and rt.count("sp_scan_kernelILi1024E") == 1
+
+
+def test_no_whole_block_phase_where_no_item_counts(rt):
+    """Items above their share of a batch of more items than blocks, all narrow, stay on a
+    warp each: the kernel without the whole-block phase runs them."""
+    n = 2000
+    rng = np.random.default_rng(2)
+    a = workloads.random_bases(rng, 700)
+    off, lens = np.zeros(n, np.int64), rng.integers(200, 700, n).astype(np.int32)
+    for cigar in (True, False):
+        rt.clear()
+        got = api.align_sw_batch_packed(a, off, lens, a, off, lens, scoring=(2, -3, 3, 1), with_cigar=cigar)
+        assert got.status == api.Status.ok, got.error
+        with_phase, without = ((BLOCKS, WARPS) if cigar else ("sw16so_kernelILb1E", "sw16so_kernelILb0E"))
+        assert rt.count(without) == 1 and rt.count(with_phase) == 0

@@ -291,10 +291,10 @@ struct Ctx {
     char* dev = nullptr;
     size_t dev_cap = 0;
     uint64_t dev_gen = 0;           // bumped whenever the device arena is reallocated
-    cudaGraphExec_t gexec = nullptr;  // the learned WFA path, captured once per launch shape
+    cudaGraphExec_t gexec = nullptr;  // the learned WFA path of the last launch shape that came twice in a row
     std::vector<uint64_t> gkey, gseen;
     int glaunches = 0;                // library kernels in gexec
-    cudaGraphExec_t swexec = nullptr; // the SW device work of a call or range, captured once per launch shape
+    cudaGraphExec_t swexec = nullptr; // the SW device work of a call or range, likewise
     std::vector<uint64_t> swkey, swseen;
     int swlaunches = 0;               // library kernels in swexec
     char* host = nullptr;
@@ -2370,9 +2370,9 @@ int32_t ga_sw_device_ex(const ga_device_batch* b, ga_sw_scoring sc, int32_t trac
     D.out_off = b->out_off; D.n = n;
 
     // A synchronous traceback call with a cell limit replays the CUDA graph of
-    // its launch shape: the first call of a shape reads the plan back to size
-    // the per-warp memory and captures the launches in plan mode (sizes read
-    // on the device); a replay whose plan needs more memory than that, or a
+    // its launch shape: the first two calls of a shape in a row read the plan
+    // back to size the per-warp memory and enqueue the launches in plan mode
+    // (sizes read on the device), the second captures them; a replay whose plan needs more memory than that, or a
     // launch that the graph lacks (the pairs behind the same pointers grew, or
     // moved to a list that was empty), is flagged by the kernels and the
     // planner (ERR_SCRATCH) and runs again through the read-back path.
@@ -2447,8 +2447,9 @@ int32_t ga_sw_device_ex(const ga_device_batch* b, ga_sw_scoring sc, int32_t trac
     }
     run_layout(c->dev, &dctr, &dedge, &ddirs);
     if (graph) {
-        // the launches of this shape in plan mode, captured with the memsets,
-        // the purity pass and the planner, then replayed (this call included)
+        // the launches of this shape in plan mode behind the purity pass (with
+        // the fills) and the planner: enqueued as they are, or, when the call
+        // before had this shape, captured and launched as a graph
         auto enqueue = [&]() -> cudaError_t {
             cudaError_t x = purity(dctr);
             if (x == cudaSuccess && route) x = launch_sw_route(D, sc.match, sc.gap_open, dfeat, dy, dtry, st);

@@ -13,7 +13,7 @@ struct WfaArgs {
     int32_t* out_score;
     int32_t* out_len;
     char* out_cigar;
-    int32_t* stack;          // per warp slot: (smax+1)^2 offsets (trace only)
+    int32_t* stack;          // per warp slot (cap + 1)^2 offsets, per block of the block kernel (smax + 1)^2 (trace only)
     int64_t stack_slot;
     int32_t* counter;        // next pair index
     int32_t* err;

@@ -199,7 +199,9 @@ int32_t ga_wfa_device(const ga_device_batch* batch, int32_t smax, int32_t trace,
  * bucketed queues served by persistent kernels (one pair per lane for small
  * predicted distances, one pair per warp otherwise, large distances on whole
  * blocks), replayed as one CUDA graph when a launch shape repeats; results are
- * the same as without it. */
+ * the same as without it.  A learned call on a stream that cannot begin a
+ * capture (the legacy stream, or one the caller is capturing) is refused unless
+ * it repeats the call before it: sizes, pointers and settings. */
 int32_t ga_wfa_device_ex(const ga_device_batch* batch, int32_t smax, int32_t trace, const ga_options* opt,
                          int32_t* out_score, int32_t* out_len, char* out_cigar, void* stream,
                          const char** err);

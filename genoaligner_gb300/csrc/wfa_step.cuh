@@ -135,7 +135,7 @@ __device__ int wfa_forward(const uint64_t* __restrict__ P, const uint64_t* __res
         if (TRACE) stk[0] = off0;
     }
     gsync<G>(gmask);
-    int reach = 0;
+    [[maybe_unused]] int reach = 0;
     for (int s = 1; s <= smax; ++s) {
         const int hi = wave_hi(s, n, kfinal, smax);
         int32_t* const row = TRACE ? stk + (int64_t)s * s + s : nullptr;
@@ -159,11 +159,16 @@ __device__ int wfa_forward(const uint64_t* __restrict__ P, const uint64_t* __res
             }
         }
         gsync<G>(gmask);
-        reach = cur[kfinal];
-        if (reach >= n) return s;
+        if constexpr (REACH) {
+            reach = cur[kfinal];
+            if (reach >= n) return s;
+        } else {
+            if (cur[kfinal] >= n) return s;
+        }
         int32_t* t = prev; prev = cur; cur = t;
     }
-    return REACH ? -1 - max(reach, 0) : -1;
+    if constexpr (REACH) return -1 - max(reach, 0);
+    else return -1;
 }
 
 // The walk's choice at a cell from the wavefront before: the offset it came from

@@ -840,6 +840,7 @@ static cudaError_t enqueue_wfa(Ctx* c, const WfaScratch& S, PairDesc D, int smax
             (e = cudaStreamWaitEvent(c->side, c->forked, 0)) != cudaSuccess) return e;
         WfaBlockArgs first = B;
         first.A.blk_count = nullptr;
+        first.packed = true;
         e = launch_wfa_block(first, S.blocks, K_WFA_ROUTED, st);
         const cudaError_t e2 = launch_routed(R, S.lane_slots, S.slots, c->side);
         cudaEventRecord(c->joined, c->side);

@@ -109,16 +109,30 @@ struct RoutedArgs {
 };
 
 // Pairs on whole blocks (wfa_block.cu): the first *big_count of the warp queue
-// (null: none), then the warp kernels' unresolved ones (A.blk, A.blk_count null: none)
-// unless they are more than few, which the warps take once more, then those of A.far
-// (A.far_count null: none).  A.stack: per block (A.smax + 1)^2 offsets.
+// (null: none), those of A.far (A.far_count null: none), then the warp kernels'
+// unresolved ones (A.blk, A.blk_count null: none) unless they are more than few, which
+// the warps take once more.  A.stack: per block (A.smax + 1)^2 offsets.
 struct WfaBlockArgs {
     WfaArgs A;
     const int2* big = nullptr;
     const int32_t* big_count = nullptr;
     int32_t* next;
     int32_t few = INT32_MAX;
+    bool packed = false;                  // beside the warp kernels: first_item
 };
+// First item of block b of the block kernel's grid (every item below `grid` is one
+// block's; later ones are taken as blocks come free).  Blocks fill the multiprocessors
+// one each, then a second each.  Alone, the kernel's first items go to blocks
+// in that order, a multiprocessor each: 300 pairs of 2.5 kb, score-only, 470 -> 431 us
+// against items by arrival.  Beside the warp kernels the two blocks of a multiprocessor
+// take neighbours, so that the ones without an item leave whole multiprocessors to the
+// warps: 461 pairs of 2.5 kb, 202 of them on blocks, with CIGARs 703 us, 990 spread;
+// by arrival 700 to 960, whichever way a build happened to fall.
+__host__ __device__ inline int first_item(int b, int grid, bool packed)
+{
+    const int half = (grid + 1) / 2;
+    return !packed ? b : (b < half ? 2 * b : 2 * (b - half) + 1);
+}
 int wfa_block_slots(int smax, bool trace, int sm_count);
 cudaError_t launch_wfa_block(const WfaBlockArgs& B, int blocks, int kernel_id, cudaStream_t st);
 // Words that a batch's first kernel sets for the later ones: counters, records and

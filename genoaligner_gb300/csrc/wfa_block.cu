@@ -91,19 +91,21 @@ __global__ void __launch_bounds__(BLK_T, 2) wfa_block_kernel(WfaBlockArgs B)
     __shared__ int s_q, s_at[3];
     const WfaArgs& A = B.A;
     const int t = threadIdx.x, smax = A.smax;
-    const int left = A.blk_count ? *A.blk_count : 0;
-    const int nbig = B.big_count ? *B.big_count : 0, nblk = nbig + (left > B.few ? 0 : left);
-    const int cnt = nblk + (A.far_count ? *A.far_count : 0);
+    // (the pairs that look longest before the rest of those left)
+    const int nbig = B.big_count ? *B.big_count : 0, nfar = nbig + (A.far_count ? *A.far_count : 0);
+    const int left = A.blk_count ? *A.blk_count : 0, cnt = nfar + (left > B.few ? 0 : left);
     int32_t* const wf0 = bsmem;
     int32_t* const wf1 = bsmem + 2 * smax + 3;
     int32_t* const stk = TRACE ? A.stack + blockIdx.x * ((int64_t)(smax + 1) * (smax + 1)) : nullptr;
-    for (;;) {
-        if (t == 0) s_q = atomicAdd(B.next, 1);
+    auto next_item = [&]() {
+        if (t == 0) s_q = gridDim.x + atomicAdd(B.next, 1);
         __syncthreads();
         const int q = s_q;
         __syncthreads();
-        if (q >= cnt) break;
-        const int p = q < nbig ? B.big[q].x : (q < nblk ? A.blk[q - nbig] : A.far[q - nblk]);
+        return q;
+    };
+    for (int q = first_item(blockIdx.x, gridDim.x, B.packed); q < cnt; q = next_item()) {
+        const int p = q < nbig ? B.big[q].x : (q < nfar ? A.far[q - nbig] : A.blk[q - nfar]);
         const int m = A.D.a_len[p], n = A.D.b_len[p];
         if (m <= 0 || n <= 0) {
             const int len = m <= 0 ? max(n, 0) : m;

@@ -1293,7 +1293,7 @@ static int sw_coop_warps(int l, bool trace, const ga_tune& T)
 
 // The plan, built on the device (sw_plan.cu) into `dwork`, its record into dres.
 // launched: when set, the launches are those of launch_plan for it -- the block sizes are
-// its, the 16-bit launch has the whole-block phase only if it counts such items, and
+// its, a list has whole-block items only if it counts some, and
 // pairs that no launch of its takes set ERR_SCRATCH at err; otherwise the device's choice.
 static cudaError_t enqueue_plan_sw(const PairDesc& D, const ga_sw_scoring& sc, bool trace, int64_t cell_limit,
                                    int32_t too_large_score, int32_t* out_score, int32_t* dwork, int32_t* scratch,
@@ -1306,11 +1306,12 @@ static cudaError_t enqueue_plan_sw(const PairDesc& D, const ga_sw_scoring& sc, b
         A.launched = 0;
         for (int l = 0; l < SP_LISTS; ++l) A.launched |= (launched->ints[l] > 0) << l;
         A.handover = launched->n_opt > 0;
+        A.decide_even = 0;
         A.err = err;
     }
     A.coop_limit = sw_coop_limit(T);
     for (int l = 0; l < SP_LISTS; ++l) {
-        A.coop_warps[l] = l == SP_L16 && launched && launched->ncoop[l] <= 0 ? 0 : sw_coop_warps(l, trace, T);
+        A.coop_warps[l] = launched && launched->ncoop[l] <= 0 ? 0 : sw_coop_warps(l, trace, T);
         A.coop_block[l] = launched ? launched->w[l] : 0;
     }
     A.sms = device_sms();
@@ -1397,7 +1398,12 @@ static SwPlan bound_plan_sw(const ga_sw_request* reqs, int32_t n, bool trace, in
     const int64_t cells = parts * all.cells;
     const int W32 = sw_coop_block(all.largest, all.cols, cells, device_sms());
     int64_t coop[SP_LISTS];
-    for (int l = SP_L32; l < SP_LISTS; ++l) coop[l] = sp_coop_cells(limit, cells, sw_coop_warps(l, trace, T));
+    bool blocks[SP_LISTS];
+    for (int l = SP_L32; l < SP_LISTS; ++l) {
+        const int64_t warps = sw_coop_warps(l, trace, T);
+        coop[l] = sp_coop_cells(limit, cells, warps);
+        blocks[l] = !sw_even_many((int64_t)parts * n, all.largest, cells, all.cols, warps);
+    }
     for (int32_t i = 0; i < n; ++i) {
         const int m = reqs[i].text_len, nn = reqs[i].pattern_len;
         if (cell_limit >= 0 && m > 0 && nn > 0 && ((int64_t)m + 1) * ((int64_t)nn + 1) > cell_limit) continue;
@@ -1425,8 +1431,8 @@ static SwPlan bound_plan_sw(const ga_sw_request* reqs, int32_t n, bool trace, in
         if (trace) {
             int64_t words = sw32ck_dir_words(m, nn, T.sw_long_log2);
             const int64_t c = (int64_t)std::max(m, 0) * std::max(nn, 0);
-            if (c > coop[l]) words = sw_coop_share(words, W32, sw32_own_words(m, nn, T.sw_long_log2));
-            if (c > std::min(limit, SW_COOP_MIN) && limit >= 0) {
+            if (blocks[l] && c > coop[l]) words = sw_coop_share(words, W32, sw32_own_words(m, nn, T.sw_long_log2));
+            if (blocks[l] && c > std::min(limit, SW_COOP_MIN) && limit >= 0) {
                 P.ncoop[l] = 1;
                 P.w[l] = W32;
             }
@@ -1444,7 +1450,8 @@ static SwPlan bound_plan_sw(const ga_sw_request* reqs, int32_t n, bool trace, in
     const int64_t warps16 = sw_coop_warps(SP_L16, trace, T), coop16 = sp_coop_cells(limit, cells16, warps16);
     const int W16 = sw_coop_block(largest16, maxN16, cells16, device_sms());
     const bool few16 = W16 * ((n16 + 1) / 2) * parts <= warps16;
-    if ((int64_t)maxM16 * maxN16 > coop16 && (few16 || sw16_by_cells(maxN16))) {
+    if ((int64_t)maxM16 * maxN16 > coop16 && (few16 || sw16_by_cells(maxN16)) &&
+        !sw_even_many((n16 + 1) / 2 * parts, largest16, cells16, maxN16, warps16)) {
         P.ncoop[SP_L16] = 1;
         P.w[SP_L16] = W16;
         // with a block for each item, the largest per-warp memory is a share of the

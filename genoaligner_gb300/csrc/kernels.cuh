@@ -304,6 +304,7 @@ struct SwPlanArgs {
     int32_t coop_warps[SP_LISTS];     // per list: resident warps of its kernel, 0 if it has no whole-block phase
     int32_t coop_block[SP_LISTS];     // ... and the warps of such a block, 0: chosen here (sw_coop_block)
     int32_t parts = 1;           // ranges like this one that run at once: together they are the device's work
+    int32_t decide_even = 1;     // sw_even_many is decided here (0: by the launches' host, which clears coop_warps)
     int32_t sms;
     int32_t score_only;          // 1: lists of the score-only kernels (sw16so, sw_kernel)
     // The launches that follow were chosen before this plan: the lists they take (a bit

@@ -166,7 +166,9 @@ __device__ __forceinline__ void sp_pack_list(const SwPlanArgs& P, const long lon
 {
     const long long cnt = res[SP_COUNT + l];
     int32_t* w = P.work + res[SP_BASE + l];
-    const int64_t coop = sp_coop_cells(P.coop_limit, sp_item_cells(P, res, l), P.coop_warps[l]);
+    const int64_t cells = sp_item_cells(P, res, l), all = P.parts * (l == SP_L16 ? (cnt + 1) / 2 : cnt);
+    const bool even = P.decide_even && sw_even_many(all, res[SP_LARGEST + l], cells, (int)res[SP_COLS + l], P.coop_warps[l]);
+    const int64_t coop = even ? INT64_MAX : sp_coop_cells(P.coop_limit, cells, P.coop_warps[l]);
     const int W = (int)res[SP_COOPW + l];
     if (l == SP_L16) {
         const long long items = (cnt + 1) / 2;

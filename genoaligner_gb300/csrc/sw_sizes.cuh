@@ -135,6 +135,17 @@ __host__ __device__ inline int64_t sp_coop_cells(int64_t limit, int64_t cells, i
     const int64_t t = share < SW_COOP_MIN ? SW_COOP_MIN : share;
     return t < limit ? t : limit;
 }
+// Near-equal items, too many for that: a cell costs a block's warps 1.8 times what it
+// costs a multiprocessor full of single ones, so a list that gives every multiprocessor
+// some six items and more, none above 1.6 times the mean, stays on warps whatever their
+// share.  (32 bits, on blocks and on warps: 900 pairs of 800 x 850 1,647 and 1,714
+// us, 1,000 1,896 and 1,733, 1,200 2,169 and 1,779; 1,000 of 3,100 x 3,200 7.7 and 9.1 ms,
+// 1,100 12.1 and 9.3.  16 bits: 1,000 items of 1,400 x 1,500 3.11 and 2.95 ms, 1,150
+// 4.43 and 2.88; 1,000 of 3,100 x 3,200 9.8 and 10.3, 1,150 13.5 and 10.1.)
+__host__ __device__ inline bool sw_even_many(int64_t items, int64_t largest, int64_t cells, int cols, int64_t warps)
+{
+    return 5 * largest * items <= 8 * cells && 40 * items > (cols >= 2048 ? 17 : 15) * warps;
+}
 // Warps of a whole-block launch's blocks, 4, 8 or 16: enough that the largest item,
 // which gets W of a multiprocessor's 16 resident warps, ends no later than the
 // multiprocessors' common work, and no more than a quarter of the 64-column bands it

@@ -51,3 +51,10 @@ def test_no_whole_block_phase_where_no_item_counts(rt):
         assert got.status == api.Status.ok, got.error
         with_phase, without = ((BLOCKS, WARPS) if cigar else ("sw16so_kernelILb1E", "sw16so_kernelILb0E"))
         assert rt.count(without) == 1 and rt.count(with_phase) == 0
+
+
+@pytest.mark.parametrize("n,length,blocks", [(1600, 1300, True), (2200, 1300, False), (1600, 3000, True),
+                                             (2000, 3000, True), (2300, 3000, False)])
+def test_near_equal_items_of_a_full_device_stay_on_warps(rt, n, length, blocks):
+    _call(n, length)                                    # n / 2 items, each above twice its share
+    assert (rt.count(BLOCKS) > 0) == blocks and (rt.count(WARPS) > 0) == (not blocks)

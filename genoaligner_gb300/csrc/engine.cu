@@ -871,8 +871,9 @@ static bool can_capture(cudaStream_t st)
 // first time, and captured when the same key comes again at once (`seen`: the call
 // before's): batches whose sizes differ from call to call, which no graph serves twice,
 // do not pay for one (SW batches of 1 to 3,558 pairs in turn: 40 to 70 us a call).  A
-// stream on which no capture can begin takes the key of the call before alone, by its
-// graph or, not yet captured, as it is.  `launches` keeps
+// stream on which no capture can begin takes the key of the call before alone: the legacy
+// one by its graph or, not yet captured, as it is; one that the caller is capturing as it
+// is, since no graph can be launched into a capture.  `launches` keeps
 // the number of library kernels the graph holds (counted once per replay).
 static cudaError_t replay_graph(cudaGraphExec_t& exec, std::vector<uint64_t>& have, std::vector<uint64_t>& seen,
                                 const std::vector<uint64_t>& key, int& launches, cudaStream_t st,
@@ -881,6 +882,7 @@ static cudaError_t replay_graph(cudaGraphExec_t& exec, std::vector<uint64_t>& ha
     const bool again = seen == key, can = can_capture(st);
     if (!again && !can) return cudaErrorStreamCaptureUnsupported;
     seen = key;
+    if (!can && st != cudaStreamLegacy) return enqueue();
     if (!exec || have != key) {
         if (!again || !can) return enqueue();
         // one capture at a time in the process (the ranges of a ranged call

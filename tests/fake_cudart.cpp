@@ -3,7 +3,8 @@
 // nothing, and a log of what a real runtime would have been asked to do.  Rules
 // of the real one that the tests rest on are kept: a launch with more dynamic
 // shared memory than its function's limit on the current device fails, and a
-// stream that is being captured, or the legacy one, cannot begin a capture.
+// stream that is being captured, or the legacy one, cannot begin a capture, and no
+// graph is launched into a capture.
 #include <cuda_runtime_api.h>
 
 #include <cstdio>
@@ -172,7 +173,12 @@ cudaError_t cudaGraphInstantiate(cudaGraphExec_t* e, cudaGraph_t, unsigned long 
 }
 cudaError_t cudaGraphDestroy(cudaGraph_t g) { std::free(g); return cudaSuccess; }
 cudaError_t cudaGraphExecDestroy(cudaGraphExec_t e) { std::free(e); return cudaSuccess; }
-cudaError_t cudaGraphLaunch(cudaGraphExec_t, cudaStream_t) { note("replay"); return cudaSuccess; }
+cudaError_t cudaGraphLaunch(cudaGraphExec_t, cudaStream_t s)
+{
+    if (of(s) && of(s)->capturing) return set(cudaErrorStreamCaptureUnsupported);
+    note("replay");
+    return cudaSuccess;
+}
 
 cudaError_t cudaEventCreate(cudaEvent_t* e) { *e = reinterpret_cast<cudaEvent_t>(get(1)); return cudaSuccess; }
 cudaError_t cudaEventCreateWithFlags(cudaEvent_t* e, unsigned) { return cudaEventCreate(e); }

@@ -115,7 +115,9 @@ def test_streams_that_cannot_be_captured(rt, legacy):
     assert refused(other, other_out)
     for _ in range(2):
         api.wfa_device(b, 64, True, *out, learned=True)
-    assert not refused(b, out) and rt.count("replay") == 1
+    assert not refused(b, out)
+    # a captured shape: replayed, or enqueued into the caller's capture, which takes no graph launch
+    assert rt.count("replay") == (1 if legacy else 0) and rt.log()
     api.wfa_device(other, 64, True, *other_out, learned=True)
     assert refused(b, out) and not refused(other, other_out)
 

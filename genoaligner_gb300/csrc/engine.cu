@@ -866,6 +866,16 @@ static bool can_capture(cudaStream_t st)
     return status == cudaStreamCaptureStatusNone;
 }
 
+// The context's memory is in use until the caller's stream gets here.  Not on a stream
+// under capture: nothing runs there, and waiting for an event recorded into a capture
+// invalidates that capture and fails after it.
+static void mark_pending(Ctx* c, cudaStream_t st)
+{
+    if (st != cudaStreamLegacy && !can_capture(st)) return;
+    cudaEventRecord(c->done, st);
+    c->pending = true;
+}
+
 // Replays `exec` when `key` (everything the enqueued launches bake in) is the
 // one it was captured for.  Another key's launches are enqueued as they are the
 // first time, and captured when the same key comes again at once (`seen`: the call
@@ -2267,8 +2277,7 @@ int32_t ga_wfa_device_ex(const ga_device_batch* b, int32_t smax, int32_t trace, 
         rc = GA_DEVICE_ERROR;
     }
     if (stream) {
-        cudaEventRecord(c->done, st);
-        c->pending = true;
+        mark_pending(c, st);
     } else if (cudaStreamSynchronize(st) != cudaSuccess) {
         cudaGetLastError();
         if (err) *err = E_SYNC;
@@ -2485,8 +2494,7 @@ int32_t ga_sw_device_ex(const ga_device_batch* b, ga_sw_scoring sc, int32_t trac
                     dctr + 32, st, dscr, nullptr, c) != cudaSuccess)
         return fail(E_LAUNCH);
     if (stream) {
-        cudaEventRecord(c->done, st);
-        c->pending = true;
+        mark_pending(c, st);
     } else if (cudaStreamSynchronize(st) != cudaSuccess) {
         return fail(E_SYNC);
     }

@@ -189,7 +189,10 @@ typedef struct ga_device_batch {
 /* WFA over a device batch.  out_score[i] (-1 unresolved), out_len[i] (CIGAR
  * length, 0 when trace == 0 or unresolved), out_cigar as above.  Enqueued on
  * `stream` (a cudaStream_t; NULL = this call's own stream, synchronised before
- * return).  Returns a status; `err` gets a static string on failure. */
+ * return).  Returns a status; `err` gets a static string on failure.  A graph
+ * that the caller captures from it holds the library's pooled memory: do not
+ * replay it beside other calls, nor after a larger batch than any before (the
+ * pool then moves); ga_wfa_device_noalloc has no such limit but the overlap. */
 int32_t ga_wfa_device(const ga_device_batch* batch, int32_t smax, int32_t trace,
                       int32_t* out_score, int32_t* out_len, char* out_cigar,
                       void* stream, const char** err);
